@@ -28,6 +28,8 @@
 
 #include "ocean_b200.h"
 #include "grid_barrier.cuh"
+#include "helm_common.cuh"
+#include "helm_pcg.cuh"
 #include "helmholtz.cuh"
 
 namespace oc {
@@ -48,16 +50,6 @@ using Tile8 = TileShape<8, 8>;
 using TileWide = TileShape<128, 16>;  // level 0 of large grids: one tile per CTA, one NumPy leaf per row
 // per-level tile shape codes (HLevel::shape)
 enum { SHAPE_32 = 0, SHAPE_3216 = 1, SHAPE_16 = 2, SHAPE_8 = 3, SHAPE_WIDE = 4 };
-
-// ------------------------------------------------------------------ the solve's CTAs
-// A solve runs on the CTAs of its launch, or, in a batched launch that solves
-// several systems at once, on one system's share of them: s_grid.cta is the
-// CTA's index among the solve's CTAs and s_grid.ncta their number. Every
-// work-distribution loop and the barrier use these instead of the launch's grid.
-struct SolveGrid {
-    int cta, ncta;
-};
-static __shared__ SolveGrid s_grid;
 
 // ------------------------------------------------------------------ barrier
 // the bounded grid barrier of grid_barrier.cuh on the solver's counter and status
@@ -82,38 +74,6 @@ __device__ __forceinline__ void cpa_wait_all() {
 }
 
 // ------------------------------------------------------------------ level operators
-struct Cell {
-    int e, ie, iw, jn, js;  // flat index and its four neighbours (periodic)
-};
-
-__device__ __forceinline__ Cell cell_of(const HLevel& L, int e) {
-    const int j = e / L.nx, i = e - j * L.nx;
-    Cell c;
-    c.e = e;
-    c.ie = j * L.nx + (i + 1 == L.nx ? 0 : i + 1);
-    c.iw = j * L.nx + (i == 0 ? L.nx - 1 : i - 1);
-    c.jn = (j + 1 == L.ny ? 0 : j + 1) * L.nx + i;
-    c.js = (j == 0 ? L.ny - 1 : j - 1) * L.nx + i;
-    return c;
-}
-
-// (A x)[e] with x read through L2 (other CTAs write it): VarOperator.apply
-// (solvers_var.py:47-53)
-__device__ __forceinline__ double apply_at(const HLevel& L, double coef, const double* x, const Cell& c) {
-    const double m = L.mask[c.e];
-    const double xm = __ldcg(x + c.e) * m;
-    const double xe = __ldcg(x + c.ie) * L.mask[c.ie];
-    const double xw = __ldcg(x + c.iw) * L.mask[c.iw];
-    const double xn = __ldcg(x + c.jn) * L.mask[c.jn];
-    const double xs = __ldcg(x + c.js) * L.mask[c.js];
-    const double fx = L.Ku[c.e] * (xe - xm);
-    const double fxw = L.Ku[c.iw] * (xm - xw);
-    const double fy = L.Kv[c.e] * (xn - xm);
-    const double fys = L.Kv[c.js] * (xm - xs);
-    const double lap = (fx - fxw) / L.dx2 + (fy - fys) / L.dy2;
-    return (xm - coef * lap) * m + xm * (1.0 - m);
-}
-
 // Gauss-Seidel value of cell e from the neighbours' current x (solvers_var.py:55-69)
 __device__ __forceinline__ double gs_at(const HLevel& L, const double* x, const double* b, const Cell& c) {
     const double nb = L.cx * (L.Ku[c.e] * __ldcg(x + c.ie) + L.Ku[c.iw] * __ldcg(x + c.iw)) +
@@ -207,37 +167,14 @@ __device__ void leaf_phase(const HelmParams& H, F f, double* outA, double* outB)
         const double a = leaf_sum_warp(va, len);
         const double bsum = outB ? leaf_sum_warp(vb, len) : 0.0;
         if (lane == 0) {
-            outA[L] = a;
-            if (outB) outB[L] = bsum;
+            const int slot = H.leaf_slot[L];
+            outA[slot] = a;
+            if (outB) outB[slot] = bsum;
         }
     }
 }
 
-// the fold's plan (ops, then the height offsets): a shared-memory copy made at
-// the start of the solve when it fits, else the global arrays
-struct FoldPlan {
-    const int2* ops;
-    const int* height_start;
-};
-
-// fold the leaf sums by NumPy's tree, in every CTA (the result is the same
-// everywhere); sm holds n_leaves doubles
-__device__ double tree_fold(const HelmParams& H, const FoldPlan& F, const double* leaf, double* sm) {
-    for (int t = threadIdx.x; t < H.n_leaves; t += blockDim.x) sm[t] = __ldcg(leaf + t);
-    __syncthreads();
-    for (int h = 0; h < H.n_heights; ++h) {
-        for (int t = F.height_start[h] + threadIdx.x; t < F.height_start[h + 1]; t += blockDim.x) {
-            const int2 op = F.ops[t];
-            sm[op.x] = sm[op.x] + sm[op.y];
-        }
-        __syncthreads();
-    }
-    const double r = sm[0];
-    __syncthreads();
-    return r;
-}
-
-// The same fold for grids whose leaf sums do not fit one CTA's shared memory
+// The fold of the leaf sums for grids with more slots than one CTA folds
 // (H.big_fold): the tree is cut below the nodes of at most a block's worth of
 // leaves. Each block subtree is folded by one CTA and its root written to
 // `broot`; after a grid barrier every CTA folds the top of the tree over the
@@ -276,65 +213,16 @@ __device__ double fold_blocks(const HelmParams& H, const double* leaf, double* b
     return r;
 }
 
-// The same fold when NumPy's tree over the leaves is perfect (2^m leaves, node
-// (i, i + 2^h) at height h; H.perfect_lanes = P > 0): each lane folds P
-// consecutive leaves in registers, the lanes of a warp fold their subtrees by
-// shuffles, and warp 0 folds the warps' subtrees. Every addition is the tree's
-// (left + right), so the result is bit-identical to tree_fold's, with two CTA
-// barriers instead of one per height.
-template <int P>
-__device__ __forceinline__ double lane_tree(const double* v) {
-    if constexpr (P == 1)
-        return v[0];
-    else
-        return lane_tree<P / 2>(v) + lane_tree<P / 2>(v + P / 2);
-}
-
-template <int P>
-__device__ double perfect_fold(int n, const double* leaf, double* sm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwa = n / (32 * P);  // warps in use: a power of two, at most the CTA's
-    if (warp < nwa) {
-        double v[P];
-        const double* src = leaf + warp * 32 * P + lane * P;
-#pragma unroll
-        for (int q = 0; q < P; ++q) v[q] = __ldcg(src + q);
-        double x = lane_tree<P>(v);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_down_sync(0xffffffffu, x, o);
-            if ((lane & (2 * o - 1)) == 0) x = x + y;
-        }
-        if (lane == 0) sm[warp] = x;
+// the sum of one of the leaf buffers (leafA, leafB or leafC) in NumPy's order, in
+// every CTA (the result is the same everywhere)
+__device__ __forceinline__ double fold_sum(const HelmParams& H, const double* leaf, double* sm, bool& ok) {
+    if (!H.big_fold) {
+        double r[1];
+        const double* lv[1] = {leaf};
+        slots_fold_any<1>(H.n_slots, lv, sm, r);
+        __syncthreads();  // sm is the tiles' next
+        return r[0];
     }
-    __syncthreads();
-    if (warp == 0) {
-        double x = lane < nwa ? sm[lane] : 0.0;
-        for (int o = 1; o < nwa; o <<= 1) {
-            const double y = __shfl_down_sync(0xffffffffu, x, o);
-            if ((lane & (2 * o - 1)) == 0) x = x + y;
-        }
-        __syncwarp();
-        if (lane == 0) sm[0] = x;
-    }
-    __syncthreads();
-    const double r = sm[0];
-    __syncthreads();
-    return r;
-}
-
-// the sum of one of the leaf buffers (leafA, leafB or leafC) in NumPy's order
-__device__ __forceinline__ double fold_sum(const HelmParams& H, const FoldPlan& F, const double* leaf, double* sm,
-                                           bool& ok) {
-    switch (H.perfect_lanes) {
-        case 1: return perfect_fold<1>(H.n_leaves, leaf, sm);
-        case 2: return perfect_fold<2>(H.n_leaves, leaf, sm);
-        case 4: return perfect_fold<4>(H.n_leaves, leaf, sm);
-        case 8: return perfect_fold<8>(H.n_leaves, leaf, sm);
-        case 16: return perfect_fold<16>(H.n_leaves, leaf, sm);
-        default: break;
-    }
-    if (!H.big_fold) return tree_fold(H, F, leaf, sm);
     double* broot = leaf == H.leafA ? H.broot : (leaf == H.leafB ? H.broot + H.n_blocks : H.broot + 2 * H.n_blocks);
     return fold_blocks(H, leaf, broot, sm, ok);
 }
@@ -883,16 +771,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
     // with H.persist0 the first 4 RN doubles hold level 0's coefficient tile for the
     // whole solve; every other use of shared memory works above them
     double* persist = H.persist0 ? smem_all : nullptr;
-    double* const ops_base = smem_all + (H.persist0 ? 4 * TileWide::RN : 0);
-    double* sm = ops_base + H.ops_smem;
-    FoldPlan fold{H.ops, H.height_start};
-    if (H.ops_smem) {
-        int2* so = reinterpret_cast<int2*>(ops_base);
-        int* sh = reinterpret_cast<int*>(so + H.n_ops);
-        for (int t = threadIdx.x; t < H.n_ops; t += blockDim.x) so[t] = H.ops[t];
-        for (int t = threadIdx.x; t <= H.n_heights; t += blockDim.x) sh[t] = H.height_start[t];
-        fold = FoldPlan{so, sh};  // first read after the barrier that ends the first leaf phase
-    }
+    double* sm = smem_all + (H.persist0 ? 4 * TileWide::RN : 0);
     const HLevel& L0 = H.lv[0];
     const double* rhs = H.rhs;
     double* x = L0.x;
@@ -914,7 +793,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                },
                H.leafA, nullptr);
     ok = grid_sync(H);
-    const double norm_b = ok ? sqrt(fold_sum(H, fold, H.leafA, sm, ok)) : 0.0;
+    const double norm_b = ok ? sqrt(fold_sum(H, H.leafA, sm, ok)) : 0.0;
     if (persist) persist_level0(H, persist);  // the coefficients are fixed during the solve
     if (H.coarse_persist && s_grid.cta == 0) {
         coarse_coef_load(H, persist, sm);
@@ -953,7 +832,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                     if (!ok) break;
                 }
                 iters = it;
-                const double res = sqrt(fold_sum(H, fold, H.leafA, sm, ok));
+                const double res = sqrt(fold_sum(H, H.leafA, sm, ok));
                 if (!ok) break;
                 if (res <= tol) {
                     conv = 1;
@@ -1016,7 +895,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                        H.leafB, nullptr);
             ok = grid_sync(H);
             if (!ok) goto done;
-            double rz = fold_sum(H, fold, H.leafB, sm, ok);
+            double rz = fold_sum(H, H.leafB, sm, ok);
             if (!ok) goto done;
             conv = 0;
             for (int it = 1; it <= H.max_iter; ++it) {
@@ -1029,7 +908,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                            H.leafC, nullptr);
                 ok = grid_sync(H);
                 if (!ok) break;
-                const double alpha = rz / fold_sum(H, fold, H.leafC, sm, ok);
+                const double alpha = rz / fold_sum(H, H.leafC, sm, ok);
                 if (!ok) break;
                 leaf_phase(H,
                            [&](int e) {
@@ -1050,7 +929,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                 ok = grid_sync(H);
                 if (!ok) break;
                 iters = it;
-                const double res = sqrt(fold_sum(H, fold, H.leafA, sm, ok));
+                const double res = sqrt(fold_sum(H, H.leafA, sm, ok));
                 if (!ok) break;
                 if (res <= tol) {
                     conv = 1;
@@ -1068,7 +947,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                     ok = grid_sync(H);
                     if (!ok) break;
                 }
-                const double rz_new = fold_sum(H, fold, H.leafB, sm, ok);
+                const double rz_new = fold_sum(H, H.leafB, sm, ok);
                 if (!ok) break;
                 const double beta = rz_new / rz;
                 for (int e = grid_team().first; e < L0.n; e += grid_team().stride)
@@ -1168,6 +1047,27 @@ struct PwNode {
     int lo, height;
 };
 
+// The tree embedded in a perfect one: the slot of each leaf, in order, under a
+// node of height `height` (2^height slots) whose first slot is `slot`. A leaf
+// above height 0 takes the first slot of its subtree.
+static int pairwise_height(long n) {
+    if (n <= 128) return 0;
+    long h = n / 2;
+    h -= h % 8;
+    return std::max(pairwise_height(h), pairwise_height(n - h)) + 1;
+}
+
+static void pairwise_slots(long n, int height, int slot, std::vector<int>& slots) {
+    if (n <= 128) {
+        slots.push_back(slot);
+        return;
+    }
+    long h = n / 2;
+    h -= h % 8;
+    pairwise_slots(h, height - 1, slot, slots);
+    pairwise_slots(n - h, height - 1, slot + (1 << (height - 1)), slots);
+}
+
 static PwNode pairwise_build(long start, long n, std::vector<int>& leaves,
                              std::vector<std::vector<int2>>& by_height) {
     if (n <= 128) {
@@ -1182,27 +1082,6 @@ static PwNode pairwise_build(long start, long n, std::vector<int>& leaves,
     if ((int)by_height.size() < height) by_height.resize(height);
     by_height[height - 1].push_back(make_int2(a.lo, b.lo));
     return {a.lo, height};
-}
-
-// P > 0 when the tree over the leaves is perfect -- 2^m leaves, the nodes of
-// height h (0: pairs of leaves) exactly (i, i + 2^h) for i a multiple of 2^(h+1)
-// -- with at least 32 leaves: the leaves per lane of perfect_fold for `warps`
-// warps (at most 16); 0 otherwise
-static int perfect_lanes(int n, const std::vector<std::vector<int2>>& by_height, int warps) {
-    if (n < 32 || (n & (n - 1)) != 0) return 0;
-    int m = 0;
-    while ((1 << m) < n) ++m;
-    if ((int)by_height.size() != m) return 0;
-    for (int h = 0; h < m; ++h) {
-        std::vector<int2> ops = by_height[h];
-        const int step = 1 << (h + 1);
-        if ((int)ops.size() != n / step) return 0;
-        std::sort(ops.begin(), ops.end(), [](int2 a, int2 b) { return a.x < b.x; });
-        for (int q = 0; q < (int)ops.size(); ++q)
-            if (ops[q].x != q * step || ops[q].y != q * step + (1 << h)) return 0;
-    }
-    const int P = std::max(1, n / (32 * warps));
-    return P <= 16 ? P : 0;
 }
 
 // leaves of NumPy's pairwise tree over n contiguous elements
@@ -1353,7 +1232,7 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     H.Ap = (double*)dalloc(sizeof(double) * n);
     // pairwise plan (two-level for grids whose leaf sums exceed shared memory)
     std::vector<int> leaves;
-    std::vector<std::vector<int2>> by_height;
+    std::vector<std::vector<int2>> by_height;  // of the whole tree; the embedded fold does not need it
     TwoLevelPlan two;
     H.big_fold = pairwise_leaves((long)n) > kFoldOneLevelLeaves ? 1 : 0;
     if (H.big_fold) {
@@ -1363,41 +1242,40 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         pairwise_build(0, (long)n, leaves, by_height);
     }
     leaves.push_back((int)n);
-    std::vector<int> hstart{0};
-    std::vector<int2> ops;
-    for (auto& v : by_height) {
-        ops.insert(ops.end(), v.begin(), v.end());
-        hstart.push_back((int)ops.size());
-    }
     H.n_leaves = (int)leaves.size() - 1;
-    H.n_heights = (int)by_height.size();
-    H.perfect_lanes = H.big_fold ? 0 : perfect_lanes(H.n_leaves, by_height, block_ / 32);
+    // the leaves' slots in the perfect tree (at least one warp's 32); the two-level
+    // fold reads the leaves in order
+    std::vector<int> slots;
+    if (H.big_fold) {
+        for (int q = 0; q < H.n_leaves; ++q) slots.push_back(q);
+        H.n_slots = H.n_leaves;
+    } else {
+        const int height = pairwise_height((long)n);
+        pairwise_slots((long)n, height, 0, slots);
+        H.n_slots = std::max(32, 1 << height);
+    }
     int* d_leaves = (int*)dalloc(sizeof(int) * leaves.size());
-    int* d_hstart = (int*)dalloc(sizeof(int) * hstart.size());
-    int2* d_ops = (int2*)dalloc(sizeof(int2) * std::max<size_t>(1, ops.size()));
-    H.leafA = (double*)dalloc(sizeof(double) * H.n_leaves);
-    H.leafB = (double*)dalloc(sizeof(double) * H.n_leaves);
-    H.leafC = (double*)dalloc(sizeof(double) * H.n_leaves);
+    int* d_slots = (int*)dalloc(sizeof(int) * slots.size());
+    H.leafA = (double*)dalloc(sizeof(double) * H.n_slots);  // zeroed: slots without a leaf stay 0
+    H.leafB = (double*)dalloc(sizeof(double) * H.n_slots);
+    H.leafC = (double*)dalloc(sizeof(double) * H.n_slots);
     unsigned long long* bar = (unsigned long long*)dalloc(sizeof(unsigned long long));
     H.log_cap = log_cap;
     H.log_iters = (int*)dalloc(sizeof(int) * log_cap);
     H.log_conv = (int*)dalloc(sizeof(int) * log_cap);
     H.log_count = (int*)dalloc(sizeof(int));
-    if (!H.r || !H.z || !H.p || !H.Ap || !d_leaves || !d_hstart || !d_ops || !H.leafA || !H.leafB || !H.leafC ||
+    if (!H.r || !H.z || !H.p || !H.Ap || !d_leaves || !d_slots || !H.leafA || !H.leafB || !H.leafC ||
         !bar || !H.log_iters || !H.log_conv || !H.log_count) {
         err = "cudaMalloc failed (Helmholtz work)";
         return OC_ERR_CUDA;
     }
     cudaMemcpy(d_leaves, leaves.data(), sizeof(int) * leaves.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(d_hstart, hstart.data(), sizeof(int) * hstart.size(), cudaMemcpyHostToDevice);
-    if (!ops.empty()) cudaMemcpy(d_ops, ops.data(), sizeof(int2) * ops.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(d_slots, slots.data(), sizeof(int) * slots.size(), cudaMemcpyHostToDevice);
     H.leaf_start = d_leaves;
-    H.height_start = d_hstart;
-    H.ops = d_ops;
-    H.n_ops = (int)ops.size();
+    H.leaf_slot = d_slots;
     H.bar_count = bar;
     H.wait_cycles = kBarrierCycles;
-    size_t fold_doubles = (size_t)H.n_leaves;  // shared memory the fold needs
+    size_t fold_doubles = 32;  // shared memory the fold needs
     if (H.big_fold) {
         H.n_blocks = (int)two.blocks.size();
         std::vector<int> top_hstart{0};
@@ -1493,7 +1371,7 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     const size_t coarse_work = 6 * coarse_cells + (H.coarse_from < H.n_levels ? (size_t)H.lv[H.coarse_from].n : 0);
     const size_t mg_work = mg_levels ? std::max<size_t>(tile_work, coarse_work) : 0;
     // in a batched launch a system has fewer CTAs than tiles: no persistent level-0
-    // tile (its six arrays are loaded per tile instead) and no shared copy of the plan
+    // tile (its six arrays are loaded per tile instead)
     size_t tile_work_b = 0;
     if (mg_levels) {
         for (int l = 0; l < n_grid; ++l) tile_work_b = std::max<size_t>(tile_work_b, 6 * (size_t)rn_of(H.lv[l].shape));
@@ -1507,13 +1385,6 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa{};
     cudaFuncGetAttributes(&fa, k_helm_solve);  // static shared memory (the barrier's word) comes first
-    // the fold's plan joins shared memory when it fits beside the rest
-    const size_t plan_doubles = (sizeof(int2) * ops.size() + sizeof(int) * hstart.size() + sizeof(double) - 1) / sizeof(double);
-    H.ops_smem = 0;
-    if (!H.big_fold && smem_ + sizeof(double) * plan_doubles + fa.sharedSizeBytes <= (size_t)smem_optin) {
-        H.ops_smem = (int)plan_doubles;
-        smem_ += sizeof(double) * plan_doubles;
-    }
     if (smem_ + fa.sharedSizeBytes > (size_t)smem_optin) {
         err = "Helmholtz grid too large for the single-pass reduction tree";
         return OC_ERR_UNSUPPORTED;
@@ -1546,6 +1417,11 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         H.coarse_persist = (H.persist0 && mg_levels && H.coarse_from > 0 && H.coarse_from < H.n_levels &&
                             grid_ > tiles0 && ccells <= (size_t)TileWide::RN) ? 1 : 0;
     }
+    // PCG-Jacobi with the vectors on the chip (its operator relies on a 0/1 mask)
+    bool unit_mask = true;
+    for (size_t c = 0; c < n && unit_mask; ++c) unit_mask = mask_host[c] == 0.0 || mask_host[c] == 1.0;
+    pcg_ = !refined && kind == HK_PCG_JACOBI && unit_mask && !H.big_fold &&
+           pcg_plan(leaves, H.n_slots, nx, pcg_plan_);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         err = std::string("Helmholtz init: ") + cudaGetErrorString(e);
@@ -1604,7 +1480,6 @@ HelmParams HelmSolver::batched_params(const double* rhs, double* x) const {
     H.persist0 = 0;
     H.coarse_persist = 0;
     H.warm = warm_ ? 1 : 0;
-    H.ops_smem = 0;
     return H;
 }
 
@@ -1728,6 +1603,51 @@ void helm_batch_free(HelmBatch& b) {
 
 int HelmSolver::solve(const double* rhs, double* x, cudaStream_t s, std::string& err) {
     if (refined_) return refined_->solve(rhs, x, s, err);
+    if (pcg_) {
+        const HLevel& L = hp_.lv[0];
+        PcgParams P{};
+        P.nx = L.nx;
+        P.ny = L.ny;
+        P.n = L.n;
+        P.max_iter = hp_.max_iter;
+        P.warm = warm_ ? 1 : 0;
+        P.coef = hp_.coef;
+        P.rtol = hp_.rtol;
+        P.dx2 = L.dx2;
+        P.dy2 = L.dy2;
+        P.mask = L.mask;
+        P.Ku = L.Ku;
+        P.Kv = L.Kv;
+        P.inv_diag = L.inv_diag;
+        P.rhs = rhs;
+        P.x = x;
+        P.r = hp_.r;
+        P.z = hp_.z;
+        P.Ap = hp_.Ap;
+        P.n_leaves = hp_.n_leaves;
+        P.n_slots = hp_.n_slots;
+        P.leaf_start = hp_.leaf_start;
+        P.leaf_slot = hp_.leaf_slot;
+        P.leafA = hp_.leafA;
+        P.leafB = hp_.leafB;
+        P.leafC = hp_.leafC;
+        P.own_max = pcg_plan_.own_max;
+        P.window = pcg_plan_.window;
+        P.lead = pcg_plan_.mode == PCG_ONE ? 0 : L.nx;
+        P.bar_count = hp_.bar_count;
+        P.status = hp_.status;
+        P.wait_cycles = hp_.wait_cycles;
+        P.log_iters = hp_.log_iters;
+        P.log_conv = hp_.log_conv;
+        P.log_count = hp_.log_count;
+        P.log_cap = hp_.log_cap;
+        const cudaError_t e = pcg_launch(pcg_plan_, P, s);
+        if (e != cudaSuccess) {
+            err = std::string("Helmholtz PCG launch: ") + cudaGetErrorString(e);
+            return OC_ERR_CUDA;
+        }
+        return OC_OK;
+    }
     HelmParams H = hp_;
     H.rhs = rhs;
     H.lv[0].x = x;

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "helm_pcg.cuh"
 #include "helm_refined.cuh"
 #include "oc_internal.cuh"
 
@@ -43,16 +44,14 @@ struct HelmParams {
     // NumPy pairwise-summation plan of the level-0 vectors
     int n_leaves;
     const int* leaf_start;    // n_leaves + 1
-    int n_heights;
-    const int* height_start;  // n_heights + 1 offsets into ops
-    const int2* ops;          // (lo, mid): value[lo] += value[mid]
-    int n_ops;
-    int ops_smem;             // doubles of shared memory holding a copy of ops and height_start (0: none)
-    int perfect_lanes;        // > 0: the tree is perfect, folded with this many leaves per lane (perfect_fold)
+    // the leaves' slots in the perfect binary tree the sums are folded by; the leaf
+    // buffers have n_slots values, 0 where no leaf is
+    int n_slots;
+    const int* leaf_slot;
     double* leafA;
     double* leafB;
     double* leafC;
-    // two-level fold when the leaf sums exceed shared memory (big_fold): block
+    // two-level fold of more than 16,384 leaves (big_fold): block
     // subtrees (first leaf, leaves, offset into bh_start, heights) with their ops
     // relative to the block's first leaf, then the top of the tree over the roots
     int big_fold, n_blocks, top_heights;
@@ -119,6 +118,8 @@ class HelmSolver {
     HelmParams hp_{};
     RefinedHelm* refined_ = nullptr;  // kind HK_REFINED: the solves go here
     bool warm_ = false;
+    bool pcg_ = false;  // the on-chip PCG-Jacobi kernel takes the solves
+    PcgPlan pcg_plan_{};
     std::vector<void*> allocs_;
     int grid_ = 0, block_ = 512;
     size_t smem_ = 0, smem_batched_ = 0;

@@ -1,0 +1,83 @@
+"""The Helmholtz solve at the sizes where its launch form changes, against the oracle.
+
+PCG-Jacobi runs on one CTA, on one cluster of CTAs or on every SM, and keeps all,
+some or only the search direction in shared memory; the leaf sums are folded in a
+perfect tree in which grids of other sizes leave slots empty. Iteration counts and
+solutions are the oracle's bit for bit in every form.
+"""
+
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from oracle import ocean_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(nx, ny, seed, walls=False):
+    rng = np.random.default_rng(seed)
+    dx, dy = 4.0e6 / nx, 5.0e6 / ny
+    mask = np.ones((ny, nx))
+    mask[ny // 4:ny // 3, nx // 5:nx // 2] = 0.0
+    ku = (0.5 + 0.5 * rng.random((ny, nx))) * mask * np.roll(mask, -1, 1)
+    kv = (0.5 + 0.5 * rng.random((ny, nx))) * mask * np.roll(mask, -1, 0)
+    if walls:
+        ku[:, -1] = 0.0
+        kv[-1, :] = 0.0
+    return dx, dy, 0.4 * dx * dy, ku, kv, mask, rng.standard_normal((ny, nx)) * mask
+
+
+@pytest.mark.parametrize("nx,ny", [
+    (8, 4), (9, 7), (128, 4), (32, 64),   # one CTA, from less than one leaf to its largest
+    (45, 46), (41, 640), (640, 41),       # one cluster; short and long rows
+    (251, 187), (256, 256),               # uneven leaves; the largest cluster
+    (257, 256), (512, 512),               # every SM, all vectors on the chip
+    (1000, 720),                          # r and A p on the chip
+    (1300, 1260), (5000, 300),            # only the window of p; rows longer than a range
+    (600, 2), (3001, 3),                  # a window that would meet itself: the general kernel
+])
+def test_pcg_jacobi_forms_match_oracle(nx, ny):
+    from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+    dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, 100 * nx + ny)
+    solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind="pcg_jacobi",
+                          rtol=1e-10)
+    ref = orc.Helmholtz(nx, ny, 4.0e6, 5.0e6, coef, ku, kv, mask, "pcg_jacobi", 1e-10, 2000)
+    for r in (rhs, rhs[::-1].copy() * mask, np.zeros_like(rhs)):
+        x, rep = solver.solve(r)
+        xr, itr, ok = ref.solve(r)
+        assert rep.iterations == itr and rep.converged == ok
+        assert np.array_equal(x, xr)
+    solver.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(40, 30), (120, 130), (400, 390)])
+def test_pcg_jacobi_stops_at_max_iter(nx, ny):
+    """A solve that does not converge leaves its last iterate and says so, in every form."""
+    from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+    dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx)
+    solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind="pcg_jacobi",
+                          rtol=1e-12, max_iter=3)
+    ref = orc.Helmholtz(nx, ny, 4.0e6, 5.0e6, coef, ku, kv, mask, "pcg_jacobi", 1e-12, 3)
+    x, rep = solver.solve(rhs)
+    xr, itr, ok = ref.solve(rhs)
+    assert not ok and not rep.converged and rep.iterations == itr == 3
+    assert np.array_equal(x, xr)
+    solver.close()
+
+
+@pytest.mark.parametrize("kind,nx,ny", [("pcg_rbgs", 50, 34), ("pcg_rbgs", 251, 187), ("rbgs", 37, 29),
+                                        ("multigrid", 24, 16), ("multigrid", 152, 104)])
+def test_uneven_leaf_trees_match_oracle(kind, nx, ny):
+    """Grids whose leaf tree is not perfect, through the other solvers (closed at the
+    edges: across the wrap of an odd size, neighbours have the same colour)."""
+    from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+    dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx + ny, walls=True)
+    solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind=kind, rtol=1e-10)
+    ref = orc.Helmholtz(nx, ny, 4.0e6, 5.0e6, coef, ku, kv, mask, kind, 1e-10, 2000)
+    x, rep = solver.solve(rhs)
+    xr, itr, ok = ref.solve(rhs)
+    assert rep.iterations == itr and rep.converged == ok
+    assert np.array_equal(x, xr)
+    solver.close()
