@@ -13,6 +13,13 @@
 //   then p = z + beta p over the window: z of the rows outside the range is read
 //   from the owners, and their p is formed again here by the same operations on
 //   the same values instead of waiting for a third barrier.
+// A warp takes a leaf at a time, its cells and their sum; with every SM at work, where a
+// CTA has tens of leaves, the cells are spread over all threads instead, whatever their
+// leaf, and the leaves summed afterwards, eight lanes to a leaf. 1000 x 720: 904 us a
+// solve by warps, 812 spread; 251 x 187 on a cluster 490 against 560, 128 x 4 on one CTA
+// 245 against 309, where the extra barrier and pass cost more than idle warps do.
+// (With the vectors in L2, four barriers and two shuffles a value the three took 1326,
+// 1023 and 1505 us.)
 // The number of CTAs follows the grid size (pcg_plan): one CTA, whose barriers are
 // __syncthreads, for the smallest grids; one cluster of up to 16 CTAs, with the
 // cluster's hardware barrier; else every SM with the bounded grid barrier.
@@ -64,20 +71,61 @@ __device__ __forceinline__ void pcg_fold(const PcgParams& H, const double* const
     }
 }
 
+// NumPy's pairwise sums of the two values f(e) gives per cell, over each of the CTA's
+// leaves, into the leaves' slots of outA and outB. Eight lanes sum a leaf, four leaves a
+// warp: lane j forms interleaved accumulator j in its sequential order, the eight are
+// folded ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)) by shuffles, and the len mod 8 last cells
+// are added one by one.
+template <class F>
+__device__ __forceinline__ void leaf_group_sums(int nlf, const int* lstart, const int* lslot, F f, double* outA,
+                                                double* outB) {
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    for (int l0 = (threadIdx.x >> 5) * 4; l0 < nlf; l0 += PCG_WARPS * 4) {
+        const int l = l0 + (lane >> 3);
+        const int st = l < nlf ? lstart[l] : 0, len = l < nlf ? lstart[l + 1] - st : 0, m = len & ~7;
+        double2 acc = make_double2(0.0, 0.0);
+        if (m) {
+            acc = f(st + j);
+#pragma unroll 5
+            for (int t = 8; t < m; t += 8) {
+                const double2 v = f(st + t + j);
+                acc.x = acc.x + v.x;
+                acc.y = acc.y + v.y;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            acc.x = acc.x + __shfl_xor_sync(0xffffffffu, acc.x, o);
+            if (outB) acc.y = acc.y + __shfl_xor_sync(0xffffffffu, acc.y, o);
+        }
+        for (int t = m; t < len; ++t) {
+            const double2 v = f(st + t);
+            acc.x = acc.x + v.x;
+            acc.y = acc.y + v.y;
+        }
+        if (j == 0 && l < nlf) {
+            outA[lslot[l]] = acc.x;
+            if (outB) outB[lslot[l]] = acc.y;
+        }
+    }
+}
+
 // KEEP: PCG_KEEP_ALL x, r, A p and the coefficients in shared memory; PCG_KEEP_RA
 // r and A p; PCG_KEEP_P only the window of p
 template <int MODE, int KEEP>
 __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) {
     extern __shared__ __align__(16) double s_pcg[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int cta = blockIdx.x, ncta = gridDim.x;
     const int nx = H.nx, n = H.n;
     const int lf0 = (int)((long long)H.n_leaves * cta / ncta), lf1 = (int)((long long)H.n_leaves * (cta + 1) / ncta);
     const int s0 = H.leaf_start[lf0], own = H.leaf_start[lf1] - s0;
     // shared memory: the warps' leaf buffers, fold scratch (or the leaf buffers of
     // a single CTA), the window of p, then what KEEP keeps
+    constexpr bool SPREAD = MODE == PCG_GRID;
+    const int lane = tid & 31, warp = tid >> 5;
     double* bufs = s_pcg + warp * 2 * LEAF_PAD;
-    double* scratch = s_pcg + PCG_WARPS * 2 * LEAF_PAD;
+    double* scratch = s_pcg + (SPREAD ? 0 : PCG_WARPS * 2 * LEAF_PAD);
     double* pw = scratch + 3 * 128;
     double* next = pw + H.window;
     double *r, *ap, *x, *ke = nullptr, *kw = nullptr, *kn = nullptr, *ks = nullptr, *id = nullptr;
@@ -100,7 +148,15 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
     } else {
         x = H.x + s0;
     }
-    unsigned char* flag = reinterpret_cast<unsigned char*>(next);  // 1: wet, 2: last column, 4: first column
+    // own leaves: where each starts in the range, and its slot
+    const int nlf = lf1 - lf0;
+    int* lstart = reinterpret_cast<int*>(next);
+    int* lslot = lstart + H.leaves_max + 1;
+    unsigned char* flag = reinterpret_cast<unsigned char*>(lslot + H.leaves_max + 1);  // 1: wet, 2: last column, 4: first
+    for (int t = tid; t <= nlf; t += PCG_THREADS) {
+        lstart[t] = H.leaf_start[lf0 + t] - s0;
+        if (t < nlf) lslot[t] = H.leaf_slot[lf0 + t];
+    }
     double* leafs[3];
     if constexpr (MODE == PCG_ONE) {
         leafs[0] = scratch;
@@ -141,38 +197,30 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
     __syncthreads();
     // b = rhs mask, the residual of the starting iterate (0, or the x given), z = r / diag;
     // |b|^2 and <r, z> by leaves (solvers_var.py:163-168, 181-185)
-    for (int L = lf0 + warp; L < lf1; L += PCG_WARPS) {
-        const int st = H.leaf_start[L] - s0, len = H.leaf_start[L + 1] - s0 - st;
-        for (int t = lane; t < len; t += 32) {
-            const int e = st + t, g = s0 + e;
-            const double b = H.rhs[g] * H.mask[g];
-            double re = b;
-            if (H.warm) {
-                HLevel L0;
-                L0.mask = H.mask;
-                L0.Ku = const_cast<double*>(H.Ku);
-                L0.Kv = const_cast<double*>(H.Kv);
-                L0.dx2 = H.dx2;
-                L0.dy2 = H.dy2;
-                re = b - apply_at(L0, H.coef, H.x, cell_of(nx, H.ny, g));
-            }
-            if constexpr (KEEP == PCG_KEEP_ALL) x[e] = H.warm ? __ldcg(H.x + g) : 0.0;
-            else if (!H.warm) x[e] = 0.0;
-            const double ze = H.inv_diag[g] * re;
-            r[e] = re;
-            ap[e] = ze;
-            if constexpr (MODE != PCG_ONE) H.z[g] = ze;
-            bufs[t] = b * b;
-            bufs[LEAF_PAD + t] = re * ze;
+    for (int e = tid; e < own; e += PCG_THREADS) {
+        const int g = s0 + e;
+        double re = H.rhs[g] * H.mask[g];
+        if (H.warm) {
+            HLevel L0;
+            L0.mask = H.mask;
+            L0.Ku = const_cast<double*>(H.Ku);
+            L0.Kv = const_cast<double*>(H.Kv);
+            L0.dx2 = H.dx2;
+            L0.dy2 = H.dy2;
+            re = re - apply_at(L0, H.coef, H.x, cell_of(nx, H.ny, g));
         }
-        __syncwarp();
-        const double2 sums = leaf_sums(bufs, bufs + LEAF_PAD, len);
-        if (lane == 0) {
-            leafs[0][H.leaf_slot[L]] = sums.x;
-            leafs[1][H.leaf_slot[L]] = sums.y;
-        }
-        __syncwarp();
+        if constexpr (KEEP == PCG_KEEP_ALL) x[e] = H.warm ? __ldcg(H.x + g) : 0.0;
+        else if (!H.warm) x[e] = 0.0;
+        const double ze = H.inv_diag[g] * re;
+        r[e] = re;
+        ap[e] = ze;
+        if constexpr (MODE != PCG_ONE) H.z[g] = ze;
     }
+    __syncthreads();
+    leaf_group_sums(nlf, lstart, lslot, [&](int e) {
+        const double b = H.rhs[s0 + e] * H.mask[s0 + e];
+        return make_double2(b * b, r[e] * ap[e]);
+    }, leafs[0], leafs[1]);
     ok = pcg_sync<MODE>(H);
     if (ok) {
         const double* lv[2] = {leafs[0], leafs[1]};
@@ -194,45 +242,105 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
         }
         for (int it = 1; it <= H.max_iter; ++it) {
             __syncthreads();
-            for (int L = lf0 + warp; L < lf1; L += PCG_WARPS) {
-                const int st = H.leaf_start[L] - s0, len = H.leaf_start[L + 1] - s0 - st;
+            if constexpr (SPREAD) {
+                // four of a thread's cells together: all their loads, then the arithmetic and the
+                // stores (past the range's end a thread repeats the last cell and stores nothing)
+                for (int e0 = tid; e0 < own; e0 += 4 * PCG_THREADS) {
+                    double pe[4], de[4], dw[4], dn[4], ds[4], c_e[4], c_w[4], c_n[4], c_s[4], m[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int t = lane + 32 * q;
-                    if (t < len) {
-                        const int e = st + t, w = e + lead;
+                    for (int q = 0; q < 4; ++q) {
+                        const int eq = e0 + q * PCG_THREADS, e = eq < own ? eq : own - 1, w = e + lead;
                         const int fl = flag[e];
-                        const double m = (fl & 1) ? 1.0 : 0.0;
-                        double e_, w_, n_, s_;  // face coefficients east, west, north, south
+                        m[q] = (fl & 1) ? 1.0 : 0.0;
                         if constexpr (KEEP == PCG_KEEP_ALL) {
-                            e_ = ke[e];
-                            w_ = kw[e];
-                            n_ = kn[e];
-                            s_ = ks[e];
+                            c_e[q] = ke[e];
+                            c_w[q] = kw[e];
+                            c_n[q] = kn[e];
+                            c_s[q] = ks[e];
                         } else {
                             const int g = s0 + e;
-                            e_ = __ldg(H.Ku + g);
-                            w_ = __ldg(H.Ku + ((fl & 4) ? g + nx - 1 : g - 1));
-                            n_ = __ldg(H.Kv + g);
-                            s_ = __ldg(H.Kv + (g - nx < 0 ? g - nx + n : g - nx));
+                            c_e[q] = __ldg(H.Ku + g);
+                            c_w[q] = __ldg(H.Ku + ((fl & 4) ? g + nx - 1 : g - 1));
+                            c_n[q] = __ldg(H.Kv + g);
+                            c_s[q] = __ldg(H.Kv + (g - nx < 0 ? g - nx + n : g - nx));
                         }
+                        pe[q] = pw[w];
+                        de[q] = pw[(fl & 2) ? w + 1 - nx : w + 1];
+                        dw[q] = pw[(fl & 4) ? w - 1 + nx : w - 1];
+                        dn[q] = pw[north(w)];
+                        ds[q] = pw[south(w)];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int e = e0 + q * PCG_THREADS;
+                        if (e >= own) break;
                         // VarOperator.apply (solvers_var.py:47-53); p is 0 on dry cells
                         // (z = r / diag, and r is a masked difference), so p mask is p
-                        const double pe = pw[w];
-                        const double fx = e_ * (pw[(fl & 2) ? w + 1 - nx : w + 1] - pe);
-                        const double fxw = w_ * (pe - pw[(fl & 4) ? w - 1 + nx : w - 1]);
-                        const double fy = n_ * (pw[north(w)] - pe);
-                        const double fys = s_ * (pe - pw[south(w)]);
+                        const double fx = c_e[q] * (de[q] - pe[q]);
+                        const double fxw = c_w[q] * (pe[q] - dw[q]);
+                        const double fy = c_n[q] * (dn[q] - pe[q]);
+                        const double fys = c_s[q] * (pe[q] - ds[q]);
                         const double lap = (fx - fxw) / H.dx2 + (fy - fys) / H.dy2;
-                        const double a = (pe - H.coef * lap) * m + pe * (1.0 - m);
-                        ap[e] = a;
-                        bufs[t] = pe * a;
+                        ap[e] = (pe[q] - H.coef * lap) * m[q] + pe[q] * (1.0 - m[q]);
                     }
                 }
-                __syncwarp();
-                const double2 sums = leaf_sums(bufs, bufs, len);
-                if (lane == 0) leafs[2][H.leaf_slot[L]] = sums.x;
-                __syncwarp();
+                __syncthreads();
+                leaf_group_sums(nlf, lstart, lslot, [&](int e) { return make_double2(pw[e + lead] * ap[e], 0.0); }, leafs[2],
+                                nullptr);
+            } else {
+                for (int L = warp; L < nlf; L += PCG_WARPS) {
+                    const int st = lstart[L], len = lstart[L + 1] - st;
+                    // a lane's four cells together: all their loads, then the arithmetic, then
+                    // the stores (past the leaf's end a lane repeats its last cell and stores nothing)
+                    double pe[4], de[4], dw[4], dn[4], ds[4], c_e[4], c_w[4], c_n[4], c_s[4], m[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int t = lane + 32 * q, e = st + (t < len ? t : len - 1), w = e + lead;
+                        const int fl = flag[e];
+                        m[q] = (fl & 1) ? 1.0 : 0.0;
+                        if constexpr (KEEP == PCG_KEEP_ALL) {
+                            c_e[q] = ke[e];
+                            c_w[q] = kw[e];
+                            c_n[q] = kn[e];
+                            c_s[q] = ks[e];
+                        } else {
+                            const int g = s0 + e;
+                            c_e[q] = __ldg(H.Ku + g);
+                            c_w[q] = __ldg(H.Ku + ((fl & 4) ? g + nx - 1 : g - 1));
+                            c_n[q] = __ldg(H.Kv + g);
+                            c_s[q] = __ldg(H.Kv + (g - nx < 0 ? g - nx + n : g - nx));
+                        }
+                        pe[q] = pw[w];
+                        de[q] = pw[(fl & 2) ? w + 1 - nx : w + 1];
+                        dw[q] = pw[(fl & 4) ? w - 1 + nx : w - 1];
+                        dn[q] = pw[north(w)];
+                        ds[q] = pw[south(w)];
+                    }
+                    double av[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        // VarOperator.apply (solvers_var.py:47-53); p is 0 on dry cells
+                        // (z = r / diag, and r is a masked difference), so p mask is p
+                        const double fx = c_e[q] * (de[q] - pe[q]);
+                        const double fxw = c_w[q] * (pe[q] - dw[q]);
+                        const double fy = c_n[q] * (dn[q] - pe[q]);
+                        const double fys = c_s[q] * (pe[q] - ds[q]);
+                        const double lap = (fx - fxw) / H.dx2 + (fy - fys) / H.dy2;
+                        av[q] = (pe[q] - H.coef * lap) * m[q] + pe[q] * (1.0 - m[q]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int t = lane + 32 * q;
+                        if (t < len) {
+                            ap[st + t] = av[q];
+                            bufs[t] = pe[q] * av[q];
+                        }
+                    }
+                    __syncwarp();
+                    const double2 sums = leaf_sums(bufs, bufs, len);
+                    if (lane == 0) leafs[2][lslot[L]] = sums.x;
+                    __syncwarp();
+                }
             }
             ok = pcg_sync<MODE>(H);
             if (!ok) break;
@@ -242,36 +350,77 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
                 pcg_fold<MODE, 1>(H, lv, scratch, pap);
             }
             const double alpha = rz / pap[0];
-            for (int L = lf0 + warp; L < lf1; L += PCG_WARPS) {
-                const int st = H.leaf_start[L] - s0, len = H.leaf_start[L + 1] - s0 - st;
+            if constexpr (SPREAD) {
+                for (int e0 = tid; e0 < own; e0 += 4 * PCG_THREADS) {
+                    double xe[4], re[4], pe[4], ae[4], di[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int t = lane + 32 * q;
-                    if (t < len) {
-                        const int e = st + t;
-                        const double xe = x[e] + alpha * pw[e + lead];
-                        const double re = r[e] - alpha * ap[e];
-                        x[e] = xe;
-                        r[e] = re;
-                        double d;
-                        if constexpr (KEEP == PCG_KEEP_ALL) d = id[e];
-                        else d = __ldg(H.inv_diag + s0 + e);
-                        const double ze = d * re;
+                    for (int q = 0; q < 4; ++q) {
+                        const int eq = e0 + q * PCG_THREADS, e = eq < own ? eq : own - 1;
+                        xe[q] = x[e];
+                        re[q] = r[e];
+                        pe[q] = pw[e + lead];
+                        ae[q] = ap[e];
+                        if constexpr (KEEP == PCG_KEEP_ALL) di[q] = id[e];
+                        else di[q] = __ldg(H.inv_diag + s0 + e);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int e = e0 + q * PCG_THREADS;
+                        if (e >= own) break;
+                        const double rn = re[q] - alpha * ae[q];
+                        const double ze = di[q] * rn;
+                        x[e] = xe[q] + alpha * pe[q];
+                        r[e] = rn;
                         ap[e] = ze;  // z, until the next A p
                         // the rows a neighbouring range reads
                         if constexpr (MODE != PCG_ONE)
                             if (e < nx || e >= own - nx) H.z[s0 + e] = ze;
-                        bufs[t] = re * re;
-                        bufs[LEAF_PAD + t] = re * ze;
                     }
                 }
-                __syncwarp();
-                const double2 sums = leaf_sums(bufs, bufs + LEAF_PAD, len);
-                if (lane == 0) {
-                    leafs[0][H.leaf_slot[L]] = sums.x;
-                    leafs[1][H.leaf_slot[L]] = sums.y;
+                __syncthreads();
+                leaf_group_sums(nlf, lstart, lslot, [&](int e) {
+                    const double re = r[e];
+                    return make_double2(re * re, re * ap[e]);
+                }, leafs[0], leafs[1]);
+            } else {
+                for (int L = warp; L < nlf; L += PCG_WARPS) {
+                    const int st = lstart[L], len = lstart[L + 1] - st;
+                    double xe[4], re[4], pe[4], ae[4], di[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int t = lane + 32 * q, e = st + (t < len ? t : len - 1);
+                        xe[q] = x[e];
+                        re[q] = r[e];
+                        pe[q] = pw[e + lead];
+                        ae[q] = ap[e];
+                        if constexpr (KEEP == PCG_KEEP_ALL) di[q] = id[e];
+                        else di[q] = __ldg(H.inv_diag + s0 + e);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int t = lane + 32 * q;
+                        if (t < len) {
+                            const int e = st + t;
+                            const double rn = re[q] - alpha * ae[q];
+                            const double ze = di[q] * rn;
+                            x[e] = xe[q] + alpha * pe[q];
+                            r[e] = rn;
+                            ap[e] = ze;  // z, until the next A p
+                            // the rows a neighbouring range reads
+                            if constexpr (MODE != PCG_ONE)
+                                if (e < nx || e >= own - nx) H.z[s0 + e] = ze;
+                            bufs[t] = rn * rn;
+                            bufs[LEAF_PAD + t] = rn * ze;
+                        }
+                    }
+                    __syncwarp();
+                    const double2 sums = leaf_sums(bufs, bufs + LEAF_PAD, len);
+                    if (lane == 0) {
+                        leafs[0][lslot[L]] = sums.x;
+                        leafs[1][lslot[L]] = sums.y;
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
             ok = pcg_sync<MODE>(H);
             if (!ok) break;
@@ -287,14 +436,28 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
             }
             const double beta = f[1] / rz;
             rz = f[1];
-            for (int w = tid; w < H.window_of(own); w += PCG_THREADS) {
-                const int e = w - lead;
-                int g = s0 + e;
-                if (g < 0) g += n;
-                if (g >= n) g -= n;
-                const double ze = (e >= 0 && e < own) ? ap[e] : __ldcg(H.z + g);
-                pw[w] = ze + beta * pw[w];
+            // the rows outside the range first: their z is on its way while the range's own is used
+            if constexpr (MODE != PCG_ONE) {
+                constexpr int K = 4;
+                for (int h0 = tid; h0 < 2 * nx; h0 += K * PCG_THREADS) {
+                    double z[K];
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const int h = h0 + k * PCG_THREADS;
+                        int g = h < nx ? s0 - nx + h : s0 + own + h - nx;
+                        if (g < 0) g += n;
+                        if (g >= n) g -= n;
+                        z[k] = h < 2 * nx ? __ldcg(H.z + g) : 0.0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const int h = h0 + k * PCG_THREADS, w = h < nx ? h : own + h;
+                        if (h < 2 * nx) pw[w] = z[k] + beta * pw[w];
+                    }
+                }
             }
+#pragma unroll 4
+            for (int e = tid; e < own; e += PCG_THREADS) pw[e + lead] = ap[e] + beta * pw[e + lead];
         }
     }
     if constexpr (KEEP == PCG_KEEP_ALL) {
@@ -319,19 +482,17 @@ typedef void (*PcgKernel)(const PcgParams);
 
 static PcgKernel pcg_kernel(int mode, int keep) {
     if (mode == PCG_ONE) return k_helm_pcg<PCG_ONE, PCG_KEEP_ALL>;
-    if (mode == PCG_CLUSTER)
-        return keep == PCG_KEEP_ALL ? (PcgKernel)k_helm_pcg<PCG_CLUSTER, PCG_KEEP_ALL>
-                                    : (PcgKernel)k_helm_pcg<PCG_CLUSTER, PCG_KEEP_RA>;
+    if (mode == PCG_CLUSTER) return k_helm_pcg<PCG_CLUSTER, PCG_KEEP_ALL>;
     return keep == PCG_KEEP_ALL  ? (PcgKernel)k_helm_pcg<PCG_GRID, PCG_KEEP_ALL>
            : keep == PCG_KEEP_RA ? (PcgKernel)k_helm_pcg<PCG_GRID, PCG_KEEP_RA>
                                  : (PcgKernel)k_helm_pcg<PCG_GRID, PCG_KEEP_P>;
 }
 
-// shared memory of a launch whose largest range has `own` cells and window `window`
-static size_t pcg_smem(int keep, size_t own, size_t window) {
-    const size_t doubles = (size_t)PCG_WARPS * 2 * LEAF_PAD + 3 * 128 + window +
+// shared memory of a launch whose largest range has `own` cells, window `window` and `leaves` leaves
+static size_t pcg_smem(int mode, int keep, size_t own, size_t window, size_t leaves) {
+    const size_t doubles = (mode == PCG_GRID ? 0 : PCG_WARPS * 2 * LEAF_PAD) + 3 * 128 + window +
                            (keep == PCG_KEEP_ALL ? 8 * own : (keep == PCG_KEEP_RA ? 2 * own : 0));
-    return doubles * sizeof(double) + ((own + 15) & ~(size_t)15);
+    return doubles * sizeof(double) + 2 * (leaves + 1) * sizeof(int) + ((own + 15) & ~(size_t)15);
 }
 
 // the kernels' shared-memory allowance on this device; it only grows, so every
@@ -356,16 +517,17 @@ static bool pcg_try(int mode, int keep, int ncta, const std::vector<int>& leaves
                     PcgPlan& plan) {
     const int n_leaves = (int)leaves.size() - 1;
     if (ncta > n_leaves) return false;
-    int own = 0;
+    int own = 0, most = 0;
     for (int c = 0; c < ncta; ++c) {
         const int a = (int)((long long)n_leaves * c / ncta), b = (int)((long long)n_leaves * (c + 1) / ncta);
         own = std::max(own, leaves[b] - leaves[a]);
+        most = std::max(most, b - a);
     }
     const int n = leaves.back();
     const int window = mode == PCG_ONE ? n : own + 2 * nx;
     // a window must not meet itself: its rows above and below belong to other ranges
     if (mode != PCG_ONE && window > n) return false;
-    const size_t smem = pcg_smem(keep, (size_t)own, (size_t)window);
+    const size_t smem = pcg_smem(mode, keep, (size_t)own, (size_t)window, (size_t)most);
     cudaFuncAttributes fa{};
     PcgKernel k = pcg_kernel(mode, keep);
     if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) {
@@ -373,7 +535,7 @@ static bool pcg_try(int mode, int keep, int ncta, const std::vector<int>& leaves
         return false;
     }
     if (smem + fa.sharedSizeBytes > optin || !pcg_allow(k, smem, dev)) return false;
-    plan = PcgPlan{mode, keep, ncta, own, window, smem};
+    plan = PcgPlan{mode, keep, ncta, own, window, most, smem};
     return true;
 }
 
@@ -387,28 +549,26 @@ bool pcg_plan(const std::vector<int>& leaves, int n_slots, int nx, PcgPlan& plan
         return true;
     if (n <= PCG_CLUSTER_CELLS) {
         for (int c : {16, 8}) {
-            for (int keep : {PCG_KEEP_ALL, PCG_KEEP_RA}) {
-                if (!pcg_try(PCG_CLUSTER, keep, c, leaves, nx, dev, (size_t)optin, plan)) continue;
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3(c);
-                cfg.blockDim = dim3(PCG_THREADS);
-                cfg.dynamicSmemBytes = plan.smem;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = (unsigned)c;
-                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                int clusters = 0;
-                if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)pcg_kernel(PCG_CLUSTER, keep), &cfg) ==
-                        cudaSuccess && clusters >= 1)
-                    return true;
-                cudaGetLastError();
-            }
+            if (!pcg_try(PCG_CLUSTER, PCG_KEEP_ALL, c, leaves, nx, dev, (size_t)optin, plan)) continue;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(c);
+            cfg.blockDim = dim3(PCG_THREADS);
+            cfg.dynamicSmemBytes = plan.smem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)c;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)pcg_kernel(PCG_CLUSTER, PCG_KEEP_ALL), &cfg) ==
+                    cudaSuccess && clusters >= 1)
+                return true;
+            cudaGetLastError();
         }
     }
     for (int keep : {PCG_KEEP_ALL, PCG_KEEP_RA, PCG_KEEP_P})
-        if (pcg_try(PCG_GRID, keep, sms, leaves, nx, dev, (size_t)optin, plan)) {
+        if (pcg_try(PCG_GRID, keep, std::min(sms, (int)leaves.size() - 1), leaves, nx, dev, (size_t)optin, plan)) {
             int per_sm = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_kernel(PCG_GRID, keep), PCG_THREADS, plan.smem);
             if (per_sm >= 1) return true;

@@ -25,6 +25,7 @@ struct PcgParams {
     const int *leaf_start, *leaf_slot;
     double *leafA, *leafB, *leafC;
     int own_max, window;  // cells of the largest range, and of its window of p
+    int leaves_max;       // leaves of the range that has most
     int lead;             // window cells before the range (the row below): nx, or 0 for one CTA
     unsigned long long* bar_count;
     int* status;
@@ -35,7 +36,7 @@ struct PcgParams {
 };
 
 struct PcgPlan {
-    int mode, keep, ncta, own_max, window;
+    int mode, keep, ncta, own_max, window, leaves_max;
     size_t smem;
 };
 

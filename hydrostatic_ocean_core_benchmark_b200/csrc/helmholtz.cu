@@ -1633,6 +1633,7 @@ int HelmSolver::solve(const double* rhs, double* x, cudaStream_t s, std::string&
         P.leafC = hp_.leafC;
         P.own_max = pcg_plan_.own_max;
         P.window = pcg_plan_.window;
+        P.leaves_max = pcg_plan_.leaves_max;
         P.lead = pcg_plan_.mode == PCG_ONE ? 0 : L.nx;
         P.bar_count = hp_.bar_count;
         P.status = hp_.status;
