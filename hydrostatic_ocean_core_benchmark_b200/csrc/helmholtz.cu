@@ -34,43 +34,21 @@
 
 namespace oc {
 
-static constexpr int kCoarseCells = 1024;
-// fine-level tiles: interior TX x TY cells plus a halo of HALO cells, enough
-// for four red-black half-sweeps and one residual on a shrinking region
-static constexpr int HALO = 5;
-template <int TX_, int TY_>
-struct TileShape {
-    static constexpr int TX = TX_, TY = TY_;
-    static constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO, RN = RW * RH;
-};
-using Tile32 = TileShape<32, 32>;
-using Tile3216 = TileShape<32, 16>;
-using Tile16 = TileShape<16, 16>;
-using Tile8 = TileShape<8, 8>;
-using TileWide = TileShape<128, 16>;  // level 0 of large grids: one tile per CTA, one NumPy leaf per row
-// per-level tile shape codes (HLevel::shape)
-enum { SHAPE_32 = 0, SHAPE_3216 = 1, SHAPE_16 = 2, SHAPE_8 = 3, SHAPE_WIDE = 4 };
+// grids of at most this many cells run their multigrid solve wholly in one CTA
+static constexpr int kOneCtaCells = 2560;
+static constexpr int kSolveThreads = 512;  // threads of a solve's CTA
+static constexpr int kLeafRow = 136;  // a warp's row of 128 values, the next row in other banks
 
 // ------------------------------------------------------------------ barrier
 // the bounded grid barrier of grid_barrier.cuh on the solver's counter and status
 __device__ __forceinline__ void grid_sync_begin(const HelmParams& H) { grid_sync_begin(H.status); }
 
 __device__ __forceinline__ bool grid_sync(const HelmParams& H) {
+    if (s_grid.ncta == 1) {  // a solve in one CTA waits for nobody
+        __syncthreads();
+        return true;
+    }
     return grid_sync(H.bar_count, H.status, (unsigned)s_grid.ncta, H.wait_cycles);
-}
-
-// ------------------------------------------------------------------ asynchronous copies
-// cp.async into shared memory without a register round trip, so a thread's
-// copies are all in flight at once. The 8-byte form goes through L1, which is not
-// coherent with other SMs' writes, so it serves only arrays that stay constant
-// during the solve (the level coefficients); b and x, which other CTAs of the
-// launch write, are read through L2 (__ldcg).
-__device__ __forceinline__ void cpa_ca8(double* sdst, const double* gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cpa_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
 // ------------------------------------------------------------------ level operators
@@ -227,551 +205,167 @@ __device__ __forceinline__ double fold_sum(const HelmParams& H, const double* le
     return fold_blocks(H, leaf, broot, sm, ok);
 }
 
-// ------------------------------------------------------------------ tiled multigrid
-// A fine level is processed tile by tile in shared memory. The down phase loads
-// x, b and the coefficients of a tile plus a HALO-wide ring, runs the two
-// pre-smoothing sweeps (four red-black half-sweeps) on a region that shrinks by
-// one cell per half-sweep, and forms the restricted residual of the interior;
-// the up phase adds the prolonged coarse correction and runs the two reverse
-// post-smoothing sweeps the same way. Every value in the valid region is the
-// one the whole-grid sweep produces (same inputs, same operations), so the
-// result is identical to sweeping the level with a grid barrier between
-// half-sweeps, with two barriers per level instead of nine.
-__device__ __forceinline__ int wrap_any(int i, int n) {
-    if (i >= 0 && i < n) return i;
-    if (i < 0 && i + n >= 0) return i + n;
-    if (i >= n && i - n < n) return i - n;
-    const int r = i % n;
-    return r < 0 ? r + n : r;
-}
+}  // namespace oc
 
-struct TileRefs {
-    double *x, *b, *ku, *kv, *id, *m;
-};
+#include "helm_mg.cuh"
 
-template <class S>
-__device__ __forceinline__ TileRefs tile_refs(double* base) {
-    TileRefs t;
-    t.x = base;
-    t.b = base + S::RN;
-    t.ku = base + 2 * S::RN;
-    t.kv = base + 3 * S::RN;
-    t.id = base + 4 * S::RN;
-    t.m = base + 5 * S::RN;
-    return t;
-}
+namespace oc {
 
-// load a tile region of level L whose interior starts at (i0, j0); x from xin
-// (or zero), plus the coarse correction e * mask when C is given
-// (with `coef` false the coefficients ku, kv, id, m are already in place).
-// A thread gathers CH of its cells at a time into registers and only then
-// writes them to shared memory: the tile arrays reach here as plain pointers,
-// so the compiler may not move a later cell's global loads above an earlier
-// cell's stores, and cell by cell the loads of a thread would run one L2 round
-// trip after another.
-template <class S, int CH, bool COEF>
-__device__ __forceinline__ void tile_load_chunks(const HLevel& L, int i0, int j0, const double* xin,
-                                                 const HLevel* C, TileRefs t) {
-    const int nt = blockDim.x;
-    for (int base = threadIdx.x; base < S::RN; base += CH * nt) {
-        double xv[CH], bv[CH];
-#pragma unroll
-        for (int q = 0; q < CH; ++q) {
-            const int r = base + q * nt;
-            xv[q] = bv[q] = 0.0;
-            if (r < S::RN) {
-                const int rj = r / S::RW, ri = r - rj * S::RW;
-                const int gi = wrap_any(i0 - HALO + ri, L.nx), gj = wrap_any(j0 - HALO + rj, L.ny);
-                const int g = gj * L.nx + gi;
-                if (COEF) {
-                    // the coefficients, constant during the solve: asynchronous copies
-                    cpa_ca8(t.ku + r, L.Ku + g);
-                    cpa_ca8(t.kv + r, L.Kv + g);
-                    cpa_ca8(t.id + r, L.inv_diag + g);
-                    cpa_ca8(t.m + r, L.mask + g);
-                }
-                double x = xin ? __ldcg(xin + g) : 0.0;
-                if (C) x = x + __ldcg(C->x + (gj >> 1) * C->nx + (gi >> 1)) * (COEF ? L.mask[g] : t.m[r]);
-                xv[q] = x;
-                bv[q] = __ldcg(L.b + g);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CH; ++q) {
-            const int r = base + q * nt;
-            if (r < S::RN) {
-                t.x[r] = xv[q];
-                t.b[r] = bv[q];
-            }
-        }
-    }
-    if (COEF) cpa_wait_all();
-}
-
-template <class S>
-__device__ void tile_load(const HLevel& L, int i0, int j0, const double* xin, const HLevel* C,
-                          TileRefs t, bool coef = true) {
-    if (coef)
-        tile_load_chunks<S, 2, true>(L, i0, j0, xin, C, t);
-    else
-        tile_load_chunks<S, 4, false>(L, i0, j0, xin, C, t);
-    __syncthreads();
-}
-
-// Level 0's coefficients stay in shared memory for a whole solve when every
-// level-0 tile has a CTA of its own (H.persist0): the first RN x 4 doubles hold
-// the CTA's tile's ku, kv, id and m, and the tile phases of level 0 load only x
-// and b. Everything else works above them.
-template <class S>
-__device__ __forceinline__ TileRefs tile_refs_persist(double* persist, double* work) {
-    TileRefs t;
-    t.ku = persist;
-    t.kv = persist + S::RN;
-    t.id = persist + 2 * S::RN;
-    t.m = persist + 3 * S::RN;
-    t.x = work;
-    t.b = work + S::RN;
-    return t;
-}
-
-// With a CTA of its own for every level-0 tile, the tiles go to the last CTAs
-// (tile = CTA - (CTAs - tiles)), so CTA 0, which runs the coarse levels, keeps
-// its persistent region for their coefficients (H.coarse_persist).
-__device__ __forceinline__ int level0_tile_of_cta(int tiles) { return s_grid.cta - (s_grid.ncta - tiles); }
-
-__device__ void persist_level0(const HelmParams& H, double* persist) {
-    using S = TileWide;
+// ------------------------------------------------------------------ multigrid in one CTA
+// The stationary multigrid of a grid of at most kOneCtaCells cells by one CTA: every
+// level's coefficients, x and b stay in its shared memory for the solve, all
+// barriers are the CTA's, and nothing but the right-hand side and the solution
+// crosses global memory. Same operations and sums as the grid-wide form. Squares are
+// formed cell by cell into the scratch, in the grid's order, and summed there by
+// leaves, four leaves per warp.
+__device__ __noinline__ void helm_one_cta(int& iters, int& conv) {
+    const HelmParams& H = s_helm;
     const HLevel& L = H.lv[0];
-    const int tx = (L.nx + S::TX - 1) / S::TX;
-    const int tile = level0_tile_of_cta(tx * ((L.ny + S::TY - 1) / S::TY));
-    if (tile < 0) return;
-    const int i0 = (tile % tx) * S::TX, j0 = (tile / tx) * S::TY;
-    for (int r = threadIdx.x; r < S::RN; r += blockDim.x) {
-        const int rj = r / S::RW, ri = r - rj * S::RW;
-        const int g = wrap_any(j0 - HALO + rj, L.ny) * L.nx + wrap_any(i0 - HALO + ri, L.nx);
-        persist[r] = L.Ku[g];
-        persist[S::RN + r] = L.Kv[g];
-        persist[2 * S::RN + r] = L.inv_diag[g];
-        persist[3 * S::RN + r] = L.mask[g];
+    coarse_tab_init(0, -1);
+    const CoarseTab& T = s_ct[0];
+    const bool unit = H.unit_mask != 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* sq = smem_all + s_cres;                    // the squares, after the levels
+    double* slots = sq + T.n;                          // leaf sums, then the leaves' starts and slots
+    int* start = reinterpret_cast<int*>(slots + H.n_slots);
+    int* slot = start + H.n_leaves + 1;
+    coarse_coef_load();
+    for (int t = threadIdx.x; t < H.n_slots; t += kSolveThreads) slots[t] = 0.0;
+    for (int t = threadIdx.x; t <= H.n_leaves; t += kSolveThreads) {
+        start[t] = H.leaf_start[t];
+        if (t < H.n_leaves) slot[t] = H.leaf_slot[t];
     }
-    __syncthreads();
-}
-
-// one red-black half-sweep of colour `colour` on the region ring >= SHRINK. On
-// even-sized levels the colour of a region cell follows from its region
-// coordinates (a wrap by an even size keeps the parity), so only the cells of
-// that colour are visited; odd-sized levels test each cell.
-template <class S, int SHRINK>
-__device__ void tile_half_sweep_t(const HLevel& L, int i0, int j0, TileRefs t, int colour) {
-    constexpr int RW = S::RW, RH = S::RH;
-    constexpr int ROWS = RH - 2 * SHRINK, COLS = RW - 2 * SHRINK;
-    constexpr int HALF = (COLS + 1) / 2;
-    const bool even = ((L.nx | L.ny) & 1) == 0;
-    if (even) {
-        for (int q = threadIdx.x; q < ROWS * HALF; q += blockDim.x) {
-            const int rj = SHRINK + q / HALF;
-            const int ri = SHRINK + ((colour - i0 - j0 - rj - SHRINK) & 1) + 2 * (q % HALF);
-            if (ri >= RW - SHRINK) continue;
-            const int r = rj * RW + ri;
-            const double nb = L.cx * (t.ku[r] * t.x[r + 1] + t.ku[r - 1] * t.x[r - 1]) +
-                              L.cy * (t.kv[r] * t.x[r + RW] + t.kv[r - RW] * t.x[r - RW]);
-            t.x[r] = t.id[r] * (t.b[r] + nb) * t.m[r];
-        }
-    } else {
-        for (int r = threadIdx.x; r < S::RN; r += blockDim.x) {
-            const int rj = r / RW, ri = r - rj * RW;
-            if (ri < SHRINK || ri >= RW - SHRINK || rj < SHRINK || rj >= RH - SHRINK) continue;
-            const int gi = wrap_any(i0 - HALO + ri, L.nx), gj = wrap_any(j0 - HALO + rj, L.ny);
-            if (((gi + gj) & 1) != colour) continue;
-            const double nb = L.cx * (t.ku[r] * t.x[r + 1] + t.ku[r - 1] * t.x[r - 1]) +
-                              L.cy * (t.kv[r] * t.x[r + RW] + t.kv[r - RW] * t.x[r - RW]);
-            t.x[r] = t.id[r] * (t.b[r] + nb) * t.m[r];
-        }
-    }
-    __syncthreads();
-}
-
-// four half-sweeps with colours c0, 1 - c0, c0, 1 - c0 on a region shrinking by one ring each
-template <class S>
-__device__ __forceinline__ void tile_four_half_sweeps(const HLevel& L, int i0, int j0, TileRefs t, int c0) {
-    tile_half_sweep_t<S, 1>(L, i0, j0, t, c0);
-    tile_half_sweep_t<S, 2>(L, i0, j0, t, 1 - c0);
-    tile_half_sweep_t<S, 3>(L, i0, j0, t, c0);
-    tile_half_sweep_t<S, 4>(L, i0, j0, t, 1 - c0);
-}
-
-// (b - A x) * mask at region cell r (VarOperator.apply, solvers_var.py:47-53)
-template <class S>
-__device__ __forceinline__ double tile_residual(const HLevel& L, double coef, TileRefs t, int r) {
-    constexpr int RW = S::RW;
-    const double m = t.m[r];
-    const double xm = t.x[r] * m;
-    const double xe = t.x[r + 1] * t.m[r + 1];
-    const double xw = t.x[r - 1] * t.m[r - 1];
-    const double xn = t.x[r + RW] * t.m[r + RW];
-    const double xs = t.x[r - RW] * t.m[r - RW];
-    const double fx = t.ku[r] * (xe - xm);
-    const double fxw = t.ku[r - 1] * (xm - xw);
-    const double fy = t.kv[r] * (xn - xm);
-    const double fys = t.kv[r - RW] * (xm - xs);
-    const double lap = (fx - fxw) / L.dx2 + (fy - fys) / L.dy2;
-    const double ax = (xm - coef * lap) * m + xm * (1.0 - m);
-    return (t.b[r] - ax) * m;
-}
-
-template <class S>
-__device__ void tile_store_x(const HLevel& L, int i0, int j0, TileRefs t, double* xout) {
-    for (int r = threadIdx.x; r < S::TX * S::TY; r += blockDim.x) {
-        const int cj = r / S::TX, ci = r - cj * S::TX;
-        const int gi = i0 + ci, gj = j0 + cj;
-        if (gi >= L.nx || gj >= L.ny) continue;
-        xout[gj * L.nx + gi] = t.x[(cj + HALO) * S::RW + ci + HALO];
-    }
-}
-
-// down phase of level l: pre-smoothing, restricted residual into level l+1
-// (solvers_var.py:141-147); x of level l+1 starts at zero implicitly
-template <class S>
-__device__ void mg_down(const HelmParams& H, int l, const double* xin, double* xout, double* smem,
-                        double* persist = nullptr) {
-    const HLevel& L = H.lv[l];
-    const HLevel& C = H.lv[l + 1];
-    const int tx = (L.nx + S::TX - 1) / S::TX, ty = (L.ny + S::TY - 1) / S::TY;
-    const bool keep = persist != nullptr;
-    TileRefs t = keep ? tile_refs_persist<S>(persist, smem) : tile_refs<S>(smem);
-    for (int tile = keep ? level0_tile_of_cta(tx * ty) : s_grid.cta; tile < tx * ty; tile += s_grid.ncta) {
-        if (tile < 0) continue;  // CTA-uniform: this CTA holds no persistent tile
-        const int i0 = (tile % tx) * S::TX, j0 = (tile / tx) * S::TY;
-        tile_load<S>(L, i0, j0, xin, nullptr, t, !keep);
-        tile_four_half_sweeps<S>(L, i0, j0, t, 0);
-        constexpr int NC = (S::TX / 2) * (S::TY / 2);  // coarse cells of the tile
-        if constexpr (4 * NC <= 1024 && (4 * NC) % 32 == 0 && S::TX != TileWide::TX) {
-            // four lanes per coarse cell, one child residual each, summed by the
-            // first of them in the order a + b + c + d (the loop bound is a
-            // multiple of 32, so whole warps take part in the shuffles)
-            for (int q = threadIdx.x; q < 4 * NC; q += blockDim.x) {
-                const int r = q >> 2, child = q & 3;
-                const int cj = r / (S::TX / 2), ci = r - cj * (S::TX / 2);
-                const int I = i0 / 2 + ci, J = j0 / 2 + cj;
-                const int rr = (HALO + 2 * cj + (child >> 1)) * S::RW + HALO + 2 * ci + (child & 1);
-                const double val = tile_residual<S>(L, H.coef, t, rr);
-                const double b = __shfl_down_sync(0xffffffffu, val, 1);
-                const double c = __shfl_down_sync(0xffffffffu, val, 2);
-                const double d = __shfl_down_sync(0xffffffffu, val, 3);
-                if (child == 0 && I < C.nx && J < C.ny) C.b[J * C.nx + I] = 0.25 * (val + b + c + d);
-            }
-        } else {
-            for (int r = threadIdx.x; r < NC; r += blockDim.x) {
-                const int cj = r / (S::TX / 2), ci = r - cj * (S::TX / 2);
-                const int I = i0 / 2 + ci, J = j0 / 2 + cj;
-                if (I >= C.nx || J >= C.ny) continue;
-                const int r00 = (HALO + 2 * cj) * S::RW + HALO + 2 * ci;
-                const double a = tile_residual<S>(L, H.coef, t, r00);
-                const double b = tile_residual<S>(L, H.coef, t, r00 + 1);
-                const double c = tile_residual<S>(L, H.coef, t, r00 + S::RW);
-                const double d = tile_residual<S>(L, H.coef, t, r00 + S::RW + 1);
-                C.b[J * C.nx + I] = 0.25 * (a + b + c + d);
-            }
-        }
-        tile_store_x<S>(L, i0, j0, t, xout);
-        __syncthreads();
-    }
-}
-
-// up phase of level l: x + prolong(x_coarse) * mask, then the two reverse sweeps
-// (solvers_var.py:148-150). With `leaves`, level 0's tiles are one NumPy leaf
-// per interior row (128 cells starting at a multiple of 128): after the sweeps
-// every interior cell and its four neighbours hold the new x, so each warp forms
-// the squared residual (b - A x)^2 of one row and its leaf sum in NumPy's order
-// -- the per-cycle residual norm without another pass over the grid.
-template <class S>
-__device__ void mg_up(const HelmParams& H, int l, const double* xin, const HLevel& C, double* xout,
-                      double* smem, double* leaves, double* persist = nullptr) {
-    const HLevel& L = H.lv[l];
-    const int tx = (L.nx + S::TX - 1) / S::TX, ty = (L.ny + S::TY - 1) / S::TY;
-    const bool keep = persist != nullptr;
-    TileRefs t = keep ? tile_refs_persist<S>(persist, smem) : tile_refs<S>(smem);
-    for (int tile = keep ? level0_tile_of_cta(tx * ty) : s_grid.cta; tile < tx * ty; tile += s_grid.ncta) {
-        if (tile < 0) continue;  // CTA-uniform: this CTA holds no persistent tile
-        const int i0 = (tile % tx) * S::TX, j0 = (tile / tx) * S::TY;
-        tile_load<S>(L, i0, j0, xin, &C, t, !keep);
-        tile_four_half_sweeps<S>(L, i0, j0, t, 1);
-        tile_store_x<S>(L, i0, j0, t, xout);
-        if constexpr (S::TX == 128) {
-            if (leaves) {
-                const int lane = threadIdx.x & 31;
-                for (int cj = threadIdx.x >> 5; cj < S::TY; cj += blockDim.x >> 5) {
-                    if (j0 + cj >= L.ny) continue;  // warp-uniform
-                    double va[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const double d = tile_residual<S>(L, H.coef, t, (cj + HALO) * S::RW + HALO + lane + 32 * q);
-                        va[q] = d * d;
-                    }
-                    const double a = leaf_sum_warp(va, 128);
-                    if (lane == 0) leaves[((j0 + cj) * L.nx + i0) / 128] = a;
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// ---- coarse levels: all of them inside CTA 0, in shared memory
-struct CoarseRefs {
-    double *x, *b, *ku, *kv, *id, *m;
-};
-
-// the coarse levels' arrays take 6 x (sum of their cells) doubles; the restriction
-// scratch (one value per cell of the first coarse level) follows them
-__device__ __forceinline__ double* coarse_scratch(const HelmParams& H, double* base) {
-    int tot = 0;
-    for (int q = H.coarse_from; q < H.n_levels; ++q) tot += H.lv[q].n;
-    return base + 6 * tot;
-}
-
-// coef: where ku, kv, id and m live when they persist for the solve (CTA 0's
-// persistent region), else null (they follow x and b in `base`)
-__device__ __forceinline__ CoarseRefs coarse_refs(const HelmParams& H, double* base, int l,
-                                                  double* coef = nullptr) {
-    int off = 0, tot = 0;
-    for (int q = H.coarse_from; q < H.n_levels; ++q) {
-        if (q < l) off += H.lv[q].n;
-        tot += H.lv[q].n;
-    }
-    double* cb = coef ? coef : base + 2 * tot;
-    CoarseRefs c;
-    c.x = base + off;
-    c.b = base + tot + off;
-    c.ku = cb + off;
-    c.kv = cb + tot + off;
-    c.id = cb + 2 * tot + off;
-    c.m = cb + 3 * tot + off;
-    return c;
-}
-
-// the coarse levels' coefficients into `coef` (asynchronous copies; the caller
-// waits for them before its next CTA barrier)
-__device__ void coarse_coef_load(const HelmParams& H, double* coef, double* base) {
-    for (int l = H.coarse_from; l < H.n_levels; ++l) {
-        const HLevel& L = H.lv[l];
-        CoarseRefs s = coarse_refs(H, base, l, coef);
-        for (int e = threadIdx.x; e < L.n; e += blockDim.x) {
-            cpa_ca8(s.ku + e, L.Ku + e);
-            cpa_ca8(s.kv + e, L.Kv + e);
-            cpa_ca8(s.id + e, L.inv_diag + e);
-            cpa_ca8(s.m + e, L.mask + e);
-        }
-    }
-}
-
-// Gauss-Seidel update of coarse cell (i, j) = e; with C, the neighbours carry
-// the coarse correction x + prolong(e) * mask (the first reverse half-sweep)
-__device__ __forceinline__ void coarse_cell_update(const HLevel& L, CoarseRefs s, int i, int j, int e,
-                                                   const CoarseRefs* C, const HLevel* LC) {
-    const int nx = L.nx;
-    const int i_e = i + 1 == nx ? 0 : i + 1, i_w = i == 0 ? nx - 1 : i - 1;
-    const int j_n = j + 1 == L.ny ? 0 : j + 1, j_s = j == 0 ? L.ny - 1 : j - 1;
-    const int ie = j * nx + i_e, iw = j * nx + i_w, jn = j_n * nx + i, js = j_s * nx + i;
-    double xe = s.x[ie], xw = s.x[iw], xn = s.x[jn], xs = s.x[js];
-    if (C) {
-        const int cnx = LC->nx;
-        xe = xe + C->x[(j >> 1) * cnx + (i_e >> 1)] * s.m[ie];
-        xw = xw + C->x[(j >> 1) * cnx + (i_w >> 1)] * s.m[iw];
-        xn = xn + C->x[(j_n >> 1) * cnx + (i >> 1)] * s.m[jn];
-        xs = xs + C->x[(j_s >> 1) * cnx + (i >> 1)] * s.m[js];
-    }
-    const double nb = L.cx * (s.ku[e] * xe + s.ku[iw] * xw) + L.cy * (s.kv[e] * xn + s.kv[js] * xs);
-    s.x[e] = s.id[e] * (s.b[e] + nb) * s.m[e];
-}
-
-// one colour of a coarse-level sweep by the CTA. On even-sized levels only the
-// cells of that colour are visited (cell q of the colour: row q / (nx/2), column
-// 2 (q mod nx/2) + the row's parity offset); odd-sized levels test each cell.
-__device__ void coarse_half_sweep(const HLevel& L, CoarseRefs s, int colour, const CoarseRefs* C,
-                                  const HLevel* LC) {
-    const int nx = L.nx;
-    if (((nx | L.ny) & 1) == 0) {
-        const int hx = nx >> 1, nh = L.n >> 1;
-        for (int q = threadIdx.x; q < nh; q += blockDim.x) {
-            const int j = q / hx;
-            const int i = 2 * (q - j * hx) + ((j + colour) & 1);
-            coarse_cell_update(L, s, i, j, j * nx + i, C, LC);
-        }
-    } else {
-        for (int e = threadIdx.x; e < L.n; e += blockDim.x) {
-            const int j = e / nx, i = e - j * nx;
-            if (((i + j) & 1) != colour) continue;
-            coarse_cell_update(L, s, i, j, e, C, LC);
-        }
-    }
-    __syncthreads();
-}
-
-__device__ double coarse_residual(const HLevel& L, double coef, CoarseRefs s, int e) {
-    const int j = e / L.nx, i = e - j * L.nx;
-    const int ie = j * L.nx + (i + 1 == L.nx ? 0 : i + 1), iw = j * L.nx + (i == 0 ? L.nx - 1 : i - 1);
-    const int jn = (j + 1 == L.ny ? 0 : j + 1) * L.nx + i, js = (j == 0 ? L.ny - 1 : j - 1) * L.nx + i;
-    const double m = s.m[e];
-    const double xm = s.x[e] * m, xe = s.x[ie] * s.m[ie], xw = s.x[iw] * s.m[iw];
-    const double xn = s.x[jn] * s.m[jn], xs = s.x[js] * s.m[js];
-    const double fx = s.ku[e] * (xe - xm), fxw = s.ku[iw] * (xm - xw);
-    const double fy = s.kv[e] * (xn - xm), fys = s.kv[js] * (xm - xs);
-    const double lap = (fx - fxw) / L.dx2 + (fy - fys) / L.dy2;
-    const double ax = (xm - coef * lap) * m + xm * (1.0 - m);
-    return (s.b[e] - ax) * m;
-}
-
-// the V-cycle below and including level cf, by CTA 0 alone; reads level cf's b
-// (and x when cf is the finest level) from global memory, writes level cf's x
-// coef: the coarse coefficients kept for the whole solve (coarse_coef_load at its
-// start), or null to load them here
-__device__ void mg_coarse(const HelmParams& H, double* smem, const double* xin_cf, double* xout_cf,
-                          double* coef = nullptr) {
-    const int cf = H.coarse_from, nl = H.n_levels;
-    // the level coefficients (constant during the solve) by asynchronous copies, all
-    // in flight at once; level cf's b and x (written by this launch) through L2
-    if (!coef) coarse_coef_load(H, nullptr, smem);
-    {
-        const HLevel& L = H.lv[cf];
-        CoarseRefs s = coarse_refs(H, smem, cf, coef);
-        for (int e = threadIdx.x; e < L.n; e += blockDim.x) {
-            const double bv = __ldcg(L.b + e);
-            const double xv = xin_cf ? __ldcg(xin_cf + e) : 0.0;
-            s.b[e] = bv;
-            s.x[e] = xv;
-        }
+    for (int e = threadIdx.x; e < T.n; e += kSolveThreads) {
+        const int j = fast_div(e, T.nmag), o = coarse_pos(T, e - j * T.nx, j);
+        const double r = H.rhs[e] * __ldg(L.mask + e);
+        smem_all[T.b + o] = r;
+        smem_all[T.x + o] = H.warm ? L.x[e] : 0.0;
+        sq[e] = r * r;
     }
     cpa_wait_all();
     __syncthreads();
-    for (int l = cf; l < nl; ++l) {
-        const HLevel& L = H.lv[l];
-        CoarseRefs s = coarse_refs(H, smem, l, coef);
-        for (int h = 0; h < 4; ++h) coarse_half_sweep(L, s, h & 1, nullptr, nullptr);
-        if (l + 1 < nl) {
-            // the residual of every cell of level l (a coarser level exists only
-            // below an even-sized one, so they are exactly the 2x2 children),
-            // then the children's mean per coarse cell
-            const HLevel& C = H.lv[l + 1];
-            CoarseRefs c = coarse_refs(H, smem, l + 1, coef);
-            double* res = coarse_scratch(H, smem);
-            for (int f = threadIdx.x; f < L.n; f += blockDim.x) res[f] = coarse_residual(L, H.coef, s, f);
-            __syncthreads();
-            for (int e = threadIdx.x; e < C.n; e += blockDim.x) {
-                const int J = e / C.nx, I = e - J * C.nx;
-                const int f00 = (2 * J) * L.nx + 2 * I;
-                c.b[e] = 0.25 * (res[f00] + res[f00 + 1] + res[f00 + L.nx] + res[f00 + L.nx + 1]);
-                c.x[e] = 0.0;
+    // the square root of the squares' sum in NumPy's pairwise order
+    auto norm = [&]() {
+        for (int l0 = 4 * warp; l0 < H.n_leaves; l0 += 4 * (kSolveThreads / 32)) {
+            const int l = l0 + (lane >> 3), j = lane & 7;
+            const int st = l < H.n_leaves ? start[l] : 0, len = l < H.n_leaves ? start[l + 1] - st : 0, m = len & ~7;
+            double acc = 0.0;
+            if (m) {
+                acc = sq[st + j];
+#pragma unroll 4
+                for (int t = 8; t < m; t += 8) acc = acc + sq[st + t + j];
+            }
+            acc = acc + __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc = acc + __shfl_xor_sync(0xffffffffu, acc, 2);
+            acc = acc + __shfl_xor_sync(0xffffffffu, acc, 4);
+            for (int t = m; t < len; ++t) acc = acc + sq[st + t];
+            if (l < H.n_leaves && j == 0) slots[slot[l]] = acc;
+        }
+        __syncthreads();
+        const double x = H.n_slots == 32 ? warp_tree<1>(slots, false) : warp_tree<2>(slots, false);
+        return sqrt(__shfl_sync(0xffffffffu, x, 0));
+    };
+    const double norm_b = norm();
+    iters = 0;
+    conv = 1;
+    if (norm_b != 0.0) {
+        const double tol = H.rtol * norm_b;
+        conv = 0;
+        for (int it = 1; it <= H.max_iter; ++it) {
+            coarse_cycle();
+            iters = it;
+            // the residual of the stopping test is not masked (solvers_var.py:170-179)
+            if (T.even) {
+                for (int f = threadIdx.x; f < T.n; f += kSolveThreads) {
+                    const int p = f >= T.nh, q = f - p * T.nh;
+                    const double d = coarse_residual(T, H.coef, unit, p, q, false);
+                    const int j = fast_div(q, T.hmag);
+                    sq[j * T.nx + 2 * (q - j * T.hx) + ((p + j) & 1)] = d * d;
+                }
+            } else {
+                const double *x = smem_all + T.x, *mk = smem_all + T.m;
+                for (int e = threadIdx.x; e < T.n; e += kSolveThreads) {
+                    const Cell c = cell_of(L, e);
+                    const double m = mk[e], xm = x[e] * m;
+                    const double fx = smem_all[T.ku + e] * (x[c.ie] * mk[c.ie] - xm);
+                    const double fxw = smem_all[T.ku + c.iw] * (xm - x[c.iw] * mk[c.iw]);
+                    const double fy = smem_all[T.kv + e] * (x[c.jn] * mk[c.jn] - xm);
+                    const double fys = smem_all[T.kv + c.js] * (xm - x[c.js] * mk[c.js]);
+                    const double lap = (fx - fxw) / T.dx2 + (fy - fys) / T.dy2;
+                    const double d = smem_all[T.b + e] - ((xm - H.coef * lap) * m + xm * (1.0 - m));
+                    sq[e] = d * d;
+                }
             }
             __syncthreads();
-        }
-    }
-    {  // the coarsest level: its reverse sweeps follow the forward ones directly
-        const HLevel& L = H.lv[nl - 1];
-        CoarseRefs s = coarse_refs(H, smem, nl - 1, coef);
-        for (int h = 0; h < 4; ++h) coarse_half_sweep(L, s, 1 - (h & 1), nullptr, nullptr);
-    }
-    for (int l = nl - 2; l >= cf; --l) {
-        const HLevel& L = H.lv[l];
-        CoarseRefs s = coarse_refs(H, smem, l, coef);
-        CoarseRefs c = coarse_refs(H, smem, l + 1, coef);
-        coarse_half_sweep(L, s, 1, &c, &H.lv[l + 1]);
-        coarse_half_sweep(L, s, 0, nullptr, nullptr);
-        coarse_half_sweep(L, s, 1, nullptr, nullptr);
-        coarse_half_sweep(L, s, 0, nullptr, nullptr);
-    }
-    const HLevel& L = H.lv[cf];
-    CoarseRefs s = coarse_refs(H, smem, cf, coef);
-    for (int e = threadIdx.x; e < L.n; e += blockDim.x) xout_cf[e] = s.x[e];
-    __syncthreads();
-}
-
-// smoothing only (the coarsest level when it is too large for CTA 0): two
-// forward or two reverse sweeps
-__device__ void mg_smooth(const HelmParams& H, int l, const double* xin, double* xout, bool reverse,
-                          double* smem) {
-    const HLevel& L = H.lv[l];
-    const int tx = (L.nx + Tile32::TX - 1) / Tile32::TX, ty = (L.ny + Tile32::TY - 1) / Tile32::TY;
-    TileRefs t = tile_refs<Tile32>(smem);
-    for (int tile = s_grid.cta; tile < tx * ty; tile += s_grid.ncta) {
-        const int i0 = (tile % tx) * Tile32::TX, j0 = (tile / tx) * Tile32::TY;
-        tile_load<Tile32>(L, i0, j0, xin, nullptr, t);
-        tile_four_half_sweeps<Tile32>(L, i0, j0, t, reverse ? 1 : 0);
-        tile_store_x<Tile32>(L, i0, j0, t, xout);
-        __syncthreads();
-    }
-}
-
-// one V(2,2) cycle on x0 (level 0's current x); returns the buffer holding the
-// new x (x0 or level 0's second buffer). Levels below coarse_from have a grid
-// down and up phase; the rest run in CTA 0, or, when every level is too large
-// for it, the coarsest level is smoothed on the grid.
-__device__ double* vcycle_tiled(const HelmParams& H, double* x0, double* x0b, double* smem, double* persist,
-                                bool& ok) {
-    const int cf = H.coarse_from, nl = H.n_levels;
-    // CTA 0 keeps the coarse coefficients in its persistent region when it holds no level-0 tile
-    double* ccoef = (H.coarse_persist && s_grid.cta == 0) ? persist : nullptr;
-    if (cf == 0) {
-        if (s_grid.cta == 0) mg_coarse(H, smem, x0, x0b);
-        ok = grid_sync(H);
-        return x0b;
-    }
-    const int ndown = cf < nl ? cf : nl - 1;
-    for (int l = 0; l < ndown && ok; ++l) {
-        const double* xin = l == 0 ? x0 : nullptr;
-        double* xout = l == 0 ? x0b : H.lv[l].x;
-        switch (H.lv[l].shape) {
-            case SHAPE_WIDE: mg_down<TileWide>(H, l, xin, xout, smem, l == 0 ? persist : nullptr); break;
-            case SHAPE_3216: mg_down<Tile3216>(H, l, xin, xout, smem); break;
-            case SHAPE_16: mg_down<Tile16>(H, l, xin, xout, smem); break;
-            case SHAPE_8: mg_down<Tile8>(H, l, xin, xout, smem); break;
-            default: mg_down<Tile32>(H, l, xin, xout, smem); break;
-        }
-        ok = grid_sync(H);
-    }
-    if (!ok) return x0;
-    if (cf < nl) {
-        if (s_grid.cta == 0) mg_coarse(H, smem, nullptr, H.lv[cf].x2, ccoef);
-        ok = grid_sync(H);
-    } else {
-        const int l = nl - 1;
-        double* xa = (l == 0) ? x0b : H.lv[l].x;
-        double* xb = (l == 0) ? x0 : H.lv[l].x2;
-        mg_smooth(H, l, l == 0 ? x0 : nullptr, xa, false, smem);
-        ok = grid_sync(H);
-        if (!ok) return x0;
-        mg_smooth(H, l, xa, xb, true, smem);
-        ok = grid_sync(H);
-        if (l == 0) return x0;
-    }
-    // ascend: level l reads its down-phase result and level l+1's final x (in x2)
-    for (int l = ndown - 1; l >= 0 && ok; --l) {
-        const double* xin = (l == 0) ? x0b : H.lv[l].x;
-        double* xout = (l == 0) ? x0 : H.lv[l].x2;
-        HLevel C = H.lv[l + 1];
-        C.x = H.lv[l + 1].x2;
-        switch (H.lv[l].shape) {
-            case SHAPE_WIDE:
-                mg_up<TileWide>(H, l, xin, C, xout, smem, H.fused_res ? H.leafA : nullptr, l == 0 ? persist : nullptr);
+            const double res = norm();
+            if (res <= tol) {
+                conv = 1;
                 break;
-            case SHAPE_3216: mg_up<Tile3216>(H, l, xin, C, xout, smem, nullptr); break;
-            case SHAPE_16: mg_up<Tile16>(H, l, xin, C, xout, smem, nullptr); break;
-            case SHAPE_8: mg_up<Tile8>(H, l, xin, C, xout, smem, nullptr); break;
-            default: mg_up<Tile32>(H, l, xin, C, xout, smem, nullptr); break;
+            }
         }
-        ok = grid_sync(H);
     }
-    return x0;
+    for (int e = threadIdx.x; e < T.n; e += kSolveThreads) {
+        const int j = fast_div(e, T.nmag);
+        L.x[e] = smem_all[T.x + coarse_pos(T, e - j * T.nx, j)];
+    }
+}
+
+// the leaf sums of the squared residual of x (not masked, as the stopping test takes it)
+// into leafA, beside level 0's down phase: on the CTAs without a tile when each of
+// their warps then has at most one leaf, else on all, those with the fewest tiles first
+__device__ __noinline__ void residual_leaves(const double* x) {
+    const HelmParams& H = s_helm;
+    const HLevel& L0 = H.lv[0];
+    // with CTAs to spare the tiles sit on the last ones
+    const int idle = s_grid.ncta - level_tiles(L0), warps = kSolveThreads / 32;
+    const bool apart = idle > 0 && idle * warps >= H.n_leaves;
+    const int rank = s_grid.cta;
+    const int n = apart ? idle : s_grid.ncta;
+    if (rank >= n) return;
+    const int lane = threadIdx.x & 31;
+    for (int L = (threadIdx.x >> 5) * n + rank; L < H.n_leaves; L += n * warps) {
+        const int s = H.leaf_start[L], len = H.leaf_start[L + 1] - s;
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            v[q] = 0.0;
+            if (lane + 32 * q < len) {
+                const int e = s + lane + 32 * q;
+                const double d = __ldcg(L0.b + e) - apply_at(L0, H.coef, x, cell_of(L0, e));
+                v[q] = d * d;
+            }
+        }
+        const double a = leaf_sum_warp(v, len);
+        if (lane == 0) H.leafA[H.leaf_slot[L]] = a;
+    }
 }
 
 // ------------------------------------------------------------------ the solve kernel
 // A whole solve on the CTAs s_grid names (set by the kernel, followed by a CTA
 // barrier, before the call).
-__device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* smem_all) {
-    // with H.persist0 the first 4 RN doubles hold level 0's coefficient tile for the
+__device__ __forceinline__ void solve_log(const HelmParams& H, bool ok, int iters, int conv) {
+    if (s_grid.cta != 0 || threadIdx.x != 0) return;
+    const int idx = *H.log_count;
+    if (idx < H.log_cap) {
+        H.log_iters[idx] = ok ? iters : -1;
+        H.log_conv[idx] = ok ? conv : 0;
+    }
+    *H.log_count = idx + 1;
+}
+
+__device__ __forceinline__ void helm_solve_body() {
+    const HelmParams& H = s_helm;
+    if (H.one_cta) {
+        int its, cv;
+        helm_one_cta(its, cv);
+        solve_log(H, true, its, cv);
+        return;
+    }
+    // with H.persist0 the first 4 SN doubles (6 with its x and b) hold level 0's tile for the
     // whole solve; every other use of shared memory works above them
-    double* persist = H.persist0 ? smem_all : nullptr;
-    double* sm = smem_all + (H.persist0 ? 4 * TileWide::RN : 0);
+    const int persist = H.persist0 ? 0 : -1;
+    const int smo = H.persist0 ? (H.keep_x0 ? 6 : 4) * TileWide::SN : 0;
+    double* sm = smem_all + smo;
     const HLevel& L0 = H.lv[0];
     const double* rhs = H.rhs;
     double* x = L0.x;
@@ -794,9 +388,10 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                H.leafA, nullptr);
     ok = grid_sync(H);
     const double norm_b = ok ? sqrt(fold_sum(H, H.leafA, sm, ok)) : 0.0;
-    if (persist) persist_level0(H, persist);  // the coefficients are fixed during the solve
-    if (H.coarse_persist && s_grid.cta == 0) {
-        coarse_coef_load(H, persist, sm);
+    if (persist >= 0) persist_level0(smo, persist);  // the coefficients are fixed during the solve
+    if (s_grid.cta == 0 && H.coarse_from < H.n_levels) coarse_tab_init(smo, coarse_coef_at(H, smo, persist));
+    if (s_grid.cta == 0 && H.coarse_from < H.n_levels && s_coarse_held) {
+        coarse_coef_load();
         cpa_wait_all();
         __syncthreads();
     }
@@ -807,9 +402,24 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
             // stationary iteration with the true residual (solvers_var.py:170-179)
             conv = 0;
             double* xc = x;  // the level-0 buffer holding the current iterate
+            // Where the up phase does not form the residual's leaf sums, they are formed
+            // beside the next cycle's first phase, on the CTAs that have no tile in it if
+            // they are enough: a grid barrier and a pass of their own less per cycle, for
+            // one phase that the last cycle runs in vain.
+            const bool piped = H.kind == HK_MULTIGRID && !H.fused_res && H.coarse_from > 0 && H.n_levels > 1;
             for (int it = 1; it <= H.max_iter && ok; ++it) {
                 if (H.kind == HK_MULTIGRID) {
-                    xc = vcycle_tiled(H, xc, xc == H.lv[0].x ? H.lv[0].x2 : H.lv[0].x, sm, persist, ok);
+                    // the previous iterate's residual and its test, beside this cycle's first phase
+                    const double* xp = xc;
+                    xc = vcycle_tiled(H, xc, xc == H.lv[0].x ? H.lv[0].x2 : H.lv[0].x, smo, persist, ok,
+                                      [&]() { if (piped && it > 1) residual_leaves(xp); },
+                                      [&]() {
+                                          if (!piped || it == 1) return false;
+                                          iters = it - 1;
+                                          conv = sqrt(fold_sum(H, H.leafA, sm, ok)) <= tol ? 1 : 0;
+                                          return conv != 0 || !ok;
+                                      });
+                    if (conv) break;
                 } else {
                     colour_phase(L0, x, b0, 0, grid_team());
                     ok = grid_sync(H);
@@ -818,6 +428,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                     ok = grid_sync(H);
                 }
                 if (!ok) break;
+                if (piped && it < H.max_iter) continue;
                 // the true residual's leaf sums: formed by the last up phase when
                 // level 0's tiles are NumPy's leaves, else by a pass of their own
                 if (!(H.kind == HK_MULTIGRID && H.fused_res)) {
@@ -867,7 +478,7 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
                     }
                     okp = grid_sync(H);
                     if (!okp) return;
-                    double* zr = vcycle_tiled(H, z, L0.x2, sm, persist, okp);
+                    double* zr = vcycle_tiled(H, z, L0.x2, smo, persist, okp, []() {}, []() { return false; });
                     if (!okp || zr == z) return;
                     for (int e = grid_team().first; e < L0.n; e += grid_team().stride) z[e] = __ldcg(zr + e);
                     okp = grid_sync(H);
@@ -960,28 +571,19 @@ __device__ __forceinline__ void helm_solve_body(const HelmParams& H, double* sme
     }
 done:
     grid_sync_end(H.bar_count, s_grid.cta == 0);
-    if (s_grid.cta == 0 && threadIdx.x == 0) {
-        const int idx = *H.log_count;
-        if (idx < H.log_cap) {
-            H.log_iters[idx] = ok ? iters : -1;
-            H.log_conv[idx] = ok ? conv : 0;
-        }
-        *H.log_count = idx + 1;
-    }
+    solve_log(H, ok, iters, conv);
 }
 
 // The parameters are read through a reference throughout the solve: a copy in
 // shared memory, made once per CTA (a reference to the kernel parameter itself
 // would give every thread a copy of its own in local memory).
 __global__ void __launch_bounds__(512) k_helm_solve(HelmParams H) {
-    extern __shared__ double smem_all[];
-    __shared__ HelmParams sH;
     if (threadIdx.x == 0) s_grid = SolveGrid{(int)blockIdx.x, (int)gridDim.x};
     const int* src = reinterpret_cast<const int*>(&H);
-    int* dst = reinterpret_cast<int*>(&sH);
+    int* dst = reinterpret_cast<int*>(&s_helm);
     for (int t = threadIdx.x; t < (int)(sizeof(HelmParams) / sizeof(int)); t += blockDim.x) dst[t] = src[t];
     __syncthreads();
-    helm_solve_body(sH, smem_all);
+    helm_solve_body();
 }
 
 // Several systems in one cooperative launch: system m runs on CTAs
@@ -990,8 +592,6 @@ __global__ void __launch_bounds__(512) k_helm_solve(HelmParams H) {
 // never wait on one another.
 __global__ void __launch_bounds__(512) k_helm_solve_batched(const HelmParams* __restrict__ systems,
                                                             const int* __restrict__ cta_start, int n) {
-    extern __shared__ double smem_all[];
-    __shared__ HelmParams sH;
     __shared__ int s_m;
     if (threadIdx.x == 0) {
         int m = 0;
@@ -1001,16 +601,16 @@ __global__ void __launch_bounds__(512) k_helm_solve_batched(const HelmParams* __
     }
     __syncthreads();
     const int* src = reinterpret_cast<const int*>(systems + s_m);
-    int* dst = reinterpret_cast<int*>(&sH);
+    int* dst = reinterpret_cast<int*>(&s_helm);
     for (int t = threadIdx.x; t < (int)(sizeof(HelmParams) / sizeof(int)); t += blockDim.x) dst[t] = src[t];
     __syncthreads();
-    helm_solve_body(sH, smem_all);
+    helm_solve_body();
 }
 
 // ------------------------------------------------------------------ level rebuild
 // coarse face coefficients (solvers_var.py:118-123) and inverse diagonal
 // (solvers_var.py:39-45) of level `L` from the finer level `F`
-__global__ void k_helm_level(HLevel F, HLevel L, int coarse) {
+__global__ void k_helm_level(HLevel F, HLevel L, int coarse, int unit_mask) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.n) return;
     const int J = e / L.nx, I = e - J * L.nx;
@@ -1036,7 +636,9 @@ __global__ void k_helm_level(HLevel F, HLevel L, int coarse) {
         kvs = L.Kv[Js * L.nx + I];
     }
     const double d = 1.0 + L.cx * (ku + kuw) + L.cy * (kv + kvs);
-    L.inv_diag[e] = 1.0 / (L.mask[e] > 0.0 ? d : 1.0);
+    const double inv = 1.0 / (L.mask[e] > 0.0 ? d : 1.0);
+    L.inv_diag[e] = inv;
+    if (L.idm != L.inv_diag) L.idm[e] = unit_mask ? inv * L.mask[e] : inv;
 }
 
 // ------------------------------------------------------------------ host side
@@ -1162,6 +764,8 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     H.rtol = rtol;
     H.max_iter = max_iter;
     H.status = status;
+    H.unit_mask = 1;
+    for (size_t c = 0; c < (size_t)nx * ny && H.unit_mask; ++c) H.unit_mask = mask_host[c] == 0.0 || mask_host[c] == 1.0;
     // level geometry and masks
     std::vector<std::vector<double>> masks;
     masks.push_back(std::vector<double>(mask_host, mask_host + (size_t)nx * ny));
@@ -1208,6 +812,7 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         cudaMemcpy(m, masks[l].data(), sizeof(double) * L.n, cudaMemcpyHostToDevice);
         L.mask = m;
         L.inv_diag = (double*)dalloc(sizeof(double) * L.n);
+        L.idm = mg_levels ? (double*)dalloc(sizeof(double) * L.n) : L.inv_diag;
         L.b = (double*)dalloc(sizeof(double) * L.n);
         L.x2 = (double*)dalloc(sizeof(double) * L.n);
         if (l == 0) {
@@ -1219,11 +824,11 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
             L.Kv = (double*)dalloc(sizeof(double) * L.n);
             L.x = (double*)dalloc(sizeof(double) * L.n);
         }
-        if (!L.inv_diag || !L.b || !L.x2 || (l > 0 && (!L.Ku || !L.Kv || !L.x))) {
+        if (!L.inv_diag || !L.idm || !L.b || !L.x2 || (l > 0 && (!L.Ku || !L.Kv || !L.x))) {
             err = "cudaMalloc failed (Helmholtz levels)";
             return OC_ERR_CUDA;
         }
-        if (L.n <= kCoarseCells && H.coarse_from == H.n_levels) H.coarse_from = l;
+        if (L.n <= (l == 0 && mg_levels ? kOneCtaCells : kCoarseCells) && H.coarse_from == H.n_levels) H.coarse_from = l;
     }
     const size_t n = (size_t)nx * ny;
     H.r = (double*)dalloc(sizeof(double) * n);
@@ -1350,41 +955,60 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     for (int q = 0; q < H.n_leaves && aligned; ++q)
         aligned = leaves[q] == 128 * q && leaves[q + 1] - leaves[q] == 128;
     H.fused_res = (kind == HK_MULTIGRID && H.wide0 && aligned) ? 1 : 0;
+    // the stationary iteration's x and b too, unless a tile overhangs the grid; inside
+    // CG every cycle starts from a new right-hand side
+    H.keep_x0 = (H.persist0 && kind == HK_MULTIGRID && ny % TileWide::TY == 0) ? 1 : 0;
+    H.one_cta = (kind == HK_MULTIGRID && H.coarse_from == 0) ? 1 : 0;
+    // CTA 0 holds no level-0 tile when there are more CTAs than tiles: its persistent
+    // area then keeps the coarse levels' four coefficient arrays
+    H.coarse_persist = (H.persist0 && H.coarse_from > 0 && H.coarse_from < H.n_levels && sms > wide_tiles &&
+                        4 * coarse_cells <= 4 * (size_t)TileWide::SN) ? 1 : 0;
     // shared memory: the persistent tile (if any), then the largest of the tree
     // fold, the grid levels' tiles and the coarse levels of CTA 0
-    size_t tile_work = 0;
     const int n_grid = H.coarse_from < H.n_levels ? H.coarse_from : H.n_levels;
-    auto rn_of = [](int shape) {
+    auto sn_of = [](int shape) {
         switch (shape) {
-            case SHAPE_WIDE: return TileWide::RN;
-            case SHAPE_3216: return Tile3216::RN;
-            case SHAPE_16: return Tile16::RN;
-            case SHAPE_8: return Tile8::RN;
-            default: return Tile32::RN;
+            case SHAPE_WIDE: return TileWide::SN;
+            case SHAPE_3216: return Tile3216::SN;
+            case SHAPE_16: return Tile16::SN;
+            case SHAPE_8: return Tile8::SN;
+            default: return Tile32::SN;
         }
     };
-    if (mg_levels) {
+    // the rows of squares that a wide tile's up phase sums sit above the tile's work area
+    const size_t rows = (size_t)(kSolveThreads / 32) * kLeafRow;
+    // the work area of the grid levels; kept: level-0 arrays that are elsewhere (0, 4 or 6)
+    auto tile_work = [&](int kept) {
+        size_t w = 0;
+        if (!mg_levels) return w;
         for (int l = 0; l < n_grid; ++l)
-            tile_work = std::max<size_t>(tile_work, (l == 0 && H.persist0 ? 2 : 6) * (size_t)rn_of(H.lv[l].shape));
-        if (H.coarse_from >= H.n_levels) tile_work = std::max<size_t>(tile_work, 6 * (size_t)Tile32::RN);
-    }
-    const size_t coarse_work = 6 * coarse_cells + (H.coarse_from < H.n_levels ? (size_t)H.lv[H.coarse_from].n : 0);
-    const size_t mg_work = mg_levels ? std::max<size_t>(tile_work, coarse_work) : 0;
+            w = std::max<size_t>(w, (6 - (l == 0 ? kept : 0)) * (size_t)sn_of(H.lv[l].shape) +
+                                        (H.lv[l].shape == SHAPE_WIDE ? rows : 0));
+        if (H.coarse_from >= H.n_levels) w = std::max<size_t>(w, 6 * (size_t)Tile32::SN);
+        return w;
+    };
+    auto coarse_work = [&](bool persist) {
+        if (!mg_levels || H.coarse_from >= H.n_levels) return (size_t)0;
+        return (persist ? 2 : 6) * coarse_cells + (size_t)H.lv[H.coarse_from].n + kFoldScratch +
+               (H.one_cta ? (size_t)H.n_slots + H.n_leaves + 2 : 0);
+    };
     // in a batched launch a system has fewer CTAs than tiles: no persistent level-0
     // tile (its six arrays are loaded per tile instead)
-    size_t tile_work_b = 0;
-    if (mg_levels) {
-        for (int l = 0; l < n_grid; ++l) tile_work_b = std::max<size_t>(tile_work_b, 6 * (size_t)rn_of(H.lv[l].shape));
-        if (H.coarse_from >= H.n_levels) tile_work_b = std::max<size_t>(tile_work_b, 6 * (size_t)Tile32::RN);
-    }
-    const size_t mg_work_b = mg_levels ? std::max<size_t>(tile_work_b, coarse_work) : 0;
-    smem_batched_ = sizeof(double) * std::max<size_t>(fold_doubles, mg_work_b);
+    smem_batched_ = sizeof(double) * std::max(fold_doubles, std::max(tile_work(0), coarse_work(false)));
     // the tree fold and the V-cycle never run at the same time: one region serves both
-    smem_ = sizeof(double) * ((H.persist0 ? 4 * (size_t)TileWide::RN : 0) + std::max<size_t>(fold_doubles, mg_work));
+    auto solve_smem = [&](int kept) {
+        return sizeof(double) * (kept * (size_t)TileWide::SN +
+                                 std::max(fold_doubles, std::max(tile_work(kept), coarse_work(kept && H.coarse_persist))));
+    };
     int smem_optin = 0;
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa{};
     cudaFuncGetAttributes(&fa, k_helm_solve);  // static shared memory (the barrier's word) comes first
+    // level 0 keeps what fits: everything, its coefficients, or nothing
+    auto fits = [&](int kept) { return solve_smem(kept) + fa.sharedSizeBytes <= (size_t)smem_optin; };
+    if (H.keep_x0 && !fits(6)) H.keep_x0 = 0;
+    if (H.persist0 && !H.keep_x0 && !fits(4)) H.persist0 = H.coarse_persist = 0;
+    smem_ = solve_smem(H.keep_x0 ? 6 : (H.persist0 ? 4 : 0));
     if (smem_ + fa.sharedSizeBytes > (size_t)smem_optin) {
         err = "Helmholtz grid too large for the single-pass reduction tree";
         return OC_ERR_UNSUPPORTED;
@@ -1407,20 +1031,9 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         err = "Helmholtz solve kernel cannot be resident";
         return OC_ERR_CUDA;
     }
-    grid_ = sms * std::min(per_sm, 2);
-    // CTA 0 holds no level-0 tile when there are more CTAs than tiles: its
-    // persistent region then keeps the coarse levels' four coefficient arrays
-    {
-        size_t ccells = 0;
-        for (int l = H.coarse_from; l < H.n_levels; ++l) ccells += (size_t)H.lv[l].n;
-        const int tiles0 = ((nx + TileWide::TX - 1) / TileWide::TX) * ((ny + TileWide::TY - 1) / TileWide::TY);
-        H.coarse_persist = (H.persist0 && mg_levels && H.coarse_from > 0 && H.coarse_from < H.n_levels &&
-                            grid_ > tiles0 && ccells <= (size_t)TileWide::RN) ? 1 : 0;
-    }
+    grid_ = mg_levels && H.coarse_from == 0 ? 1 : sms * std::min(per_sm, 2);
     // PCG-Jacobi with the vectors on the chip (its operator relies on a 0/1 mask)
-    bool unit_mask = true;
-    for (size_t c = 0; c < n && unit_mask; ++c) unit_mask = mask_host[c] == 0.0 || mask_host[c] == 1.0;
-    pcg_ = !refined && kind == HK_PCG_JACOBI && unit_mask && !H.big_fold &&
+    pcg_ = !refined && kind == HK_PCG_JACOBI && H.unit_mask && !H.big_fold &&
            pcg_plan(leaves, H.n_slots, nx, pcg_plan_);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1469,7 +1082,7 @@ void HelmSolver::rebuild(cudaStream_t s) {
     for (int l = 0; l < hp_.n_levels; ++l) {
         const HLevel& L = hp_.lv[l];
         const HLevel& F = hp_.lv[l > 0 ? l - 1 : 0];
-        k_helm_level<<<(L.n + 255) / 256, 256, 0, s>>>(F, L, l > 0 ? 1 : 0);
+        k_helm_level<<<(L.n + 255) / 256, 256, 0, s>>>(F, L, l > 0 ? 1 : 0, hp_.unit_mask);
     }
 }
 
@@ -1478,7 +1091,9 @@ HelmParams HelmSolver::batched_params(const double* rhs, double* x) const {
     H.rhs = rhs;
     H.lv[0].x = x;
     H.persist0 = 0;
+    H.keep_x0 = 0;
     H.coarse_persist = 0;
+    H.one_cta = 0;
     H.warm = warm_ ? 1 : 0;
     return H;
 }

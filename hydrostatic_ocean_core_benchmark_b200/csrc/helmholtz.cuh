@@ -25,6 +25,7 @@ struct HLevel {
     double* Ku;
     double* Kv;
     double* inv_diag;
+    double* idm;  // inv_diag * mask for 0/1 masks (else inv_diag): what a multigrid sweep multiplies by
     double* x;   // current solution of the level (level 0: the caller's output)
     double* x2;  // second buffer: the smoothing phases read one and write the other
     double* b;
@@ -36,7 +37,10 @@ struct HelmParams {
     int wide0;      // level 0 runs 128 x 16 tiles
     int fused_res;  // ... whose rows are NumPy's leaves: the up phase forms the residual sums
     int persist0;   // ... one per CTA: their coefficients stay in shared memory for the solve
+    int keep_x0;    // ... and so do their x and b
     int coarse_persist;  // CTA 0 (no level-0 tile) keeps the coarse levels' coefficients in its region
+    int one_cta;    // the whole multigrid solve runs in one CTA (helm_one_cta)
+    int unit_mask;  // the masks are 0/1
     double coef, rtol;
     HLevel lv[OC_MAX_LEVELS];
     double *r, *z, *p, *Ap;  // level-0 work vectors

@@ -81,3 +81,25 @@ def test_uneven_leaf_trees_match_oracle(kind, nx, ny):
     assert rep.iterations == itr and rep.converged == ok
     assert np.array_equal(x, xr)
     solver.close()
+
+
+@pytest.mark.parametrize("nx,ny", [
+    (6, 4), (62, 30), (64, 40), (40, 64),  # one CTA: tiny, an odd coarsest level, the largest
+    (66, 40), (52, 50),                               # just above it
+    (128, 96), (128, 128),                            # tiles over one-CTA coarse levels
+    (384, 256), (384, 272),                           # wide tiles with their x and b kept
+    (512, 520), (1024, 400),                          # a partial last row of tiles; more tiles than SMs
+])
+def test_multigrid_forms_match_oracle(nx, ny):
+    """The V-cycle on one CTA and on tiles of every form."""
+    from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+    dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx + 7 * ny, walls=True)
+    solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind="multigrid",
+                          rtol=1e-8, max_iter=6)
+    ref = orc.Helmholtz(nx, ny, 4.0e6, 5.0e6, coef, ku, kv, mask, "multigrid", 1e-8, 6)
+    for r in (rhs, np.zeros_like(rhs), rhs[:, ::-1].copy()):
+        x, rep = solver.solve(r)
+        xr, itr, ok = ref.solve(r)
+        assert rep.iterations == itr and rep.converged == ok
+        assert np.array_equal(x, xr)
+    solver.close()
