@@ -360,27 +360,33 @@ int step_once(oc_handle* h, cudaStream_t s) {
         }
     }
     cudaStreamWaitEvent(s, h->join, 0);
+    // where pass m's right-hand sides go (and its column solves work in place)
+    auto target = [&](int m, double*& tu, double*& tv) {
+        if (!theta && m == c.n_picard - 1 && !split) {
+            tu = un;
+            tv = vn;
+        } else if (theta || m % 2 == 0) {
+            tu = h->ghu;
+            tv = h->ghv;
+        } else {
+            tu = h->uit;
+            tv = h->vit;
+        }
+    };
+    double *tu, *tv;
+    target(0, tu, tv);
     {
+        // the terms of the old state, and the first pass's right-hand sides from them
         Prof pr(h, s, "mom_explicit");
-        launch_mom_explicit(P, u, v, b, h->phi, h->w, h->km, h->pgx, h->pgy, h->avpv, h->avpu, h->dzu,
-                            h->dzv, h->stu, h->stv, s);
+        launch_mom_explicit(P, u, v, b, h->phi, h->w, h->km, h->gx2, h->gy2, h->pgx, h->pgy, h->avpv, h->avpu, h->dzu,
+                            h->dzv, h->stu, h->stv, tu, tv, s);
     }
     const double *uit = u, *vit = v;
     double *last_gu = nullptr, *last_gv = nullptr;
     for (int m = 0; m < c.n_picard; ++m) {
         const bool last = m == c.n_picard - 1;
-        double *tu, *tv;
-        if (theta) {
-            tu = h->ghu;
-            tv = h->ghv;
-        } else if (last && !split) {
-            tu = un;
-            tv = vn;
-        } else {
-            tu = (m % 2 == 0) ? h->ghu : h->uit;
-            tv = (m % 2 == 0) ? h->ghv : h->vit;
-        }
-        {
+        target(m, tu, tv);
+        if (m > 0) {
             Prof pr(h, s, "predictor_rhs");
             launch_predictor_rhs(P, u, v, uit, vit, h->pgx, h->pgy, h->avpv, h->avpu, h->dzu, h->dzv,
                                  h->stu, h->stv, h->gx2, h->gy2, tu, tv, s);
@@ -649,6 +655,12 @@ static int set_domain_impl(oc_handle* h, const double* Hh, const double* maskh, 
         P.dzr[k] = h->dzr[k];
         P.thin[k] = h->cfg.min_partial * h->dzr[k];
         P.dz_nom[k] = h->cfg.h0 / nz;  // the reference's nominal H/nz (model3d_v05.py:247)
+    }
+    for (int k = 0; k < nz; ++k) {
+        P.fdz[k] = face_host(P.face_rule, P.dzr[k], P.dzr[k]);
+        P.rfdz[k] = P.fdz[k] > 0.0 ? 1.0 / P.fdz[k] : 0.0;
+        const double dzi = k > 0 ? 0.5 * (P.fdz[k - 1] + P.fdz[k]) : 0.0;
+        P.rfdzi[k] = dzi > 0.0 ? 1.0 / dzi : 0.0;
     }
     for (int k = 0; k <= nz; ++k) P.edge64[k] = P.edge[k];
     for (int k = 0; k < nz; ++k) P.dzr64[k] = P.dzr[k];
@@ -951,8 +963,9 @@ int oc_autotune(oc_handle* h, int32_t* mom_levels, int32_t* tracer_levels) {
         mk = best_of(P.mom_kl, [&](int kl) {
             KPT<float> Q = P;
             Q.mom_kl = kl;
-            launch_mom_explicit(Q, h->U32[c], h->V32[c], h->B[c], h->phi, h->w32, h->km32, h->pgx32, h->pgy32,
-                                h->avpv32, h->avpu32, h->dzu32, h->dzv32, h->stu32, h->stv32, s);
+            launch_mom_explicit(Q, h->U32[c], h->V32[c], h->B[c], h->phi, h->w32, h->km32, h->gx2, h->gy2, h->pgx32,
+                                h->pgy32, h->avpv32, h->avpu32, h->dzu32, h->dzv32, h->stu32, h->stv32, h->ghu32,
+                                h->ghv32, s);
         });
         tk = best_of(P.tr_kl, [&](int kl) {
             KPT<float> Q = P;
@@ -966,8 +979,8 @@ int oc_autotune(oc_handle* h, int32_t* mom_levels, int32_t* tracer_levels) {
         mk = best_of(P.mom_kl, [&](int kl) {
             KP Q = P;
             Q.mom_kl = kl;
-            launch_mom_explicit(Q, h->U[c], h->V[c], h->B[c], h->phi, h->w, h->km, h->pgx, h->pgy, h->avpv, h->avpu,
-                                h->dzu, h->dzv, h->stu, h->stv, s);
+            launch_mom_explicit(Q, h->U[c], h->V[c], h->B[c], h->phi, h->w, h->km, h->gx2, h->gy2, h->pgx, h->pgy,
+                                h->avpv, h->avpu, h->dzu, h->dzv, h->stu, h->stv, h->ghu, h->ghv, s);
         });
         tk = best_of(P.tr_kl, [&](int kl) {
             KP Q = P;

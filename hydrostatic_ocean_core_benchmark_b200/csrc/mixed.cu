@@ -95,6 +95,12 @@ void convert_params(const KP& a, KPT<float>& b) {
         b.thin[k] = (float)a.thin[k];
         b.dz_nom[k] = (float)a.dz_nom[k];
     }
+    for (int k = 0; k < a.nz; ++k) {
+        b.fdz[k] = (float)a.fdz[k];
+        b.rfdz[k] = b.fdz[k] > 0.0f ? 1.0f / b.fdz[k] : 0.0f;
+        const float dzi = k > 0 ? 0.5f * (b.fdz[k - 1] + b.fdz[k]) : 0.0f;
+        b.rfdzi[k] = dzi > 0.0f ? 1.0f / dzi : 0.0f;
+    }
     b.kinfo = a.kinfo, b.kface = a.kface, b.face_rule = a.face_rule;
     b.mom_kl = a.mom_kl, b.tr_kl = a.tr_kl;
     b.dx64 = a.dx64, b.dy64 = a.dy64;
@@ -301,26 +307,32 @@ int step_once_mixed(oc_handle* h, cudaStream_t s) {
         }
     }
     cudaStreamWaitEvent(s, h->join, 0);
+    // where pass m's right-hand sides go (and its column solves work in place)
+    auto target = [&](int m, float*& tu, float*& tv) {
+        if (!theta && m == c.n_picard - 1) {
+            tu = un;
+            tv = vn;
+        } else if (theta || m % 2 == 0) {
+            tu = h->ghu32;
+            tv = h->ghv32;
+        } else {
+            tu = h->uit32;
+            tv = h->vit32;
+        }
+    };
+    float *tu, *tv;
+    target(0, tu, tv);
     {
+        // the terms of the old state, and the first pass's right-hand sides from them
         Prof pr(h, s, "mom_explicit");
-        launch_mom_explicit(Q, u, v, b, h->phi, h->w32, h->km32, h->pgx32, h->pgy32, h->avpv32, h->avpu32,
-                            h->dzu32, h->dzv32, h->stu32, h->stv32, s);
+        launch_mom_explicit(Q, u, v, b, h->phi, h->w32, h->km32, h->gx2, h->gy2, h->pgx32, h->pgy32, h->avpv32,
+                            h->avpu32, h->dzu32, h->dzv32, h->stu32, h->stv32, tu, tv, s);
     }
     const float *uit = u, *vit = v;
     for (int m = 0; m < c.n_picard; ++m) {
         const bool last = m == c.n_picard - 1;
-        float *tu, *tv;
-        if (theta) {
-            tu = h->ghu32;
-            tv = h->ghv32;
-        } else if (last) {
-            tu = un;
-            tv = vn;
-        } else {
-            tu = (m % 2 == 0) ? h->ghu32 : h->uit32;
-            tv = (m % 2 == 0) ? h->ghv32 : h->vit32;
-        }
-        {
+        target(m, tu, tv);
+        if (m > 0) {
             Prof pr(h, s, "predictor_rhs");
             launch_predictor_rhs(Q, u, v, uit, vit, h->pgx32, h->pgy32, h->avpv32, h->avpu32, h->dzu32, h->dzv32,
                                  h->stu32, h->stv32, h->gx2, h->gy2, tu, tv, s);

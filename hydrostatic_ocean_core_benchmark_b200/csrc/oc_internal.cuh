@@ -67,6 +67,9 @@ struct KPT {
     T dzr[OC_MAXNZ];
     T thin[OC_MAXNZ];       // min_partial * dzr
     T dz_nom[OC_MAXNZ];     // spacing of the momentum vertical advection per level
+    // where both columns of a face have their full thickness: the face's thickness at
+    // level k, 1 over it, and 1 over the spacing of the interface between k - 1 and k
+    T fdz[OC_MAXNZ], rfdz[OC_MAXNZ], rfdzi[OC_MAXNZ];
     // static 2D fields
     const T* H;
     const T* mask;
@@ -224,10 +227,31 @@ __device__ __forceinline__ T face_combine(const KPT<T>& P, T a, T b) {
     return tot > T(0.0) ? T(2.0) * a * b / tot : T(0.0);
 }
 
-// Superbee limiter of the TVD face (reference advection_v06.py:35-43)
+// Superbee limiter of the TVD face (reference advection_v06.py:35-43),
+// max(0, max(min(2r, 1), min(r, 2))) in the form its branches leave: for r < 1 the
+// first minimum is the larger one, else the second. One comparison and selects
+// replace three of the four double minima and maxima, each of which takes a
+// comparison, two selects and a NaN rule; a NaN ratio gives 2, as those do.
 template <class T>
 __device__ __forceinline__ T superbee(T r) {
-    return fmax(T(0.0), fmax(fmin(T(2.0) * r, T(1.0)), fmin(r, T(2.0))));
+    const bool low = r < T(1.0);
+    const T a = low ? T(2.0) * r : r;
+    const T cap = low ? T(1.0) : T(2.0);
+    const T psi = a < cap ? a : cap;
+    return psi > T(0.0) ? psi : T(0.0);
+}
+
+// The upwind-biased correction t of a face between c0 and c1 (d = c1 - c0) with the
+// upstream difference `far`: limited, 0.5 superbee(far / d) d, else the kappa = 1/3
+// form. Where d is 0 the ratio is far (divided by 1) and t = 0 whatever it is: the
+// limiter is finite.
+template <class T>
+__device__ __forceinline__ T face_correction(const KPT<T>& P, T far, T d, bool limited) {
+    if (limited) {
+        const T eps = d == T(0.0) ? T(1.0) : d;
+        return T(0.5) * superbee(far / eps) * d;
+    }
+    return T(0.25) * (P.one_m_kappa3 * far + P.one_p_kappa3 * d);
 }
 
 // Upwind-biased value on the face between c0 and c1 (c_m = left of c0,
@@ -238,21 +262,19 @@ __device__ __forceinline__ T superbee(T r) {
 // c1 - t equals c1 + (-t) exactly, so the bits are the same, with one division
 // instead of two and no divergent branch.
 template <class T>
-__device__ __forceinline__ T kappa_face(const KPT<T>& P, T cm, T c0, T c1, T cp, T vel, T wm, T wp, bool limited) {
+__device__ __forceinline__ T kappa_face_f(const KPT<T>& P, T cm, T c0, T c1, T cp, T vel, bool wm, bool wp,
+                                          bool limited) {
     const bool pos = vel > T(0.0);
     const T base = pos ? c0 : c1;
     const T far = pos ? (c0 - cm) : (cp - c1);
-    const T d = c1 - c0;
-    T t;
-    if (limited) {
-        const T eps = d == T(0.0) ? T(1.0) : d;
-        const T r = d == T(0.0) ? T(0.0) : far / eps;
-        t = T(0.5) * superbee(r) * d;
-    } else {
-        t = T(0.25) * (P.one_m_kappa3 * far + P.one_p_kappa3 * d);
-    }
+    const T t = face_correction(P, far, c1 - c0, limited);
     const T f = base + (pos ? t : -t);
-    return ((pos ? wm : wp) > T(0.0)) ? f : base;
+    return (pos ? wm : wp) ? f : base;
+}
+
+template <class T>
+__device__ __forceinline__ T kappa_face(const KPT<T>& P, T cm, T c0, T c1, T cp, T vel, T wm, T wp, bool limited) {
+    return kappa_face_f(P, cm, c0, c1, cp, vel, wm > T(0.0), wp > T(0.0), limited);
 }
 
 // Interior vertical face value at an interface with `above` (layer k-1),
@@ -265,15 +287,7 @@ __device__ __forceinline__ T kappa_face_z(const KPT<T>& P, T far_up, T above, T 
     const bool up = w > T(0.0);
     const T base = up ? below : above;
     const T far = up ? (below - far_dn) : (far_up - above);
-    const T d = above - below;
-    T t;
-    if (limited) {
-        const T eps = d == T(0.0) ? T(1.0) : d;
-        const T r = d == T(0.0) ? T(0.0) : far / eps;
-        t = T(0.5) * superbee(r) * d;
-    } else {
-        t = T(0.25) * (P.one_m_kappa3 * far + P.one_p_kappa3 * d);
-    }
+    const T t = face_correction(P, far, above - below, limited);
     const T f = base + (up ? t : -t);
     return (up ? has_dn : has_up) ? f : base;
 }

@@ -665,6 +665,18 @@ __device__ __forceinline__ real diff_flux(real Kk, real f_above, real f_below, r
 // reference's operations in its order.
 constexpr int MOM_TX = 32, MOM_TY = 8, MOM_RX = MOM_TX + 4, MOM_RY = MOM_TY + 4, MOM_RN = MOM_RX * MOM_RY;
 
+// The right-hand side of a momentum tridiagonal at one cell: the explicit predictor with
+// the Coriolis average `av` of the old state and `it` of the iterate, plus the
+// stress/advection increment (model3d_v05.py:387-393); f is f0 for u, -f0 for v.
+__device__ __forceinline__ real predictor(const KPR& P, real x, real f, real av, real it, real pg, real g2, real m,
+                                          real dz, real st) {
+    const real cor = P.one_m_tc * av + P.theta_cor * it;
+    real g = x + P.dt * (f * cor + pg);
+    if (P.scheme != 2) g = g - P.c1 * (g2 * m);
+    g = g + P.c3 * dz;
+    return g + st;
+}
+
 // the level's u, v and face masks of a tile plus a 2-column ring, in shared memory
 struct TileLevel {
     const real* su;
@@ -679,91 +691,178 @@ struct TileLevel {
     __device__ __forceinline__ real MV(int dj, int di) const { return k < skv[rc + dj * MOM_RX + di] ? real(1.0) : real(0.0); }
 };
 
+// What a level does to the values carried down a face's column.
+struct MomCarry {
+    real x_m1, x_0, x_p1;  // the component's velocity at levels k - 1, k, k + 1
+    real fz, df;           // vertical advective and diffusive flux through the top of level k
+};
+
+// The outputs of one component, by pointer (its own arrays of the eight, plus the right-hand side)
+struct MomOut {
+    real *pg, *av, *dz, *st, *rhs;
+};
+
+// One level of a tile whose columns, ring included, are wet and full at levels k and
+// k + 1: thicknesses and their reciprocals come from the level table, the two columns
+// of a face sit at one depth, and the face masks are those of the 2D faces (fl: bit per
+// stencil place, see mom_face_flags). COMP 0 is u: `along` is x and the other velocity
+// v; COMP 1 is v: along y, u. The terms are those of the general form below, operation
+// for operation; where a factor is 1 or a difference of equal depths 0 it is left out.
+template <int COMP>
+__device__ __forceinline__ void mom_full_level(const KPR& P, const real* __restrict__ X, const real* __restrict__ Y,
+                                               unsigned fl, int kff, int k, real x_p2, real K_1, real w_c, real w_f,
+                                               wide phc, wide phf, wide bc, wide bf, real tau, real g2, size_t at,
+                                               const MomOut& out, MomCarry& q) {
+    constexpr int A = COMP ? MOM_RX : 1, B = COMP ? 1 : MOM_RX;  // strides along the component's axis and across it
+    const real m = (fl >> 8) & 1 ? real(1.0) : real(0.0);
+    const wide dxy = COMP ? P.dy64 : P.dx64;
+    wide pgw;
+    if (P.pgf_correction) pgw = m * ((phf + bf * 0.0) - (phc + bc * 0.0)) / dxy;
+    else pgw = m * (phf - phc) / dxy * m;
+    const real pg = real(pgw);
+    out.pg[at] = pg;
+    // Coriolis average over the wet ones of four faces
+    const real y0 = Y[0], y1 = Y[-B], y2 = Y[A], y3 = Y[A - B];
+    real av;
+    if ((fl >> 9 & 15u) == 15u) {
+        av = (((y0 + y1) + y2) + y3) * real(0.25) * m;  // a division by 4 is exact
+    } else {
+        const real w0 = (fl >> 9) & 1, w1 = (fl >> 10) & 1, w2 = (fl >> 11) & 1, w3 = (fl >> 12) & 1;
+        const real den = ((w0 + w1) + w2) + w3;
+        const real num = ((w0 * y0 + w1 * y1) + w2 * y2) + w3 * y3;
+        av = (den > real(0.0) ? num / den : real(0.0)) * m;
+    }
+    out.av[at] = av;
+    // explicit vertical diffusion
+    const bool open = (fl >> 8) & 1;  // a closed face has no thickness
+    const real db = K_1 * (q.x_0 - q.x_p1) * (open ? P.rfdzi[k + 1] : real(0.0));
+    const real rdz = open ? P.rfdz[k] : real(0.0);
+    const real dz = (q.df - db) * rdz;
+    out.dz[at] = dz;
+    // advection
+    real ex = real(0.0), fb = real(0.0);
+    const real xa1 = X[-A], x0 = X[0], xb1 = X[A], xc1 = X[-B], xd1 = X[B];
+    if (P.advection != 0) {
+        fb = mom_vflux(P, k + 1, kff, q.x_m1, q.x_0, q.x_p1, x_p2, w_c, w_f);
+        const real a0 = real(0.5) * (xa1 + x0), a1 = real(0.5) * (x0 + xb1);      // along, at the cell centres
+        const real b0 = real(0.5) * (y0 + y2), bm = real(0.5) * (y1 + y3);        // across, at the corners
+        real al, ac;
+        if (P.advection >= 3) {
+            const bool lim = P.advection == 4;
+            const real c0 = kappa_face_f(P, X[-2 * A], xa1, x0, xb1, a0, fl & 1, fl & 2, lim);
+            const real c1 = kappa_face_f(P, xa1, x0, xb1, X[2 * A], a1, fl & 4, fl & 8, lim);
+            al = a1 * c1 - a0 * c0;
+            const real f0 = b0 * kappa_face_f(P, xc1, x0, xd1, X[2 * B], b0, fl & 16, fl & 32, lim);
+            const real fm = bm * kappa_face_f(P, X[-2 * B], xc1, x0, xd1, bm, fl & 64, fl & 128, lim);
+            ac = f0 - fm;
+        } else {
+            al = a1 * a1 - a0 * a0;
+            const real f0 = b0 * (real(0.5) * (x0 + xd1));
+            const real fm = bm * (real(0.5) * (xc1 + x0));
+            ac = f0 - fm;
+        }
+        const real h = COMP ? ac / P.dx + al / P.dy : al / P.dx + ac / P.dy;
+        const real a = h + (q.fz - fb) / P.dz_nom[k];
+        ex = ex - a * m;
+    }
+    if (P.a_h > real(0.0)) {
+        // horizontal Laplacian with face masks (hlap): of the cells around u, the x faces
+        // carry the u masks and the y faces the v masks; the same around v
+        const real g0 = ((fl >> (COMP ? 9 : 8)) & 1 ? real(1.0) : real(0.0)) * ((COMP ? xd1 : xb1) - x0) / P.dx;
+        const real gw = ((fl >> (COMP ? 10 : 2)) & 1 ? real(1.0) : real(0.0)) * (x0 - (COMP ? xc1 : xa1)) / P.dx;
+        const real h0 = ((fl >> (COMP ? 8 : 9)) & 1 ? real(1.0) : real(0.0)) * ((COMP ? xb1 : xd1) - x0) / P.dy;
+        const real hs = ((fl >> (COMP ? 2 : 10)) & 1 ? real(1.0) : real(0.0)) * (x0 - (COMP ? xa1 : xc1)) / P.dy;
+        ex = ex + P.a_h * (m * ((g0 - gw) / P.dx + (h0 - hs) / P.dy));
+    }
+    const real st = (k == 0) ? P.thv_dt * tau * rdz + P.dt * ex : real(0.0) + P.dt * ex;
+    out.st[at] = st;
+    out.rhs[at] = predictor(P, x0, COMP ? P.neg_f0 : P.f0, av, av, pg, g2, m, dz, st);
+    q.fz = fb;
+    q.df = db;
+    q.x_m1 = q.x_0;
+    q.x_0 = q.x_p1;
+    q.x_p1 = x_p2;
+}
+
+// the open faces of a component's stencil (region column rc; A, B: strides along its
+// axis and across; own and oth: wet levels of the faces of this and the other
+// component), one bit each: far cells of the two faces along (0..3) and across (4..7),
+// the face itself (8), the four faces of the Coriolis average (9..12)
+__device__ __forceinline__ unsigned mom_face_flags(const int* own, const int* oth, int rc, int A, int B) {
+    unsigned f = 0;
+    f |= (own[rc - 2 * A] > 0) << 0 | (own[rc + A] > 0) << 1 | (own[rc - A] > 0) << 2 | (own[rc + 2 * A] > 0) << 3;
+    f |= (own[rc - B] > 0) << 4 | (own[rc + 2 * B] > 0) << 5 | (own[rc - 2 * B] > 0) << 6 | (own[rc + B] > 0) << 7;
+    f |= (own[rc] > 0) << 8;
+    f |= (oth[rc] > 0) << 9 | (oth[rc - B] > 0) << 10 | (oth[rc + A] > 0) << 11 | (oth[rc + A - B] > 0) << 12;
+    return f;
+}
+
+// Bound by instruction issue, most of it the limiter's selects and divisions (five per
+// component and level that depend on data). Over a flat or gently sloping bottom most
+// levels of a tile are wet and full in every column, ring included, so a CTA first marches
+// those (mom_full_level) -- no thickness, depth or mask of any column is formed there
+// -- and the levels below in the general form. The first pass's right-hand sides are formed
+// here too, from values in registers: a pass over twelve arrays less. us a launch at
+// 512 x 512 x 50: 1114 before with 242 of a first k_predictor_rhs beside it, 1043 now (FP32 751
+// with 159, now 636).
 __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column(
     KPR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b,
     const wide* __restrict__ phi, const real* __restrict__ w, const real* __restrict__ km,
-    real* __restrict__ pgx, real* __restrict__ pgy, real* __restrict__ avpv,
-    real* __restrict__ avpu, real* __restrict__ dzu, real* __restrict__ dzv,
-    real* __restrict__ stu, real* __restrict__ stv) {
-    __shared__ int s_g[MOM_RN], s_ku[MOM_RN], s_kv[MOM_RN];
+    const wide* __restrict__ gx2, const wide* __restrict__ gy2, real* __restrict__ pgx, real* __restrict__ pgy,
+    real* __restrict__ avpv, real* __restrict__ avpu, real* __restrict__ dzu, real* __restrict__ dzv,
+    real* __restrict__ stu, real* __restrict__ stv, real* __restrict__ ru, real* __restrict__ rv) {
+    __shared__ int s_ku[MOM_RN], s_kv[MOM_RN];
+    __shared__ int s_full;
     __shared__ real s_u[2][MOM_RN], s_v[2][MOM_RN];  // level planes, double-buffered
     // threadIdx.z selects the component: 0 the u terms at the column's east face,
     // 1 the v terms at its north face (whole warps, so no divergence)
     const int tx = threadIdx.x, ty = threadIdx.y, comp = threadIdx.z;
     const int tid = (comp * MOM_TY + ty) * MOM_TX + tx;
-    const int nthreads = MOM_TX * MOM_TY * 2;
+    constexpr int NT = MOM_TX * MOM_TY * 2, NS = (MOM_RN + NT - 1) / NT;  // threads, region columns per thread
     const int i0 = blockIdx.x * MOM_TX, j0 = blockIdx.y * MOM_TY;
     const int i = i0 + tx, j = j0 + ty;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const bool live = i < nx && j < ny;
     const int kbeg = blockIdx.z * P.mom_kl;
     const int kend = kbeg + P.mom_kl < nz ? kbeg + P.mom_kl : nz;
-    for (int r = tid; r < MOM_RN; r += nthreads) {
-        const int rj = r / MOM_RX, ri = r - rj * MOM_RX;
-        const int gcol = wrapi(j0 - 2 + rj, ny) * nx + wrapi(i0 - 2 + ri, nx);
-        const int2 kfc = P.kface[gcol];
-        s_g[r] = gcol;
-        s_ku[r] = kfc.x;
-        s_kv[r] = kfc.y;
-    }
-    const int rc = (ty + 2) * MOM_RX + tx + 2;
-    const size_t n2 = (size_t)P.n2;
-    const int wi = wrapi(i, nx), wj = wrapi(j, ny);
-    const int c = wj * nx + wi;
-    // the face's far column (east for u, north for v) and its wet levels
-    const int cf = comp ? wrapi(j + 1, ny) * nx + wi : wj * nx + wrapi(i + 1, nx);
-    const ColGeoR gc = ColGeoR::load(P, c), gf = ColGeoR::load(P, cf);
-#ifdef OC_MIXED
-    // the pressure gradient's depths in fp64 (FP32 depths of ~4 km carry 2e-4 m errors)
-    const ColGeo64 gc64 = ColGeo64::load(P, c), gf64 = ColGeo64::load(P, cf);
-#endif
-    const int kff = comp ? P.kface[c].y : P.kface[c].x;
-    const real tau = comp ? P.tau_v[c] : P.tau_u[c];
-    const real* __restrict__ X = comp ? v : u;
-    // face thickness of the column's face at level kk (0 outside)
-    auto dzf_at = [&](int kk) {
-        if (kk < 0 || kk >= nz) return real(0.0);
-        real m;
-        return face_dz(P, kff, kk, gc.dz(P, kk, m), gf.dz(P, kk, m));
-    };
-    auto m3c_at = [&](int kk) { return (kk >= 0 && kk < gc.kb) ? real(1.0) : real(0.0); };
-    auto Xc = [&](int kk) { return (kk >= 0 && kk < nz) ? X[(size_t)kk * n2 + c] : real(0.0); };
-    // rolling values of the component at k-1, k, k+1 (and k+2 for advection)
-    real x_m1 = real(0.0), x_0 = real(0.0), x_p1 = real(0.0), dz_0 = real(0.0);
-    // fluxes through the top of level kbeg
-    real fz = real(0.0), df = real(0.0);
-    if (live) {
-        x_m1 = Xc(kbeg - 1);
-        x_0 = Xc(kbeg);
-        x_p1 = Xc(kbeg + 1);
-        const real dz_m1 = dzf_at(kbeg - 1);
-        dz_0 = dzf_at(kbeg);
-        const int kk = kbeg;
-        if (P.advection != 0)
-            fz = mom_vflux(P, kk, kff, Xc(kk - 2), x_m1, x_0, x_p1, w[(size_t)kk * n2 + c], w[(size_t)kk * n2 + cf]);
-        if (kk == 0) {
-            df = tau;
-        } else {
-            const real bot = (m3c_at(kk - 1) > real(0.0) && m3c_at(kk) == real(0.0)) ? real(1.0) : real(0.0);
-            df = diff_flux(km[(size_t)kbeg * n2 + c], x_m1, x_0, dz_m1, dz_0, bot);
+    if (tid == 0) s_full = nz;
+    __syncthreads();
+    // the region columns this thread stages, and the levels full in all columns
+    int gcol[NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+        const int r = tid + q * NT;
+        gcol[q] = -1;
+        if (r < MOM_RN) {
+            const int rj = r / MOM_RX, ri = r - rj * MOM_RX;
+            gcol[q] = wrapi(j0 - 2 + rj, ny) * nx + wrapi(i0 - 2 + ri, nx);
+            const int2 kfc = P.kface[gcol[q]];
+            s_ku[r] = kfc.x;
+            s_kv[r] = kfc.y;
+            // a face at the region's edge has a column outside of it, which may be shallower
+            int kf = P.kinfo[gcol[q]].x;
+            if (kfc.x > 0) kf = min(kf, kfc.x + 1);
+            if (kfc.y > 0) kf = min(kf, kfc.y + 1);
+            if (kf < nz) atomicMin(&s_full, kf);
         }
     }
     // level k's u and v of the region go to buffer (k - kbeg) & 1; level k + 1's
-    // copies are in flight while level k is computed (each thread copies the
-    // region cells whose s_g it wrote itself)
+    // copies are in flight while level k is computed
     auto stage = [&](int k) {
-        const size_t o = (size_t)k * n2;
+        const size_t o = (size_t)k * P.n2;
         const int buf = (k - kbeg) & 1;
-        for (int r = tid; r < MOM_RN; r += nthreads) {
-            cp_async_elem(&s_u[buf][r], u + o + s_g[r]);
-            cp_async_elem(&s_v[buf][r], v + o + s_g[r]);
-        }
+#pragma unroll
+        for (int q = 0; q < NS; ++q)
+            if (gcol[q] >= 0) {
+                cp_async_elem(&s_u[buf][tid + q * NT], u + o + gcol[q]);
+                cp_async_elem(&s_v[buf][tid + q * NT], v + o + gcol[q]);
+            }
         cp_async_commit();
     };
     stage(kbeg);
-    for (int k = kbeg; k < kend; ++k) {
-        const size_t o = (size_t)k * n2;
-        // every thread is done with the previous level, whose buffer level k + 1 takes
+    // the next level's plane: every thread is done with the previous level, whose buffer
+    // level k + 1 takes
+    auto next_level = [&](int k) {
         __syncthreads();
         if (k + 1 < kend) {
             stage(k + 1);
@@ -772,6 +871,76 @@ __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column
             cp_async_wait<0>();
         }
         __syncthreads();
+    };
+    const int rc = (ty + 2) * MOM_RX + tx + 2;
+    const size_t n2 = (size_t)P.n2;
+    const int wi = wrapi(i, nx), wj = wrapi(j, ny);
+    const int c = wj * nx + wi;
+    // the face's far column (east for u, north for v) and its wet levels
+    const int cf = comp ? wrapi(j + 1, ny) * nx + wi : wj * nx + wrapi(i + 1, nx);
+    const int kff = comp ? P.kface[c].y : P.kface[c].x;
+    const real tau = comp ? P.tau_v[c] : P.tau_u[c];
+    const real g2 = P.scheme != 2 ? real(comp ? gy2[c] : gx2[c]) : real(0.0);
+    const real* __restrict__ X = comp ? v : u;
+    auto Xc = [&](int kk) { return (kk >= 0 && kk < nz) ? X[(size_t)kk * n2 + c] : real(0.0); };
+    MomCarry q{real(0.0), real(0.0), real(0.0), real(0.0), real(0.0)};
+    if (live) {
+        q.x_m1 = Xc(kbeg - 1);
+        q.x_0 = Xc(kbeg);
+        q.x_p1 = Xc(kbeg + 1);
+        const size_t ob = (size_t)kbeg * n2;
+        if (P.advection != 0)
+            q.fz = mom_vflux(P, kbeg, kff, Xc(kbeg - 2), q.x_m1, q.x_0, q.x_p1, w[ob + c], w[ob + cf]);
+        if (kbeg == 0) {
+            q.df = tau;
+        } else {
+            const ColGeoR gc = ColGeoR::load(P, c), gf = ColGeoR::load(P, cf);
+            real m, m3c, m3a;
+            const real dz_m1 = face_dz(P, kff, kbeg - 1, gc.dz(P, kbeg - 1, m3a), gf.dz(P, kbeg - 1, m));
+            const real dz_0 = face_dz(P, kff, kbeg, gc.dz(P, kbeg, m3c), gf.dz(P, kbeg, m));
+            const real bot = (m3a > real(0.0) && m3c == real(0.0)) ? real(1.0) : real(0.0);
+            q.df = diff_flux(km[ob + c], q.x_m1, q.x_0, dz_m1, dz_0, bot);
+        }
+    }
+    __syncthreads();  // s_full
+    // levels [kbeg, kfull) have full columns at themselves and the level below
+    const int kfull = s_full - 1 < kend ? s_full - 1 : kend;
+    int k = kbeg;
+    if (k < kfull) {
+        const unsigned fl = comp ? mom_face_flags(s_kv, s_ku, rc, MOM_RX, 1) : mom_face_flags(s_ku, s_kv, rc, 1, MOM_RX);
+        for (; k < kfull; ++k) {
+            next_level(k);
+            if (!live) continue;
+            const size_t o = (size_t)k * n2, at = o + c, af = o + cf;
+            const int buf = (k - kbeg) & 1;
+            const real x_p2 = k + 2 < nz ? X[at + 2 * n2] : real(0.0);
+            const real K_1 = km[at + n2], w_c = w[at + n2], w_f = w[af + n2];
+            const wide phc = phi[at], phf = phi[af], bc = b[at], bf = b[af];
+            if (comp)
+                mom_full_level<1>(P, s_v[buf] + rc, s_u[buf] + rc, fl, kff, k, x_p2, K_1, w_c, w_f, phc, phf, bc, bf,
+                                  tau, g2, at, MomOut{pgy, avpu, dzv, stv, rv}, q);
+            else
+                mom_full_level<0>(P, s_u[buf] + rc, s_v[buf] + rc, fl, kff, k, x_p2, K_1, w_c, w_f, phc, phf, bc, bf,
+                                  tau, g2, at, MomOut{pgx, avpv, dzu, stu, ru}, q);
+        }
+    }
+    if (k >= kend) return;
+    const ColGeoR gc = ColGeoR::load(P, c), gf = ColGeoR::load(P, cf);
+#ifdef OC_MIXED
+    // the pressure gradient's depths in fp64 (FP32 depths of ~4 km carry 2e-4 m errors)
+    const ColGeo64 gc64 = ColGeo64::load(P, c), gf64 = ColGeo64::load(P, cf);
+#endif
+    // face thickness of the column's face at level kk (0 outside)
+    auto dzf_at = [&](int kk) {
+        if (kk < 0 || kk >= nz) return real(0.0);
+        real m;
+        return face_dz(P, kff, kk, gc.dz(P, kk, m), gf.dz(P, kk, m));
+    };
+    const MomOut out = comp ? MomOut{pgy, avpu, dzv, stv, rv} : MomOut{pgx, avpv, dzu, stu, ru};
+    real dz_0 = dzf_at(k);
+    for (; k < kend; ++k) {
+        const size_t o = (size_t)k * n2;
+        next_level(k);
         if (!live) continue;
         const int buf = (k - kbeg) & 1;
         const TileLevel lv{s_u[buf], s_v[buf], s_ku, s_kv, rc, k};
@@ -781,13 +950,13 @@ __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column
         real m3c, m3f;
         const real dz_c = gc.dz(P, k, m3c), dz_f = gf.dz(P, k, m3f);
         const real m3f_k = k < kff ? real(1.0) : real(0.0);
-        const real bottom_k = (m3c > real(0.0) && m3c_at(k + 1) == real(0.0)) ? real(1.0) : real(0.0);
+        const real bottom_k = (m3c > real(0.0) && k + 1 >= gc.kb) ? real(1.0) : real(0.0);
         // ---- pressure gradient at a common depth (model3d_v05.py:211-230), in
         // fp64 on both paths: it is a small difference of large potentials
         const wide phc = phi[o + c], phf = phi[o + cf];
         const wide bc = b[o + c], bf = b[o + cf];
         const wide dxy = comp ? P.dy64 : P.dx64;
-        wide pg;
+        wide pgw;
         if (P.pgf_correction) {
 #ifdef OC_MIXED
             const wide zc_c = gc64.above(P, k) + 0.5 * gc64.dz(P, k);
@@ -797,30 +966,31 @@ __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column
             const wide zc_f = gf.above(P, k) + 0.5 * dz_f;
 #endif
             const wide zf = 0.5 * (zc_c + zc_f);
-            pg = m3f_k * ((phf + bf * (zf - zc_f)) - (phc + bc * (zf - zc_c))) / dxy;
+            pgw = m3f_k * ((phf + bf * (zf - zc_f)) - (phc + bc * (zf - zc_c))) / dxy;
         } else {
-            pg = m3f_k * (phf - phc) / dxy * m3f_k;
+            pgw = m3f_k * (phf - phc) / dxy * m3f_k;
         }
-        (comp ? pgy : pgx)[o + c] = real(pg);
+        const real pg = real(pgw);
+        out.pg[o + c] = pg;
         // ---- Coriolis average of the old state (v at u points, u at v points)
-        if (comp)
-            avpu[o + c] = u_on_v_at(lv);
-        else
-            avpv[o + c] = v_on_u_at(lv);
+        const real av = comp ? u_on_v_at(lv) : v_on_u_at(lv);
+        out.av[o + c] = av;
         // ---- explicit vertical diffusion: top flux carried, bottom flux formed here
-        const real db = (k < nz - 1) ? diff_flux(K_1, x_0, x_p1, dz_0, dz_p1, bottom_k) : real(0.0);
+        const real db = (k < nz - 1) ? diff_flux(K_1, q.x_0, q.x_p1, dz_0, dz_p1, bottom_k) : real(0.0);
+        real dz;
         {
             const real mk = m3c > real(0.0) ? real(1.0) : real(0.0);
             const real id = inv_pos(dz_0);
-            const real out = (df - db) * id;
-            const real drag = P.bottom_drag * x_0 * bottom_k;
-            (comp ? dzv : dzu)[o + c] = (out - drag * id) * mk;
+            const real flux = (q.df - db) * id;
+            const real drag = P.bottom_drag * q.x_0 * bottom_k;
+            dz = (flux - drag * id) * mk;
         }
+        out.dz[o + c] = dz;
         // ---- advection and horizontal viscosity, then the stress increment
         real ex = real(0.0), fb = real(0.0);
         if (P.advection != 0) {
-            fb = mom_vflux(P, k + 1, kff, x_m1, x_0, x_p1, x_p2, w[o + n2 + c], w[o + n2 + cf]);
-            const real a = (comp ? mom_adv_v_xy(P, lv) : mom_adv_u_xy(P, lv)) + (fz - fb) / P.dz_nom[k];
+            fb = mom_vflux(P, k + 1, kff, q.x_m1, q.x_0, q.x_p1, x_p2, w[o + n2 + c], w[o + n2 + cf]);
+            const real a = (comp ? mom_adv_v_xy(P, lv) : mom_adv_u_xy(P, lv)) + (q.fz - fb) / P.dz_nom[k];
             ex = ex - a * m3f_k;
         }
         if (P.a_h > real(0.0)) {
@@ -828,21 +998,22 @@ __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column
             nb.init(wi, wj, nx, ny);
             ex = ex + P.a_h * hlap(P, nb, X, k, comp);
         }
-        (comp ? stv : stu)[o + c] = (k == 0) ? P.thv_dt * tau * inv_pos(dz_0) + P.dt * ex : real(0.0) + P.dt * ex;
+        const real st = (k == 0) ? P.thv_dt * tau * inv_pos(dz_0) + P.dt * ex : real(0.0) + P.dt * ex;
+        out.st[o + c] = st;
+        out.rhs[o + c] = predictor(P, q.x_0, comp ? P.neg_f0 : P.f0, av, av, pg, g2, m3f_k, dz, st);
         // roll down one level
-        fz = fb;
-        df = db;
-        x_m1 = x_0;
-        x_0 = x_p1;
-        x_p1 = x_p2;
+        q.fz = fb;
+        q.df = db;
+        q.x_m1 = q.x_0;
+        q.x_0 = q.x_p1;
+        q.x_p1 = x_p2;
         dz_0 = dz_p1;
     }
 }
 
 // ------------------------------------------------------------------ predictor + column solves
-// Per cell, for one Picard iteration: the explicit predictors with the iterate's
-// Coriolis average plus the stress/advection increment -- the right-hand sides
-// of the two momentum tridiagonals (model3d_v05.py:387-393).
+// Per cell, for a Picard iteration after the first (whose right-hand sides
+// k_mom_column forms): both right-hand sides with the iterate's Coriolis averages.
 __global__ void __launch_bounds__(256) k_predictor_rhs(
     KPR P, const real* __restrict__ u, const real* __restrict__ v,
     const real* __restrict__ u_it, const real* __restrict__ v_it,
@@ -858,29 +1029,14 @@ __global__ void __launch_bounds__(256) k_predictor_rhs(
     if (i >= P.nx || j >= P.ny) return;
     const int c = j * P.nx + i;
     const size_t o = (size_t)k * P.n2;
-    const real av_v = avpv[o + c], av_u = avpu[o + c];
-    // the iterate's averages; in the first pass the iterate is the old state,
-    // whose averages the explicit-terms kernel formed already by the same function
-    real it_v = av_v, it_u = av_u;
-    if (u_it != u || v_it != v) {
-        Nbr nb;
-        nb.init(i, j, P.nx, P.ny);
-        it_v = v_on_u(P, nb, v_it, o, k);
-        it_u = u_on_v(P, nb, u_it, o, k);
-    }
-    const real vcor = P.one_m_tc * av_v + P.theta_cor * it_v;
-    const real ucor = P.one_m_tc * av_u + P.theta_cor * it_u;
-    real gu, gv;
-    if (P.scheme != 2) {
-        const real m3u_k = col_m3u(P, c, k), m3v_k = col_m3v(P, c, k);
-        gu = u[o + c] + P.dt * (P.f0 * vcor + pgx[o + c]) - P.c1 * (real(gx2[c]) * m3u_k) + P.c3 * dzu[o + c];
-        gv = v[o + c] + P.dt * (P.neg_f0 * ucor + pgy[o + c]) - P.c1 * (real(gy2[c]) * m3v_k) + P.c3 * dzv[o + c];
-    } else {
-        gu = u[o + c] + P.dt * (P.f0 * vcor + pgx[o + c]) + P.c3 * dzu[o + c];
-        gv = v[o + c] + P.dt * (P.neg_f0 * ucor + pgy[o + c]) + P.c3 * dzv[o + c];
-    }
-    ru[o + c] = gu + stu[o + c];
-    rv[o + c] = gv + stv[o + c];
+    Nbr nb;
+    nb.init(i, j, P.nx, P.ny);
+    const real it_v = v_on_u(P, nb, v_it, o, k), it_u = u_on_v(P, nb, u_it, o, k);
+    const real g2x = P.scheme != 2 ? real(gx2[c]) : real(0.0), g2y = P.scheme != 2 ? real(gy2[c]) : real(0.0);
+    ru[o + c] = predictor(P, u[o + c], P.f0, avpv[o + c], it_v, pgx[o + c], g2x, col_m3u(P, c, k), dzu[o + c],
+                          stu[o + c]);
+    rv[o + c] = predictor(P, v[o + c], P.neg_f0, avpu[o + c], it_u, pgy[o + c], g2y, col_m3v(P, c, k), dzv[o + c],
+                          stv[o + c]);
 }
 
 // Per column: both momentum tridiagonals with the cell column's rows
@@ -1439,12 +1595,12 @@ void launch_phi(const KPR& P, const wide* b, wide* phi, cudaStream_t s) {
 static dim3 cell_block() { return dim3(32, 8, 1); }
 static dim3 cell_grid(const KPR& P) { return dim3((P.nx + 31) / 32, (P.ny + 7) / 8, P.nz); }
 void launch_mom_explicit(const KPR& P, const real* u, const real* v, const wide* b,
-                         const wide* phi, const real* w, const real* km, real* pgx,
-                         real* pgy, real* avpv, real* avpu, real* dzu, real* dzv,
-                         real* stu, real* stv, cudaStream_t s) {
+                         const wide* phi, const real* w, const real* km, const wide* gx2, const wide* gy2,
+                         real* pgx, real* pgy, real* avpv, real* avpu, real* dzu, real* dzv, real* stu, real* stv,
+                         real* ru, real* rv, cudaStream_t s) {
     const dim3 grid((P.nx + MOM_TX - 1) / MOM_TX, (P.ny + MOM_TY - 1) / MOM_TY, (P.nz + P.mom_kl - 1) / P.mom_kl);
-    k_mom_column<<<grid, dim3(MOM_TX, MOM_TY, 2), 0, s>>>(P, u, v, b, phi, w, km, pgx, pgy, avpv, avpu, dzu, dzv, stu,
-                                             stv);
+    k_mom_column<<<grid, dim3(MOM_TX, MOM_TY, 2), 0, s>>>(P, u, v, b, phi, w, km, gx2, gy2, pgx, pgy, avpv, avpu, dzu, dzv,
+                                             stu, stv, ru, rv);
 }
 void launch_predictor_rhs(const KPR& P, const real* u, const real* v, const real* u_it,
                           const real* v_it, const real* pgx, const real* pgy, const real* avpv,

@@ -19,9 +19,9 @@ namespace oc {
     void launch_wcol(const KPT<R>& P, const R* u, const R* v, R* w, cudaStream_t s);                            \
     void launch_phi(const KPT<R>& P, const double* b, double* phi, cudaStream_t s);                             \
     void launch_mom_explicit(const KPT<R>& P, const R* u, const R* v, const double* b, const double* phi,      \
-                             const R* w, const R* km, R* pgx, R* pgy, R* avpv, R* avpu, R* dzu, R* dzv, R* stu, \
-                             R* stv, cudaStream_t s);                                                           \
-    /* right-hand sides of the two momentum tridiagonals for one Picard pass (per cell) */                     \
+                             const R* w, const R* km, const double* gx2, const double* gy2, R* pgx, R* pgy,    \
+                             R* avpv, R* avpu, R* dzu, R* dzv, R* stu, R* stv, R* ru, R* rv, cudaStream_t s);  \
+    /* right-hand sides of the momentum tridiagonals for a later Picard pass (per cell) */                      \
     void launch_predictor_rhs(const KPT<R>& P, const R* u, const R* v, const R* u_it, const R* v_it,           \
                               const R* pgx, const R* pgy, const R* avpv, const R* avpu, const R* dzu,           \
                               const R* dzv, const R* stu, const R* stv, const double* gx2, const double* gy2,   \
