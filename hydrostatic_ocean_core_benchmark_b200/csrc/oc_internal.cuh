@@ -70,6 +70,7 @@ struct KPT {
     // where both columns of a face have their full thickness: the face's thickness at
     // level k, 1 over it, and 1 over the spacing of the interface between k - 1 and k
     T fdz[OC_MAXNZ], rfdz[OC_MAXNZ], rfdzi[OC_MAXNZ];
+    T rdz[OC_MAXNZ], rdzi[OC_MAXNZ];  // the same reciprocals of a full column's cells
     // static 2D fields
     const T* H;
     const T* mask;

@@ -1158,6 +1158,10 @@ __global__ void k_backsub(KPR P, const real* __restrict__ ghu, const real* __res
 // cell is carried to the next level as the face at its top, and the column's
 // tracer values, w and K_h roll in registers. Every face and cell value is
 // formed by the reference's operations in the reference's order.
+// Bound by instruction issue: the levels that are wet and full in every column of the tile
+// and its ring, most of them over a flat bottom, take thicknesses and reciprocals from the
+// level table and need no mask but the open faces. 512 x 512 x 50: 887 us a launch with one
+// form for all levels, 694 with the short one above the general one (FP32 548, now 438).
 constexpr int TRX = 32, TRY = 8;
 
 struct Stencil4 {
@@ -1237,6 +1241,7 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P,
     __shared__ real s_d0[RNC], s_d1[RNC];
     // level planes, double-buffered: [buffer][field] tracers, [buffer] face velocities
     __shared__ real s_f[2][2][RNC], s_u[2][RNC], s_v[2][RNC];
+    __shared__ int s_full;  // levels that are full in every column of the region
     __shared__ real sfx[2][TRY][TRX + 1];  // [field][row][west face of column]
     __shared__ real sfy[2][TRY + 1][TRX];  // [field][south face of row][column]
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -1257,6 +1262,8 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P,
     const int c = wrapi(j, ny) * nx + wrapi(i, nx);
     const ColGeoR g = ColGeoR::load(P, c);
     real* __restrict__ R0 = rT;
+    if (tid == 0) s_full = nz;
+    __syncthreads();
     for (int r = tid; r < RNC; r += TRX * TRY) {
         const int rj = r / RX, ri = r - rj * RX;
         const int gc = wrapi(j0 - 2 + rj, ny) * nx + wrapi(i0 - 2 + ri, nx);
@@ -1266,6 +1273,7 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P,
         s_k[r] = make_uchar4((unsigned char)ki.x, (unsigned char)ki.y, (unsigned char)kfc.x, (unsigned char)kfc.y);
         s_d0[r] = dx.x;
         s_d1[r] = dx.y;
+        if (ki.x < nz) atomicMin(&s_full, ki.x);
     }
     // thickness and wet flag of region column r at level k (col_dz from the staged geometry)
     auto sdz = [&](int r, int k, real& m3) {
@@ -1329,19 +1337,114 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P,
         }
         cp_async_commit();
     };
+    // the level's plane in place, level k + 1's on its way: every thread is done with the
+    // previous level, whose buffer level k + 1 takes
+    auto next_level = [&](int k) {
+        __syncthreads();
+        if (k + 1 < kend) {
+            stage(k + 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+    };
     if (adv) stage(kbeg);
-    for (int k = kbeg; k < kend; ++k) {
+    __syncthreads();  // s_full
+    // Levels [kbeg, kfull): every column of the region is wet and full there and one level
+    // below. Thicknesses and their reciprocals come from the level table, every far cell
+    // is wet, a face has the level's thickness or none (fl: open west, south, east and
+    // north faces of the cell; of the extra faces, the one this thread forms), and the
+    // diffusive flux at a cell's bottom is carried to the next level's top as the
+    // advective face is. The values are the general form's, operation for operation.
+    int k = kbeg;
+    const int kfull = s_full - 1 < kend ? s_full - 1 : kend;
+    if (k < kfull) {
+        const unsigned fl = (s_k[rc - 1].z > 0 ? 1u : 0u) | (s_k[rc - RX].w > 0 ? 2u : 0u) |
+                            (s_k[rc].z > 0 ? 4u : 0u) | (s_k[rc].w > 0 ? 8u : 0u);
+        const bool xopen = xextra && s_k[rce].z > 0, yopen = yextra && s_k[rcn].w > 0;
+        real dtop[2] = {real(0.0), real(0.0)};  // diffusive flux through the top of level k
+        if (live)
+#pragma unroll
+            for (int f = 0; f < 2; ++f)
+                dtop[f] = k == 0 ? (ts ? (f == 0 ? P.flux_t : P.flux_s) : real(0.0))
+                                 : kh_k * (fm1[f] - f0[f]) * P.rdzi[k];
+        // flux through a face whose upstream-side and downstream-side cells are c0 and c0 + st
+        auto fflux = [&](const real* F, int c0, int st, real vel, real dzf) {
+            const real a = F[c0], b = F[c0 + st];
+            real val;
+            if (P.advection == 1) val = real(0.5) * (a + b);
+            else if (P.advection >= 3) val = kappa_face_f(P, F[c0 - st], a, b, F[c0 + 2 * st], vel, true, true, P.advection == 4);
+            else val = vel > real(0.0) ? a : b;
+            return dzf * vel * val;
+        };
+        for (; k < kfull; ++k) {
+            const size_t o = (size_t)k * n2;
+            const int buf = (k - kbeg) & 1;
+            if (adv) {
+                next_level(k);
+                const real* su = s_u[buf];
+                const real* sv = s_v[buf];
+                const real dzf = P.fdz[k];
+#pragma unroll 1
+                for (int f = 0; f < nf; ++f) {
+                    const real* F = s_f[buf][f];
+                    sfx[f][ty][tx] = fflux(F, rc - 1, 1, su[rc - 1], fl & 1 ? dzf : real(0.0));
+                    sfy[f][ty][tx] = fflux(F, rc - RX, RX, sv[rc - RX], fl & 2 ? dzf : real(0.0));
+                    if (xextra) sfx[f][tx][TRX] = fflux(F, rce, 1, su[rce], xopen ? dzf : real(0.0));
+                    if (yextra) sfy[f][TRY][tx] = fflux(F, rcn, RX, sv[rcn], yopen ? dzf : real(0.0));
+                }
+                __syncthreads();
+            }
+            if (!live) continue;
+            const real w_k1 = w[o + n2 + c];
+            const real kh_k1 = kh[o + n2 + c];
+            const real inv = P.rdz[k];
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+                if (f >= nf) break;
+                const real* __restrict__ C = f == 0 ? C0 : S;
+                const real fp2 = (k + 2 < nz) ? C[o + 2 * n2 + c] : real(0.0);
+                const real surf = ts ? (f == 0 ? P.flux_t : P.flux_s) : real(0.0);
+                real tend = ts ? real(0.0) : P.neg_n2 * (real(0.5) * (w_k + w_k1));
+                real fbot = real(0.0);
+                if (adv) {
+                    fbot = tracer_vface(P, g, k + 1, fm1[f], f0[f], fp1[f], fp2, w_k1);
+                    const real hdiv = ((sfx[f][ty][tx + 1] - sfx[f][ty][tx]) / P.dx +
+                                       (sfy[f][ty + 1][tx] - sfy[f][ty][tx]) / P.dy) * inv;
+                    const real vdiv = (w_k * ftop[f] - w_k1 * fbot) * inv;
+                    tend = tend - (hdiv + vdiv);
+                }
+                if (P.k_h > real(0.0)) {
+                    // hlap with the level's open faces; F from global memory, as the tile is staged
+                    // only with advection
+                    const int ce = wrapi(j, ny) * nx + wrapi(i + 1, nx), cw = wrapi(j, ny) * nx + wrapi(i - 1, nx);
+                    const int cn = wrapi(j + 1, ny) * nx + wrapi(i, nx), cs = wrapi(j - 1, ny) * nx + wrapi(i, nx);
+                    const real gx0 = (fl & 4 ? real(1.0) : real(0.0)) * (C[o + ce] - f0[f]) / P.dx;
+                    const real gxw = (fl & 1 ? real(1.0) : real(0.0)) * (f0[f] - C[o + cw]) / P.dx;
+                    const real gy0 = (fl & 8 ? real(1.0) : real(0.0)) * (C[o + cn] - f0[f]) / P.dy;
+                    const real gys = (fl & 2 ? real(1.0) : real(0.0)) * (f0[f] - C[o + cs]) / P.dy;
+                    tend = tend + P.k_h * ((gx0 - gxw) / P.dx + (gy0 - gys) / P.dy);
+                }
+                const real dbot = kh_k1 * (f0[f] - fp1[f]) * P.rdzi[k + 1];
+                const real diff = (dtop[f] - dbot) * inv;
+                real rhs = f0[f] + P.dt * tend + P.c3 * diff;
+                if (k == 0) rhs = rhs + P.thv_dt * surf * inv;
+                (f == 0 ? R0 : rS)[o + c] = rhs;
+                dtop[f] = dbot;
+                ftop[f] = fbot;
+                fm1[f] = f0[f];
+                f0[f] = fp1[f];
+                fp1[f] = fp2;
+            }
+            w_k = w_k1;
+            kh_k = kh_k1;
+        }
+    }
+    for (; k < kend; ++k) {
         const size_t o = (size_t)k * n2;
         if (adv) {
-            // every thread is done with the previous level, whose buffer level k + 1 takes
-            __syncthreads();
-            if (k + 1 < kend) {
-                stage(k + 1);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncthreads();
+            next_level(k);
             const int buf = (k - kbeg) & 1;
             const real* su = s_u[buf];
             const real* sv = s_v[buf];
