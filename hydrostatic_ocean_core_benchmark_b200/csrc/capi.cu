@@ -662,7 +662,8 @@ static int set_domain_impl(oc_handle* h, const double* Hh, const double* maskh, 
         const double dzi = k > 0 ? 0.5 * (P.fdz[k - 1] + P.fdz[k]) : 0.0;
         P.rfdzi[k] = dzi > 0.0 ? 1.0 / dzi : 0.0;
         P.rdz[k] = 1.0 / P.dzr[k];  // level thicknesses are positive
-        P.rdzi[k] = k > 0 ? 1.0 / (0.5 * (P.dzr[k - 1] + P.dzr[k])) : 0.0;
+        P.dzi[k] = k > 0 ? 0.5 * (P.dzr[k - 1] + P.dzr[k]) : P.dzr[0];
+        P.rdzi[k] = k > 0 ? 1.0 / P.dzi[k] : 0.0;
     }
     for (int k = 0; k <= nz; ++k) P.edge64[k] = P.edge[k];
     for (int k = 0; k < nz; ++k) P.dzr64[k] = P.dzr[k];

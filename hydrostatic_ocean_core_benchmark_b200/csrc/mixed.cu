@@ -101,7 +101,8 @@ void convert_params(const KP& a, KPT<float>& b) {
         const float dzi = k > 0 ? 0.5f * (b.fdz[k - 1] + b.fdz[k]) : 0.0f;
         b.rfdzi[k] = dzi > 0.0f ? 1.0f / dzi : 0.0f;
         b.rdz[k] = 1.0f / b.dzr[k];
-        b.rdzi[k] = k > 0 ? 1.0f / (0.5f * (b.dzr[k - 1] + b.dzr[k])) : 0.0f;
+        b.dzi[k] = k > 0 ? 0.5f * (b.dzr[k - 1] + b.dzr[k]) : b.dzr[0];
+        b.rdzi[k] = k > 0 ? 1.0f / b.dzi[k] : 0.0f;
     }
     b.kinfo = a.kinfo, b.kface = a.kface, b.face_rule = a.face_rule;
     b.mom_kl = a.mom_kl, b.tr_kl = a.tr_kl;

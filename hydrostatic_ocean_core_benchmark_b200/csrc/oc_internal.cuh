@@ -71,6 +71,7 @@ struct KPT {
     // level k, 1 over it, and 1 over the spacing of the interface between k - 1 and k
     T fdz[OC_MAXNZ], rfdz[OC_MAXNZ], rfdzi[OC_MAXNZ];
     T rdz[OC_MAXNZ], rdzi[OC_MAXNZ];  // the same reciprocals of a full column's cells
+    T dzi[OC_MAXNZ];                  // and the interface spacing itself (0: the level below it)
     // static 2D fields
     const T* H;
     const T* mask;
@@ -148,6 +149,18 @@ struct ColGeoT {
         m3 = T(1.0);
         if (k < kf) return P.dzr[k];
         return k == kf ? d0 : d1;
+    }
+    // 1 over the thickness of level k, and over the spacing of the interface between
+    // k - 1 and k: from the level table while the column is full there, so no division
+    __device__ __forceinline__ T rdz(const KPT<T>& P, int k) const {
+        T m;
+        return k < kf ? P.rdz[k] : inv_pos(dz(P, k, m));
+    }
+    __device__ __forceinline__ T rdzi(const KPT<T>& P, int k) const {
+        if (k < kf) return P.rdzi[k];
+        T m;
+        const T a = dz(P, k - 1, m);
+        return inv_pos(T(0.5) * (a + dz(P, k, m)));
     }
     // depth of the top of level k: the sequential sum of the thicknesses above
     // (col_above with the column's geometry in registers)

@@ -68,16 +68,16 @@ __device__ __forceinline__ T face_dz(const KPT<T>& P, int kf, int k, T dza, T dz
     return (k < kf ? T(1.0) : T(0.0)) * face_combine(P, dza, dzb);
 }
 
-// Row k of A = I - thv dt Dz for a column (reference vertical_var.py:35-77).
+// Row k of A = I - thv dt Dz for a column (reference vertical_var.py:35-77) from the
+// reciprocals of its thickness (inv_dz) and of the interface spacings above (level 0:
+// its thickness) and below it (the last level: not used).
 template <class real>
-__device__ __forceinline__ void implicit_row(const KPT<real>& P, int k, real dzk, real m3k, real m3k1,
-                                             real dzi_k, real dzi_k1, real Kk, real Kk1,
-                                             real thv_dt_drag, real& sub, real& diag,
-                                             real& sup) {
-    const real inv_dz = inv_pos(dzk);
+__device__ __forceinline__ void implicit_row_inv(const KPT<real>& P, int k, real inv_dz, real m3k, real m3k1,
+                                                 real inv_dzi_k, real inv_dzi_k1, real Kk, real Kk1,
+                                                 real thv_dt_drag, real& sub, real& diag, real& sup) {
     const real fac = P.thv_dt * inv_dz;
-    const real at = fac * Kk * inv_pos(dzi_k);
-    const real ab = fac * Kk1 * inv_pos(dzi_k1);
+    const real at = fac * Kk * inv_dzi_k;
+    const real ab = fac * Kk1 * inv_dzi_k1;
     sub = -at;
     sup = -ab;
     diag = real(1.0) + at + ab;
@@ -94,6 +94,16 @@ __device__ __forceinline__ void implicit_row(const KPT<real>& P, int k, real dzk
         sub = real(0.0);
         sup = real(0.0);
     }
+}
+
+// the same from the thicknesses and spacings themselves
+template <class real>
+__device__ __forceinline__ void implicit_row(const KPT<real>& P, int k, real dzk, real m3k, real m3k1,
+                                             real dzi_k, real dzi_k1, real Kk, real Kk1,
+                                             real thv_dt_drag, real& sub, real& diag,
+                                             real& sup) {
+    implicit_row_inv(P, k, inv_pos(dzk), m3k, m3k1, inv_pos(dzi_k), inv_pos(dzi_k1), Kk, Kk1, thv_dt_drag, sub, diag,
+                     sup);
 }
 
 // one thread per column, 32 x 4 columns per CTA

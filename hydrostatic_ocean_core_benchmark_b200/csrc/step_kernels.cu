@@ -87,6 +87,7 @@ __device__ __forceinline__ real m3_at(const KPR& P, const Nbr& n, int dj, int di
 // interface spacing of the column (closure.py:43-62): dz[0] at the surface,
 // dz[nz-1] at the bottom, the mean of the two levels elsewhere
 __device__ __forceinline__ real col_dzi(const KPR& P, const ColGeoR& g, int k) {
+    if (k < g.kf) return P.dzi[k];
     real m;
     if (k == 0) return g.dz(P, 0, m);
     if (k == P.nz) return g.dz(P, P.nz - 1, m);
@@ -102,18 +103,16 @@ template <class KM>
 __device__ __forceinline__ void column_q(const KPR& P, const ColGeoR& g, KM Km, real* cs,
                                          real* __restrict__ q, int c, size_t n2) {
     const int nz = P.nz;
-    real m3_k, dz_k = g.dz(P, 0, m3_k);
-    real dzi_k = dz_k;
+    real rdzi_k = g.rdz(P, 0);
     real km_k = Km(0);
     real ds = real(0.0), cp = real(0.0);
 #pragma unroll 2
     for (int k = 0; k < nz; ++k) {
-        real m3_k1 = real(0.0), dz_k1 = real(0.0);
-        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
-        const real dzi_k1 = (k + 1 < nz) ? real(0.5) * (dz_k + dz_k1) : dz_k;
+        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
+        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
         const real km_k1 = Km(k + 1);
         real sub, diag, sup;
-        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
+        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
         if (k == 0) {
             cp = sup / diag;
             ds = real(1.0) / diag;
@@ -125,9 +124,7 @@ __device__ __forceinline__ void column_q(const KPR& P, const ColGeoR& g, KM Km, 
         cs[k] = cp;
         if (k + 1 < nz) q[(size_t)k * n2 + c] = ds;
         km_k = km_k1;
-        dz_k = dz_k1;
-        m3_k = m3_k1;
-        dzi_k = dzi_k1;
+        rdzi_k = rdzi_k1;
     }
     real x = ds;
     q[(size_t)(nz - 1) * n2 + c] = x;
@@ -152,10 +149,15 @@ __global__ void __launch_bounds__(128) k_qsolve(KPR P, const real* __restrict__ 
 // ------------------------------------------------------------------ TKE closure
 // One thread per column (closure.py:141-205): shear and N^2 on interfaces, the
 // mixing lengths, the implicit TKE tridiagonal (nz+1 rows), K_m/K_h, then q for
-// the new K_m. Only N^2, shear^2, the new K_m and the elimination coefficients
-// are kept per thread; the elimination right-hand sides go to e (whose old value
-// at a level is read just before) and q. With the Gaspar lengths, the lengths
-// of interface k are formed inside the forward sweep.
+// the new K_m. With the Gaspar lengths, the lengths of interface k are formed inside
+// the forward sweep. Per thread only N^2, shear^2 and column_q's elimination
+// coefficients are kept: an array per thread is in local memory, which at 512 x 512 does
+// not fit the caches (1.5 KB a column), while e, q and kh are there anyway -- the
+// elimination's right-hand sides go to e (whose old value at a level is read just
+// before), its coefficients to q, the mixing lengths to kh until K_h replaces them.
+// Reciprocals of full columns' thicknesses and spacings come from the level table.
+// 512 x 512 x 50: 817 us a launch before, 750 now (FP32 542 and 465); fewer CTAs per SM
+// make it slower, so its loads' latency bounds it, not the caches' size.
 template <int NZM>
 __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const real* __restrict__ u,
                                                  const real* __restrict__ v,
@@ -180,7 +182,8 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
 #ifndef OC_MIXED
     real nn2[NZM + 1];
 #endif
-    real sh2[NZM + 1], lk[NZM + 1], le[NZM + 1], cst[NZM + 1];
+    real le[NZM + 1], cst[NZM];
+    real sh2[NZM + 1];
     real depth = real(0.0);
     for (int k = 0; k < nz; ++k) {
         real m;
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
     }
     // shear^2 and N^2 on interfaces (closure.py:150-161)
     {
-        real uc_prev = real(0.0), vc_prev = real(0.0), dz_prev = real(0.0), m3_prev = real(0.0);
+        real uc_prev = real(0.0), vc_prev = real(0.0);
         wide b_prev = 0.0;
 #pragma unroll 2
         for (int k = 0; k < nz; ++k) {
@@ -197,29 +200,25 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
             const real uc = real(0.5) * (u[o + c] + u[o + cw]);
             const real vc = real(0.5) * (v[o + c] + v[o + cs_]);
             const wide bk = b[o + c];
-            real m3k;
-            const real dzk = g.dz(P, k, m3k);
             if (k >= 1) {
-                const real wk = m3_prev * m3k;
-                const real idz = inv_pos(real(0.5) * (dz_prev + dzk));
+                const real wk = k < g.kb ? real(1.0) : real(0.0);
+                const real idz = g.rdzi(P, k);
                 const real du = (uc_prev - uc) * idz;
                 const real dv = (vc_prev - vc) * idz;
+                sh2[k] = (du * du + dv * dv) * wk;
                 // the difference of two fp64 buoyancies (their ~1e-2 relative
                 // vertical contrast would lose digits in FP32)
                 const real db = real((b_prev - bk) * idz);
-                sh2[k] = (du * du + dv * dv) * wk;
                 nn2[k] = db * wk;
             }
             uc_prev = uc;
             vc_prev = vc;
             b_prev = bk;
-            dz_prev = dzk;
-            m3_prev = m3k;
         }
     }
     sh2[0] = real(0.0);
-    nn2[0] = real(0.0);
     sh2[nz] = real(0.0);
+    nn2[0] = real(0.0);
     nn2[nz] = real(0.0);
     // recursive lengths (closure.py:106-129) need whole-column sweeps first
     if (P.mxl_recursive) {
@@ -235,15 +234,6 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
         }
         for (int k = 1; k <= nz; ++k) le[k] = fmin(le[k], le[k - 1] + col_dzi(P, g, k));
         for (int k = nz - 1; k >= 0; --k) le[k] = fmin(le[k], le[k + 1] + col_dzi(P, g, k + 1));
-        for (int k = 0; k <= nz; ++k) {
-            real m0, m1;
-            g.dz(P, k >= 1 ? k - 1 : 0, m0);
-            g.dz(P, k, m1);
-            const real wk = (k >= 1 && k <= nz - 1) ? m0 * m1 : real(0.0);
-            const real ell = le[k] * wk;
-            lk[k] = fmax(P.l_min, sqrt(ell * ell));
-            le[k] = fmax(P.l_min, fmin(ell, ell));
-        }
     }
     // implicit TKE rows and forward sweep (closure.py:171-198)
     real rhs0 = real(0.0), ds = real(0.0), cp = real(0.0), zi = real(0.0);
@@ -254,8 +244,9 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
         const size_t o = (size_t)k * n2 + c;
         const real km_next = (k < nz) ? km[o + n2] : real(0.0);
         const real wk = (k >= 1 && k <= nz - 1) ? m3_km1 * m3_k : real(0.0);
-        const real e_old = e[o];
-        real le_k;
+        const real e_old = e[o], kh_old = kh[o];
+        const real sh2_k = sh2[k];
+        real le_k, lk_k;
         if (!P.mxl_recursive) {
             // Gaspar lengths (closure.py:65-104): march away from interface k
             // until the energy budget is spent; once the budget is zero the
@@ -292,18 +283,21 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
             }
             lu = fmin(lu, zi + P.z_0) * wk;
             ld = fmin(ld, zb + P.z_0) * wk;
-            lk[k] = fmax(P.l_min, sqrt(lu * ld));
+            lk_k = fmax(P.l_min, sqrt(lu * ld));
             le_k = fmax(P.l_min, fmin(lu, ld));
         } else {
-            le_k = le[k];
+            const real ell = le[k] * wk;
+            lk_k = fmax(P.l_min, sqrt(ell * ell));
+            le_k = fmax(P.l_min, fmin(ell, ell));
         }
-        const real prod = (km_cur - P.nu) * sh2[k] - (kh[o] - P.kappa) * nn2[k];
+        kh[o] = lk_k;  // until the back substitution, which turns it into K_h
+        const real prod = (km_cur - P.nu) * sh2_k - (kh_old - P.kappa) * nn2[k];
         const real diss = P.c_eps * sqrt(fmax(e_old, P.e_min)) / le_k;
         real a_up = real(0.0), a_dn = real(0.0);
         if (k >= 1 && k <= nz - 1) {
-            const real idzi = inv_pos(real(0.5) * (dz_km1 + dz_k));
-            a_up = P.dt * (real(0.5) * (km_prev + km_cur)) * inv_pos(dz_km1) * idzi;
-            a_dn = P.dt * (real(0.5) * (km_cur + km_next)) * inv_pos(dz_k) * idzi;
+            const real idzi = g.rdzi(P, k);
+            a_up = P.dt * (real(0.5) * (km_prev + km_cur)) * g.rdz(P, k - 1) * idzi;
+            a_dn = P.dt * (real(0.5) * (km_cur + km_next)) * g.rdz(P, k) * idzi;
         }
         real sub = -a_up, sup = -a_dn;
         real diag = real(1.0) + a_up + a_dn + P.dt * diss;
@@ -324,7 +318,7 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
             cp = sup / den;
             ds = (rhs - sub * ds) / den;
         }
-        cst[k] = cp;
+        if (k < nz) q[o] = cp;  // the elimination coefficients, until column_q
         e[o] = ds;
         km_prev = km_cur;
         km_cur = km_next;
@@ -341,7 +335,7 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
     real x = real(0.0);
     for (int k = nz; k >= 0; --k) {
         const size_t o = (size_t)k * n2 + c;
-        x = (k == nz) ? ds : e[o] - cst[k] * x;
+        x = (k == nz) ? ds : e[o] - q[o] * x;
         real m0, m1;
         g.dz(P, k >= 1 ? k - 1 : 0, m0);
         g.dz(P, k < nz ? k : 0, m1);
@@ -349,14 +343,14 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
         real en = fmax(x, P.e_min);
         en = (wk > real(0.0)) ? en : P.e_min;
         if (k == 0) en = rhs0;
-        const real kmn = P.c_k * lk[k] * sqrt(en) * wk + P.nu;
-        const real khn = (kmn - P.nu) / P.pr_t + P.kappa;
+        const real kmn = P.c_k * kh[o] * sqrt(en) * wk + P.nu;
+        const real kx = kmn - P.nu;
+        const real khn = (P.pr_t == real(1.0) ? kx : kx / P.pr_t) + P.kappa;
         e[o] = en;
         km[o] = kmn;
         kh[o] = khn;
-        lk[k] = kmn;
     }
-    column_q(P, g, [&](int k) { return lk[k]; }, cst, q, c, n2);
+    column_q(P, g, [&](int k) { return km[(size_t)k * n2 + c]; }, cst, q, c, n2);
 }
 
 // ------------------------------------------------------------------ Ku, Kv
@@ -1057,8 +1051,7 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
     const int c = nb.c;
     const ColGeoR g = ColGeoR::load(P, c);
     real cs[NZM];
-    real m3_k, dz_k = g.dz(P, 0, m3_k);
-    real dzi_k = dz_k;
+    real rdzi_k = g.rdz(P, 0);
     real km_k = km[c];
     real du = real(0.0), dv = real(0.0), cp = real(0.0);
 #pragma unroll 4
@@ -1066,11 +1059,10 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
         const size_t o = (size_t)k * n2 + c;
         const real km_k1 = km[o + n2];
         const real ru = ghu[o], rv = ghv[o];
-        real m3_k1 = real(0.0), dz_k1 = real(0.0);
-        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
-        const real dzi_k1 = (k + 1 < nz) ? real(0.5) * (dz_k + dz_k1) : dz_k;
+        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
+        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
         real sub, diag, sup;
-        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
+        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
         if (k == 0) {
             cp = sup / diag;
             du = ru / diag;
@@ -1085,9 +1077,7 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
         ghu[o] = du;
         ghv[o] = dv;
         km_k = km_k1;
-        dz_k = dz_k1;
-        m3_k = m3_k1;
-        dzi_k = dzi_k1;
+        rdzi_k = rdzi_k1;
     }
     real xu = du, xv = dv;
     {
@@ -1532,21 +1522,19 @@ __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restr
 #else
     real* __restrict__ o1 = ts ? T_out : b_out;
 #endif
-    real m3_k, dz_k = g.dz(P, 0, m3_k);
-    real dzi_k = dz_k;
+    real rdzi_k = g.rdz(P, 0);
     real kh_k = kh[c];
     real d1 = real(0.0), d2 = real(0.0), cp = real(0.0);
 #pragma unroll 4
     for (int k = 0; k < nz; ++k) {
         const size_t o = (size_t)k * n2 + c;
         const real kh_k1 = kh[o + n2];
-        real m3_k1 = real(0.0), dz_k1 = real(0.0);
-        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
-        const real dzi_k1 = (k + 1 < nz) ? real(0.5) * (dz_k + dz_k1) : dz_k;
+        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
+        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
         const real r1 = rT[o];
         const real r2 = ts ? rS[o] : real(0.0);
         real sub, diag, sup;
-        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, kh_k, kh_k1, P.thv_dt_zero, sub, diag, sup);
+        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, kh_k, kh_k1, P.thv_dt_zero, sub, diag, sup);
         if (k == 0) {
             cp = sup / diag;
             d1 = r1 / diag;
@@ -1563,9 +1551,7 @@ __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restr
             if (ts) S_out[o] = d2;
         }
         kh_k = kh_k1;
-        dz_k = dz_k1;
-        m3_k = m3_k1;
-        dzi_k = dzi_k1;
+        rdzi_k = rdzi_k1;
     }
     real x1 = d1, x2 = d2;
 #pragma unroll 4
