@@ -62,9 +62,6 @@ using namespace oc;
 
 namespace oc {
 
-// levels one CTA of k_mom_column / k_tracer_rhs marches unless tuned
-constexpr int kDefaultLevelsPerCta = 10;
-
 int fail(oc_handle* h, int code, const std::string& msg) {
     if (h) h->err = msg;
     return code;
@@ -183,8 +180,7 @@ void fill_scalars(oc_handle* h) {
     const double kap = 1.0 / 3.0;
     P.one_m_kappa3 = 1.0 - kap;
     P.one_p_kappa3 = 1.0 + kap;
-    P.mom_kl = c.nz < kDefaultLevelsPerCta ? c.nz : kDefaultLevelsPerCta;
-    P.tr_kl = P.mom_kl;
+    P.mom_kl = P.tr_kl = 0;  // default_levels sets them with the domain, unless oc_set_tiling came first
     // the fp64 copies the kernels read for their fp64 quantities (equal to the
     // fields above on this path; dx64, dy64 and the level table are set with the domain)
     P.rho0_64 = c.rho0;
@@ -776,6 +772,12 @@ static int set_domain_impl(oc_handle* h, const double* Hh, const double* maskh, 
     P.mask_v64 = P.mask_v;
     int rc = OC_OK;
     if (h->mixed && (rc = mixed_alloc(h, kinfo, dzx))) return rc;
+    if (P.mom_kl == 0) {
+        if (h->mixed) default_levels(h->P32, P.mom_kl, P.tr_kl);
+        else default_levels(P, P.mom_kl, P.tr_kl);
+    }
+    h->P32.mom_kl = P.mom_kl;
+    h->P32.tr_kl = P.tr_kl;
     rc = upload_stress(h);
     if (rc) return rc;
     if (f64) {

@@ -1681,6 +1681,37 @@ void launch_wcol(const KPR& P, const real* u, const real* v, real* w, cudaStream
 void launch_phi(const KPR& P, const wide* b, wide* phi, cudaStream_t s) {
     k_phi<<<col_grid(P), col_block(), 0, s>>>(P, b, phi);
 }
+// Levels one CTA marches, for `tiles` tiles and `resident` CTAs on the GPU at once: the
+// count whose rounds cost least, a round being its levels plus one (a CTA's start
+// forms the fluxes at its top again and fills its pipeline). A small grid takes few
+// levels, so that its tiles reach every SM; a large one takes what leaves the last
+// round fullest. us a launch of k_mom_column and k_tracer_rhs with 10 levels on every
+// grid and with these: 48 x 48 x 12 50 and 52, now 11 and 12; 128 x 4 x 32 25 and 33, now 5
+// and 5; 512 x 512 x 50 1049 and 704, now 1043 and 691.
+static int levels_per_cta(long long tiles, int nz, long long resident) {
+    int best = nz;
+    long long cost = -1;
+    for (int slabs = 1; slabs <= nz; ++slabs) {
+        const int kl = (nz + slabs - 1) / slabs;
+        const long long rounds = (tiles * ((nz + kl - 1) / kl) + resident - 1) / resident;
+        if (cost < 0 || rounds * (kl + 1) < cost) {
+            cost = rounds * (kl + 1);
+            best = kl;
+        }
+    }
+    return best;
+}
+void default_levels(const KPR& P, int& mom_kl, int& tr_kl) {
+    int dev = 0, sms = 1, m = 1, t = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_mom_column, MOM_TX * MOM_TY * 2, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, k_tracer_rhs, TRX * TRY, 0);
+    const long long mt = (long long)((P.nx + MOM_TX - 1) / MOM_TX) * ((P.ny + MOM_TY - 1) / MOM_TY);
+    const long long tt = (long long)((P.nx + TRX - 1) / TRX) * ((P.ny + TRY - 1) / TRY);
+    mom_kl = levels_per_cta(mt, P.nz, (long long)sms * (m > 0 ? m : 1));
+    tr_kl = levels_per_cta(tt, P.nz, (long long)sms * (t > 0 ? t : 1));
+}
 static dim3 cell_block() { return dim3(32, 8, 1); }
 static dim3 cell_grid(const KPR& P) { return dim3((P.nx + 31) / 32, (P.ny + 7) / 8, P.nz); }
 void launch_mom_explicit(const KPR& P, const real* u, const real* v, const wide* b,

@@ -15,6 +15,8 @@ namespace oc {
     void launch_qsolve(const KPT<R>& P, const R* km, R* q, cudaStream_t s);                                     \
     void launch_closure(const KPT<R>& P, const R* u, const R* v, const double* b, R* e, R* km, R* kh, R* q,    \
                         cudaStream_t s);                                                                        \
+    /* levels per CTA of the two level-marching kernels for this grid on the current device */                \
+    void default_levels(const KPT<R>& P, int& mom_kl, int& tr_kl);                                             \
     void launch_kukv(const KPT<R>& P, const R* q, double* Ku, double* Kv, cudaStream_t s);                      \
     void launch_wcol(const KPT<R>& P, const R* u, const R* v, R* w, cudaStream_t s);                            \
     void launch_phi(const KPT<R>& P, const double* b, double* phi, cudaStream_t s);                             \

@@ -169,8 +169,8 @@ int oc_set_domain_slab(oc_handle* h, const double* H, const double* mask, const 
  * oc_unpack_rows writes such a buffer into those rows and recomputes w for the
  * velocities now in the state. Asynchronous on `stream`. */
 /* Levels one CTA marches in the explicit-momentum and tracer right-hand-side
- * kernels (1..nz; 10 or nz by default). Every value gives the same results bit
- * for bit; only the speed depends on it. oc_set_tiling sets both; oc_autotune
+ * kernels (1..nz; by default what leaves the GPU least idle for this grid).
+ * Every value gives the same results bit for bit; only the speed depends on it. oc_set_tiling sets both; oc_autotune
  * times each kernel on the current state over a candidate list, keeps the
  * fastest and returns the choice (synchronous; on a mixed-precision handle it
  * times the FP32 kernels). No reference counterpart: the tile shapes of the
