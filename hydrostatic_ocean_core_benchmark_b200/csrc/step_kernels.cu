@@ -353,6 +353,69 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
     column_q(P, g, [&](int k) { return km[(size_t)k * n2 + c]; }, cst, q, c, n2);
 }
 
+// ------------------------------------------------------------------ sums over levels
+// Kernels whose levels are independent but for a running sum: a CTA takes LV_X columns
+// of a row with LV_Y threads each. The threads of a column form its levels' terms
+// side by side, LV_B loads deep, into shared memory; then one warp per sum adds them
+// in the order of the levels. With a thread per column (32 x 4 a CTA) a level waits for
+// the one before it, and a 128 x 128 grid puts one warp on each scheduler.
+constexpr int LV_X = 32, LV_Y = 8, LV_B = 4, LV_K = LV_Y * LV_B;
+
+// Columns up to which a thread per column leaves the SMs short of warps. Above, the
+// column's geometry, which every thread of it works out again, costs more than the
+// waiting. us a launch by columns and by levels: w at 16,384 x 50 64 and 23, at 46,937 x 37
+// 48 and 41, at 122,880 x 30 54 and 86, at 262,144 x 50 198 and 330; the back substitution at
+// 16,384 x 50 29 and 8, at 46,937 x 37 27 and 14, at 262,144 x 50 82 and 88; Ku and Kv (three
+// columns' geometry for little arithmetic: half the limit) at 16,384 x 50 35 and 13, at
+// 46,937 x 37 22 and 26. One grid alone still gains at 65,536 (back substitution 26 and 16),
+// but eight members of an ensemble, which fill the GPU together, lost 5% there.
+constexpr int kFewColumns = 49152;
+
+#define LEVELS_PROLOGUE                                          \
+    const int lv_tiles = (P.nx + LV_X - 1) / LV_X;               \
+    const int j = blockIdx.x / lv_tiles;                         \
+    const int lv_i = (blockIdx.x - j * lv_tiles) * LV_X + threadIdx.x; \
+    const bool live = lv_i < P.nx; /* the others repeat the last column and store nothing */ \
+    const int i = live ? lv_i : P.nx - 1;                        \
+    Nbr nb;                                                      \
+    nb.init(i, j, P.nx, P.ny);                                   \
+    const size_t n2 = (size_t)P.n2;                              \
+    (void)n2;                                                    \
+    (void)live;
+
+template <class T>
+static dim3 level_grid(const KPT<T>& P) { return dim3((unsigned)(((P.nx + LV_X - 1) / LV_X) * P.ny)); }
+static dim3 level_block() { return dim3(LV_X, LV_Y); }
+
+// NS running sums over the levels 0 .. nz - 1 (UP: nz - 1 .. 0): term(k, t) forms level k's
+// terms t[NS]; after each chunk of LV_K levels warp n < NS adds its sum's, calling
+// step(n, k, sum) after each level. sum starts with the first level's term.
+template <int NS, bool UP, class T, class F, class G>
+__device__ __forceinline__ void level_sums(int nz, T (*terms)[LV_K][LV_X], F term, G step) {
+    T sum = T(0.0);
+    for (int c0 = 0; c0 < nz; c0 += LV_K) {
+        const int n = nz - c0 < LV_K ? nz - c0 : LV_K;
+#pragma unroll
+        for (int q = 0; q < LV_B; ++q) {
+            const int r = threadIdx.y + q * LV_Y, rc = r < n ? r : n - 1;
+            T t[NS];
+            term(UP ? nz - 1 - (c0 + rc) : c0 + rc, t);
+#pragma unroll
+            for (int m = 0; m < NS; ++m) terms[m][r][threadIdx.x] = t[m];
+        }
+        __syncthreads();
+        if (threadIdx.y < NS) {
+#pragma unroll 4
+            for (int r = 0; r < n; ++r) {
+                const T t = terms[threadIdx.y][r][threadIdx.x];
+                sum = (c0 + r == 0) ? t : sum + t;
+                step(threadIdx.y, UP ? nz - 1 - (c0 + r) : c0 + r, sum);
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------------------ Ku, Kv
 // Ku = sum_k dz3u * min(q, q_east) * mask_u (model3d_v05.py:154-157)
 __global__ void k_kukv(KPR P, const real* __restrict__ q, wide* __restrict__ Ku,
@@ -376,6 +439,29 @@ __global__ void k_kukv(KPR P, const real* __restrict__ q, wide* __restrict__ Ku,
     }
     Ku[c] = su * P.mask_u64[c];
     Kv[c] = sv * P.mask_v64[c];
+}
+
+// the same by levels, for few columns
+__global__ void __launch_bounds__(LV_X * LV_Y, 4) k_kukv_few(KPR P, const real* __restrict__ q, wide* __restrict__ Ku,
+                                                      wide* __restrict__ Kv) {
+    __shared__ wide terms[2][LV_K][LV_X];
+    LEVELS_PROLOGUE
+    const size_t c = nb.c;
+    const size_t ce = nb.at(0, 1), cn = nb.at(1, 0);
+    const ColGeoR gc = ColGeoR::load(P, (int)c), ge = ColGeoR::load(P, (int)ce), gn = ColGeoR::load(P, (int)cn);
+    const int2 kf = P.kface[c];
+    const int nz = P.nz;
+    // depth sums in fp64 on both paths
+    level_sums<2, false>(nz, terms, [&](int k, wide* t) {
+        const size_t o = (size_t)k * n2;
+        real m;
+        const real dzc = gc.dz(P, k, m), dze = ge.dz(P, k, m), dzn = gn.dz(P, k, m);
+        const real qc = q[o + c];
+        t[0] = wide(face_dz(P, kf.x, k, dzc, dze) * fmin(qc, q[o + ce]));
+        t[1] = wide(face_dz(P, kf.y, k, dzc, dzn) * fmin(qc, q[o + cn]));
+    }, [&](int n, int k, wide sum) {
+        if (k == nz - 1 && live) (n ? Kv : Ku)[c] = sum * (n ? P.mask_v64 : P.mask_u64)[c];
+    });
 }
 
 // ------------------------------------------------------------------ w from transport divergence
@@ -406,6 +492,32 @@ __global__ void __launch_bounds__(128, 8) k_wcol(KPR P, const real* __restrict__
         acc = (k == nz - 1) ? td : acc + td;
         w[o + c] = -acc;
     }
+}
+
+// the same by levels, for few columns
+__global__ void __launch_bounds__(LV_X * LV_Y, 4) k_wcol_few(KPR P, const real* __restrict__ u, const real* __restrict__ v,
+                                                      real* __restrict__ w) {
+    __shared__ real terms[1][LV_K][LV_X];
+    LEVELS_PROLOGUE
+    const int nz = P.nz;
+    const size_t c = nb.c, cw = nb.at(0, -1), cs_ = nb.at(-1, 0);
+    const ColGeoR gc = ColGeoR::load(P, (int)c), ge = ColGeoR::load(P, nb.at(0, 1)),
+                 gw = ColGeoR::load(P, (int)cw), gn = ColGeoR::load(P, nb.at(1, 0)), gs = ColGeoR::load(P, (int)cs_);
+    const int2 kf = P.kface[c];
+    const int kuw = P.kface[cw].x, kvs = P.kface[cs_].y;
+    if (threadIdx.y == 0 && live) w[(size_t)nz * n2 + c] = real(0.0);
+    level_sums<1, true>(nz, terms, [&](int k, real* t) {
+        const size_t o = (size_t)k * n2;
+        real m3, m;
+        const real dzc = gc.dz(P, k, m3);
+        const real dzu_c = face_dz(P, kf.x, k, dzc, ge.dz(P, k, m));
+        const real dzu_w = face_dz(P, kuw, k, gw.dz(P, k, m), dzc);
+        const real dzv_c = face_dz(P, kf.y, k, dzc, gn.dz(P, k, m));
+        const real dzv_s = face_dz(P, kvs, k, gs.dz(P, k, m), dzc);
+        t[0] = m3 * ((dzu_c * u[o + c] - dzu_w * u[o + cw]) / P.dx + (dzv_c * v[o + c] - dzv_s * v[o + cs_]) / P.dy);
+    }, [&](int, int k, real sum) {
+        if (live) w[(size_t)k * n2 + c] = -sum;
+    });
 }
 
 // ------------------------------------------------------------------ buoyancy potential
@@ -1114,6 +1226,68 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
     Vg[c] = sv;
 }
 
+// The same for one component per thread (threadIdx.z), for few columns: a level's chain has
+// two divisions instead of three, and there are twice the warps. Each thread keeps the
+// elimination coefficients, so on a large grid it is the slower form. us a launch by
+// columns and by components: 16,384 x 50 60 and 51, 512 x 32 33 and 23, 46,937 x 37 39 and 31,
+// 65,536 x 32 52 and 48, 122,880 x 30 67 and 84.
+template <int NZM>
+__global__ void __launch_bounds__(128) k_momentum_solve_few(KPR P, const real* __restrict__ km,
+                                                            real* __restrict__ ghu, real* __restrict__ ghv,
+                                                            wide* __restrict__ Ug, wide* __restrict__ Vg) {
+    COLUMN_PROLOGUE
+    const int nz = P.nz;
+    const int c = nb.c;
+    const bool comp = threadIdx.z;
+    const ColGeoR g = ColGeoR::load(P, c);
+    real* __restrict__ gh = comp ? ghv : ghu;
+    real cs[NZM];
+    real rdzi_k = g.rdz(P, 0);
+    real km_k = km[c];
+    real x = real(0.0), cp = real(0.0);
+#pragma unroll 4
+    for (int k = 0; k < nz; ++k) {
+        const size_t o = (size_t)k * n2 + c;
+        const real km_k1 = km[o + n2];
+        const real r = gh[o];
+        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
+        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
+        real sub, diag, sup;
+        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
+        if (k == 0) {
+            cp = sup / diag;
+            x = r / diag;
+        } else {
+            const real den = diag - sub * cp;
+            cp = sup / den;
+            x = (r - sub * x) / den;
+        }
+        cs[k] = cp;
+        gh[o] = x;
+        km_k = km_k1;
+        rdzi_k = rdzi_k1;
+    }
+    gh[(size_t)(nz - 1) * n2 + c] = x * ((nz - 1 < g.kb) ? real(1.0) : real(0.0));
+#pragma unroll 4
+    for (int k = nz - 2; k >= 0; --k) {
+        const size_t o = (size_t)k * n2 + c;
+        x = gh[o] - cs[k] * x;
+        gh[o] = x * ((k < g.kb) ? real(1.0) : real(0.0));
+    }
+    const ColGeoR gf = ColGeoR::load(P, comp ? nb.at(1, 0) : nb.at(0, 1));
+    const int kf = comp ? P.kface[c].y : P.kface[c].x;
+    wide sum = 0.0;  // depth sum in fp64 on both paths
+#pragma unroll 4
+    for (int k = 0; k < nz; ++k) {
+        real m3c, m3f;
+        const real dzc = g.dz(P, k, m3c);
+        const real dzf = gf.dz(P, k, m3f);
+        const real t = (k < kf ? real(1.0) : real(0.0)) * face_combine(P, dzc, dzf) * gh[(size_t)k * n2 + c];
+        sum = (k == 0) ? wide(t) : sum + wide(t);
+    }
+    (comp ? Vg : Ug)[c] = sum;
+}
+
 // ------------------------------------------------------------------ back substitution
 // u = (gh_u - g dt theta q dx(eta_new) m3u) m3   (model3d_v05.py:404-406)
 __global__ void k_backsub(KPR P, const real* __restrict__ ghu, const real* __restrict__ ghv,
@@ -1128,6 +1302,31 @@ __global__ void k_backsub(KPR P, const real* __restrict__ ghu, const real* __res
     const int2 kf = P.kface[c];
 #pragma unroll 4
     for (int k = 0; k < P.nz; ++k) {
+        const size_t o = (size_t)k * n2 + c;
+        const real m3 = k < kb ? real(1.0) : real(0.0);
+        const real m3u_k = k < kf.x ? real(1.0) : real(0.0);
+        const real m3v_k = k < kf.y ? real(1.0) : real(0.0);
+        const real qk = q[o];
+        u_out[o] = (ghu[o] - P.c2 * qk * gx * m3u_k) * m3;
+        v_out[o] = (ghv[o] - P.c2 * qk * gy * m3v_k) * m3;
+    }
+}
+
+// the same by levels, for few columns
+__global__ void __launch_bounds__(LV_X * LV_Y) k_backsub_few(KPR P, const real* __restrict__ ghu,
+                                                         const real* __restrict__ ghv, const real* __restrict__ q,
+                                                         const wide* __restrict__ eta_new, real* __restrict__ u_out,
+                                                         real* __restrict__ v_out) {
+    LEVELS_PROLOGUE
+    if (!live) return;
+    const size_t c = nb.c, ce = nb.at(0, 1), cn = nb.at(1, 0);
+    // the surface gradient in fp64 on both paths (a difference of neighbouring elevations)
+    const real gx = real(P.mask_u64[c] * (eta_new[ce] - eta_new[c]) / P.dx64);
+    const real gy = real(P.mask_v64[c] * (eta_new[cn] - eta_new[c]) / P.dy64);
+    const int kb = P.kinfo[c].y;
+    const int2 kf = P.kface[c];
+#pragma unroll 4
+    for (int k = threadIdx.y; k < P.nz; k += LV_Y) {
         const size_t o = (size_t)k * n2 + c;
         const real m3 = k < kb ? real(1.0) : real(0.0);
         const real m3u_k = k < kf.x ? real(1.0) : real(0.0);
@@ -1608,26 +1807,27 @@ __global__ void k_diag_buoyancy(KPR P, const real* __restrict__ T, const real* _
 }
 
 // ------------------------------------------------------------------ transports
-// depth-integrated transports sum_k dz3u u, sum_k dz3v v (fp64 sums on both paths)
-__global__ void k_transport(KPR P, const real* __restrict__ u, const real* __restrict__ v,
-                            wide* __restrict__ U, wide* __restrict__ V) {
-    COLUMN_PROLOGUE
+// depth-integrated transports sum_k dz3u u, sum_k dz3v v (fp64 sums on both paths), by
+// levels on every grid: us a launch by columns and by levels, 128 x 4 x 32 5.1 and 1.5,
+// 16,384 x 50 13 and 15, 262,144 x 50 113 and 49
+__global__ void __launch_bounds__(LV_X * LV_Y) k_transport(KPR P, const real* __restrict__ u,
+                                                           const real* __restrict__ v, wide* __restrict__ U,
+                                                           wide* __restrict__ V) {
+    __shared__ wide terms[2][LV_K][LV_X];
+    LEVELS_PROLOGUE
     const size_t c = nb.c;
     const ColGeoR gc = ColGeoR::load(P, (int)c), ge = ColGeoR::load(P, nb.at(0, 1)), gn = ColGeoR::load(P, nb.at(1, 0));
     const int2 kf = P.kface[c];
-    wide su = 0.0, sv = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < P.nz; ++k) {
+    const int nz = P.nz;
+    level_sums<2, false>(nz, terms, [&](int k, wide* t) {
         const size_t o = (size_t)k * n2 + c;
         real m;
         const real dzc = gc.dz(P, k, m);
-        const real tu = face_dz(P, kf.x, k, dzc, ge.dz(P, k, m)) * u[o];
-        const real tv = face_dz(P, kf.y, k, dzc, gn.dz(P, k, m)) * v[o];
-        su = (k == 0) ? wide(tu) : su + wide(tu);
-        sv = (k == 0) ? wide(tv) : sv + wide(tv);
-    }
-    U[c] = su;
-    V[c] = sv;
+        t[0] = wide(face_dz(P, kf.x, k, dzc, ge.dz(P, k, m)) * u[o]);
+        t[1] = wide(face_dz(P, kf.y, k, dzc, gn.dz(P, k, m)) * v[o]);
+    }, [&](int n, int k, wide sum) {
+        if (k == nz - 1 && live) (n ? V : U)[c] = sum;
+    });
 }
 
 // ------------------------------------------------------------------ launchers
@@ -1673,10 +1873,16 @@ void launch_closure(const KPR& P, const real* u, const real* v, const wide* b, r
     NZ_DISPATCH(P.nz, (closure_nzm<NZM>(P, u, v, b, e, km, kh, q, s)));
 }
 void launch_kukv(const KPR& P, const real* q, wide* Ku, wide* Kv, cudaStream_t s) {
-    k_kukv<<<col_grid(P), col_block(), 0, s>>>(P, q, Ku, Kv);
+    if (P.n2 <= kFewColumns / 2)
+        k_kukv_few<<<level_grid(P), level_block(), 0, s>>>(P, q, Ku, Kv);
+    else
+        k_kukv<<<col_grid(P), col_block(), 0, s>>>(P, q, Ku, Kv);
 }
 void launch_wcol(const KPR& P, const real* u, const real* v, real* w, cudaStream_t s) {
-    k_wcol<<<col_grid(P), col_block(), 0, s>>>(P, u, v, w);
+    if (P.n2 <= kFewColumns)
+        k_wcol_few<<<level_grid(P), level_block(), 0, s>>>(P, u, v, w);
+    else
+        k_wcol<<<col_grid(P), col_block(), 0, s>>>(P, u, v, w);
 }
 void launch_phi(const KPR& P, const wide* b, wide* phi, cudaStream_t s) {
     k_phi<<<col_grid(P), col_block(), 0, s>>>(P, b, phi);
@@ -1732,11 +1938,19 @@ void launch_predictor_rhs(const KPR& P, const real* u, const real* v, const real
 }
 void launch_momentum_solve(const KPR& P, const real* km, real* ghu, real* ghv, wide* Ug, wide* Vg,
                            cudaStream_t s) {
-    NZ_DISPATCH(P.nz, (k_momentum_solve<NZM><<<col_grid(P), col_block(), 0, s>>>(P, km, ghu, ghv, Ug, Vg)));
+    if (P.n2 <= kFewColumns) {
+        const dim3 grid((P.nx + 31) / 32, (P.ny + 1) / 2);
+        NZ_DISPATCH(P.nz, (k_momentum_solve_few<NZM><<<grid, dim3(32, 2, 2), 0, s>>>(P, km, ghu, ghv, Ug, Vg)));
+    } else {
+        NZ_DISPATCH(P.nz, (k_momentum_solve<NZM><<<col_grid(P), col_block(), 0, s>>>(P, km, ghu, ghv, Ug, Vg)));
+    }
 }
 void launch_backsub(const KPR& P, const real* ghu, const real* ghv, const real* q,
                     const wide* eta_new, real* u_out, real* v_out, cudaStream_t s) {
-    k_backsub<<<col_grid(P), col_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
+    if (P.n2 <= kFewColumns)
+        k_backsub_few<<<level_grid(P), level_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
+    else
+        k_backsub<<<col_grid(P), col_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
 }
 void launch_tracer_rhs(const KPR& P, const real* C0, const real* S, const real* u, const real* v,
                        const real* w, const real* kh, real* rT, real* rS, cudaStream_t s) {
@@ -1753,7 +1967,7 @@ void launch_diag_buoyancy(const KPR& P, const real* T, const real* S, wide* b, c
 }
 void launch_transport(const KPR& P, const real* u, const real* v, wide* U, wide* V,
                       cudaStream_t s) {
-    k_transport<<<col_grid(P), col_block(), 0, s>>>(P, u, v, U, V);
+    k_transport<<<level_grid(P), level_block(), 0, s>>>(P, u, v, U, V);
 }
 
 }  // namespace oc
