@@ -159,6 +159,37 @@ __device__ __forceinline__ double face_thick(const KP& P, int c, int cn, int kf,
     return face_dz(P, kf, k, col_dz(P, c, k, m), col_dz(P, cn, k, m));
 }
 
+// What one cell's thread adds to an array's cells around it, collected in registers and
+// sent once per cell instead of term by term (about fifty reds to L2 per cell in
+// k_mom_adv_T). The terms for cells along x go to their lanes by shuffles (a warp is 32
+// cells of a row); only the warp's ends and the wrap send theirs themselves. At 256 x 256 x
+// 32 the two scatter kernels take 216 and 272 us.
+struct Scatter {
+    double c = 0, e = 0, ee = 0, w = 0, ww = 0, s = 0, ss = 0, n = 0, nn = 0, up = 0, up2 = 0, dn = 0;
+};
+// the lanes of the warp's row that have a cell
+__device__ __forceinline__ unsigned row_mask(int i, int nx) {
+    const int have = nx - (i - (int)(threadIdx.x & 31));
+    return have >= 32 ? 0xffffffffu : (1u << have) - 1u;
+}
+// along x; what stays for the own cell is left in g.c
+__device__ __forceinline__ void scatter_x(double* a, size_t o, const Scatter& g, double& own, int i, int j, int nx,
+                                          unsigned mask) {
+    const int lane = threadIdx.x & 31;
+    const double fe = __shfl_up_sync(mask, g.e, 1), fee = __shfl_up_sync(mask, g.ee, 2);
+    const double fw = __shfl_down_sync(mask, g.w, 1), fww = __shfl_down_sync(mask, g.ww, 2);
+    double* row = a + o + (size_t)j * nx;
+    own = g.c;
+    if (lane >= 1) own += fe;
+    if (lane >= 2) own += fee;
+    if (lane < 31 && i + 1 < nx) own += fw;
+    if (lane < 30 && i + 2 < nx) own += fww;
+    if (lane == 31 || i + 1 >= nx) atomic_add(&row[i + 1 >= nx ? i + 1 - nx : i + 1], g.e);
+    if (lane >= 30 || i + 2 >= nx) atomic_add(&row[i + 2 >= nx ? i + 2 - nx : i + 2], g.ee);
+    if (lane == 0) atomic_add(&row[i == 0 ? nx - 1 : i - 1], g.w);
+    if (lane < 2) atomic_add(&row[i <= 1 ? i - 2 + nx : i - 2], g.ww);
+}
+
 #define ADJ_PROLOGUE                                      \
     const int i = blockIdx.x * blockDim.x + threadIdx.x;  \
     const int j = blockIdx.y * blockDim.y + threadIdx.y;  \
@@ -172,80 +203,129 @@ __device__ __forceinline__ double face_thick(const KP& P, int c, int cn, int kf,
     const int cS = (j == 0 ? ny - 1 : j - 1) * nx + i;    \
     (void)cE, (void)cW, (void)cN, (void)cS, (void)nz, (void)n2;
 
-// ---------------------------------------------------------------- column solves
-// x = M^-T y for the column's implicit rows (vertical_var.py:35-77) with the
-// interface coefficient K (constant in this scope) and the bottom-row term
-// thv_dt_drag = (theta_v dt) drag: the transposed matrix has sub'[k] = sup[k-1]
-// and sup'[k] = sub[k+1]. y and x may alias.
-template <int NZM>
-__device__ void solve_transposed(const KP& P, int c, double K, double thv_dt_drag, const double* y, double* x,
-                                 size_t n2) {
-    const int nz = P.nz;
-    const ColGeo g = ColGeo::load(P, c);
-    double sub[NZM], dia[NZM], sup[NZM];
-    double m3_k, dz_k = g.dz(P, 0, m3_k);
-    double dzi_k = dz_k;
-    for (int k = 0; k < nz; ++k) {
-        double m3_k1 = 0.0, dz_k1 = 0.0;
-        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
-        const double dzi_k1 = (k + 1 < nz) ? 0.5 * (dz_k + dz_k1) : dz_k;
-        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, K, K, thv_dt_drag, sub[k], dia[k], sup[k]);
-        dz_k = dz_k1;
-        m3_k = m3_k1;
-        dzi_k = dzi_k1;
-    }
-    // Thomas on (sub' = sup[k-1], diag, sup' = sub[k+1])
-    double cs[NZM];
-    double cp = 0.0, dp = 0.0;
-    for (int k = 0; k < nz; ++k) {
-        const double a = k > 0 ? sup[k - 1] : 0.0;
-        const double bsup = k + 1 < nz ? sub[k + 1] : 0.0;
-        const double yk = y[(size_t)k * n2 + c];
-        if (k == 0) {
-            cp = bsup / dia[0];
-            dp = yk / dia[0];
-        } else {
-            const double den = dia[k] - a * cp;
-            cp = bsup / den;
-            dp = (yk - a * dp) / den;
-        }
-        cs[k] = cp;
-        x[(size_t)k * n2 + c] = dp;
-    }
-    double xn = dp;
-    for (int k = nz - 2; k >= 0; --k) {
-        const size_t o = (size_t)k * n2 + c;
-        xn = x[o] - cs[k] * xn;
-        x[o] = xn;
+// Kernels that also sum over the column: ADJ_LY threads per column take every ADJ_LY-th
+// level, and their partial sums meet in shared memory. (A thread per column waited for
+// every level's loads in turn, with 14 warps on an SM at 256 x 256.)
+constexpr int ADJ_LY = 8;
+#define ADJ_LEVELS_PROLOGUE                                              \
+    const int lv_tiles = (P.nx + 31) / 32;                               \
+    const int j = blockIdx.x / lv_tiles;                                 \
+    const int lv_i = (blockIdx.x - j * lv_tiles) * 32 + threadIdx.x;     \
+    const bool live = lv_i < P.nx;                                       \
+    const int i = live ? lv_i : P.nx - 1;                                \
+    const int nx = P.nx, ny = P.ny, nz = P.nz;                           \
+    const size_t n2 = (size_t)P.n2;                                      \
+    const int c = j * nx + i;                                            \
+    const int cE = j * nx + (i + 1 == nx ? 0 : i + 1);                   \
+    const int cW = j * nx + (i == 0 ? nx - 1 : i - 1);                   \
+    const int cN = (j + 1 == ny ? 0 : j + 1) * nx + i;                   \
+    const int cS = (j == 0 ? ny - 1 : j - 1) * nx + i;                   \
+    (void)cE, (void)cW, (void)cN, (void)cS;
+
+// the column's sums of its threads' a and b; add(0, sum of a) and add(1, sum of b) by one thread each
+template <class F>
+__device__ __forceinline__ void column_pair_sums(double a, double b, F add) {
+    __shared__ double part[2][ADJ_LY][32];
+    part[0][threadIdx.y][threadIdx.x] = a;
+    part[1][threadIdx.y][threadIdx.x] = b;
+    __syncthreads();
+    if (threadIdx.y < 2) {
+        double t = 0.0;
+#pragma unroll
+        for (int l = 0; l < ADJ_LY; ++l) t += part[threadIdx.y][l][threadIdx.x];
+        add(threadIdx.y, t);
     }
 }
 
-// cotangent of the explicit vertical diffusion Dz[f] (vertical_var.py:80-106) of
-// one face-velocity or tracer column with face thickness dzf[k], constant K,
-// the cell column's bottom rule and drag: f_b += Dz^T r_b; returns the
-// cotangent of the surface flux.
-template <int NZM>
-__device__ double explicit_dz_T(const KP& P, const double* dzf, const double* m3c, double K, double drag,
-                                const double* r_b, double* f_b) {
+// ---------------------------------------------------------------- column solves
+// x = M^-T y of two fields for the column's implicit rows (vertical_var.py:35-77) with the
+// interface coefficient K (constant in this scope) and the bottom-row term
+// thv_dt_drag = (theta_v dt) drag: the transposed matrix has sub'[k] = sup[k-1]
+// and sup'[k] = sub[k+1]. rhs(k, y) forms level k's two right-hand sides. The rows are
+// formed on the way down, once for both fields; only the elimination coefficients are
+// kept (four arrays per thread before, in local memory). Momentum at 256 x 256 x 32: 103
+// us a launch one field after the other, 54 together.
+template <int NZM, class Y>
+__device__ __forceinline__ void solve_transposed(const KP& P, int c, double K, double thv_dt_drag, Y rhs, double* xa,
+                                                 double* xb, size_t n2) {
     const int nz = P.nz;
-    double flux_b[NZM + 1];
-    for (int k = 0; k <= nz; ++k) flux_b[k] = 0.0;
+    const ColGeo g = ColGeo::load(P, c);
+    // the next row to form: its thickness, mask and the spacing above it
+    double m3_n, dz_n = g.dz(P, 0, m3_n), dzi_n = dz_n;
+    auto row = [&](int k, double& sub, double& dia, double& sup) {
+        double m3_1 = 0.0, dz_1 = 0.0;
+        if (k + 1 < nz) dz_1 = g.dz(P, k + 1, m3_1);
+        const double dzi_1 = (k + 1 < nz) ? 0.5 * (dz_n + dz_1) : dz_n;
+        implicit_row(P, k, dz_n, m3_n, m3_1, dzi_n, dzi_1, K, K, thv_dt_drag, sub, dia, sup);
+        dz_n = dz_1;
+        m3_n = m3_1;
+        dzi_n = dzi_1;
+    };
+    // Thomas on (sub' = sup[k-1], diag, sup' = sub[k+1])
+    double cs[NZM];
+    double sub, dia, sup, above = 0.0, cp = 0.0, da = 0.0, db = 0.0;
+    row(0, sub, dia, sup);
     for (int k = 0; k < nz; ++k) {
-        const double rb = m3c[k] > 0.0 ? r_b[k] : 0.0;
-        const double idz = inv_pos(dzf[k]);
-        const bool bottom = m3c[k] > 0.0 && (k + 1 >= nz || m3c[k + 1] == 0.0);
-        flux_b[k] += rb * idz;
-        flux_b[k + 1] -= rb * idz;
-        if (bottom) f_b[k] -= drag * idz * rb;
+        double sub1 = 0.0, dia1 = 0.0, sup1 = 0.0, y[2];
+        if (k + 1 < nz) row(k + 1, sub1, dia1, sup1);
+        rhs(k, y);
+        if (k == 0) {
+            cp = sub1 / dia;
+            da = y[0] / dia;
+            db = y[1] / dia;
+        } else {
+            const double den = dia - above * cp;
+            cp = sub1 / den;
+            da = (y[0] - above * da) / den;
+            db = (y[1] - above * db) / den;
+        }
+        cs[k] = cp;
+        xa[(size_t)k * n2 + c] = da;
+        xb[(size_t)k * n2 + c] = db;
+        above = sup;
+        dia = dia1;
+        sup = sup1;
     }
-    for (int k = 1; k < nz; ++k) {
-        const bool bottom_above = m3c[k - 1] > 0.0 && m3c[k] == 0.0;
-        if (bottom_above) continue;
-        const double coef = K * inv_pos(0.5 * (dzf[k - 1] + dzf[k]));
-        f_b[k - 1] += coef * flux_b[k];
-        f_b[k] -= coef * flux_b[k];
+#pragma unroll 4
+    for (int k = nz - 2; k >= 0; --k) {
+        const size_t o = (size_t)k * n2 + c;
+        da = xa[o] - cs[k] * da;
+        db = xb[o] - cs[k] * db;
+        xa[o] = da;
+        xb[o] = db;
     }
-    return flux_b[0];
+}
+
+// cotangent of the explicit vertical diffusion Dz[f] (vertical_var.py:80-106) at level
+// k of one face-velocity or tracer column, added to fb: its own level's r and those of
+// the levels beside it, through the fluxes of the two interfaces. thick(k), wet(k) and
+// r(k) give a level's face thickness, mask and cotangent; constant K, the cell column's
+// bottom rule and drag. surf gets the cotangent of the flux through the level's top.
+template <class D, class M, class R>
+__device__ __forceinline__ double explicit_dz_T(int k, int nz, D thick, M wet, R r, double K, double drag, double fb,
+                                                double& surf) {
+    const double d0 = thick(k), m0 = wet(k);
+    const double i0 = inv_pos(d0), r0 = m0 > 0.0 ? r(k) : 0.0;
+    const double mb = k + 1 < nz ? wet(k + 1) : 0.0;
+    double top = 0.0;
+    if (m0 > 0.0 && mb == 0.0) fb -= drag * i0 * r0;
+    if (k >= 1) {
+        const double da = thick(k - 1), ma = wet(k - 1);
+        top -= (ma > 0.0 ? r(k - 1) : 0.0) * inv_pos(da);
+        top += r0 * i0;
+        if (!(ma > 0.0 && m0 == 0.0)) fb -= K * inv_pos(0.5 * (da + d0)) * top;
+    } else {
+        top += r0 * i0;
+    }
+    if (k + 1 < nz && !(m0 > 0.0 && mb == 0.0)) {
+        const double db = thick(k + 1);
+        double bot = 0.0;
+        bot -= r0 * i0;
+        bot += (mb > 0.0 ? r(k + 1) : 0.0) * inv_pos(db);
+        fb += K * inv_pos(0.5 * (d0 + db)) * bot;
+    }
+    surf = top;
+    return fb;
 }
 
 // ---------------------------------------------------------------- kernels
@@ -265,13 +345,12 @@ __global__ void k_wcol_T1(KP P, const double* __restrict__ w_b, double* __restri
 __global__ void k_wcol_T2(KP P, const double* __restrict__ td_b, double* __restrict__ u_b, double* __restrict__ v_b) {
     ADJ_PROLOGUE
     const int2 kf = P.kface[c];
-    for (int k = 0; k < nz; ++k) {
-        const size_t o = (size_t)k * n2;
-        const double mc = col_m3(P, c, k), me = col_m3(P, cE, k), mn = col_m3(P, cN, k);
-        const double du = face_thick(P, c, cE, kf.x, k), dv = face_thick(P, c, cN, kf.y, k);
-        u_b[o + c] += du / P.dx64 * (mc * td_b[o + c] - me * td_b[o + cE]);
-        v_b[o + c] += dv / P.dy64 * (mc * td_b[o + c] - mn * td_b[o + cN]);
-    }
+    const int k = blockIdx.z;
+    const size_t o = (size_t)k * n2;
+    const double mc = col_m3(P, c, k), me = col_m3(P, cE, k), mn = col_m3(P, cN, k);
+    const double du = face_thick(P, c, cE, kf.x, k), dv = face_thick(P, c, cN, kf.y, k);
+    u_b[o + c] += du / P.dx64 * (mc * td_b[o + c] - me * td_b[o + cE]);
+    v_b[o + c] += dv / P.dy64 * (mc * td_b[o + c] - mn * td_b[o + cN]);
 }
 
 // EOS and implicit tracer solves: r_b = M_b^-T ((X'_b + b'_b m3 db/dX) m3) for X = T, S
@@ -282,38 +361,41 @@ __global__ void k_tracer_solve_T(KP P, const double* __restrict__ Tn, const doub
                                  double* __restrict__ rS_b) {
     ADJ_PROLOGUE
     const ColGeo g = ColGeo::load(P, c);
-    for (int k = 0; k < nz; ++k) {
+    auto rhs = [&](int k, double* y) {
         const size_t o = (size_t)k * n2 + c;
         double m3;
         const double dz = g.dz(P, k, m3);
         double dT = 0.0, dS = 0.0;
         if (m3 > 0.0) eos_partials(P, Tn[o], Sn[o], g.above(P, k) + 0.5 * dz, dT, dS);
         const double bb = bn_b[o] * m3;
-        rT_b[o] = (Tn_b[o] + bb * dT) * m3;
-        rS_b[o] = (Sn_b[o] + bb * dS) * m3;
-    }
-    solve_transposed<NZM>(P, c, P.kappa, P.thv_dt_zero, rT_b, rT_b, n2);
-    solve_transposed<NZM>(P, c, P.kappa, P.thv_dt_zero, rS_b, rS_b, n2);
+        y[0] = (Tn_b[o] + bb * dT) * m3;
+        y[1] = (Sn_b[o] + bb * dS) * m3;
+    };
+    solve_transposed<NZM>(P, c, P.kappa, P.thv_dt_zero, rhs, rT_b, rS_b, n2);
 }
 
 // tracer right-hand side rhs = c + dt tend + c3 Dz[c] + surface terms: the
 // identity and explicit vertical diffusion parts (per column; X_b written)
-template <int NZM>
 __global__ void k_tracer_rhs_T_col(KP P, const double* __restrict__ rT_b, const double* __restrict__ rS_b,
                                    double* __restrict__ T_b, double* __restrict__ S_b) {
     ADJ_PROLOGUE
-    double dz[NZM], m3[NZM], rb[NZM], fb[NZM];
-    for (int k = 0; k < nz; ++k) dz[k] = col_dz(P, c, k, m3[k]);
-    for (int f = 0; f < 2; ++f) {
-        const double* r = f == 0 ? rT_b : rS_b;
-        double* out = f == 0 ? T_b : S_b;
-        for (int k = 0; k < nz; ++k) {
-            rb[k] = P.c3 * r[(size_t)k * n2 + c];
-            fb[k] = r[(size_t)k * n2 + c];
-        }
-        explicit_dz_T<NZM>(P, dz, m3, P.kappa, 0.0, rb, fb);
-        for (int k = 0; k < nz; ++k) out[(size_t)k * n2 + c] = fb[k];
-    }
+    const int k = blockIdx.z;
+    const size_t o = (size_t)k * n2 + c;
+    const ColGeo g = ColGeo::load(P, c);
+    auto thick = [&](int kk) {
+        double m;
+        return g.dz(P, kk, m);
+    };
+    auto wet = [&](int kk) {
+        double m;
+        g.dz(P, kk, m);
+        return m;
+    };
+    double surf;
+    T_b[o] = explicit_dz_T(k, nz, thick, wet, [&](int kk) { return P.c3 * rT_b[(size_t)kk * n2 + c]; }, P.kappa, 0.0,
+                           rT_b[o], surf);
+    S_b[o] = explicit_dz_T(k, nz, thick, wet, [&](int kk) { return P.c3 * rS_b[(size_t)kk * n2 + c]; }, P.kappa, 0.0,
+                           rS_b[o], surf);
 }
 
 // tracer advection and horizontal diffusion (model3d_v05.py:466-512): tend =
@@ -332,10 +414,13 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
     const int cEE = j * nx + (i + 2 >= nx ? i + 2 - nx : i + 2);
     const int cNN = ((j + 2 >= ny) ? j + 2 - ny : j + 2) * nx + i;
     const int scheme = P.advection;
+    const unsigned mask = row_mask(i, nx);
+    double gu = 0.0, gv = 0.0, gw = 0.0;  // of the faces' own velocities, both fields
     for (int f = 0; f < 2; ++f) {
         const double* C = f == 0 ? T : S;
         const double* R = f == 0 ? rT_b : rS_b;
         double* Cb = f == 0 ? T_b : S_b;
+        Scatter gc;
         // a = d rhs / d adv term per cell: adv enters as -dt adv, adv = (hdiv + vdiv) m3
         auto acoef = [&](int cc) {
             double m;
@@ -352,12 +437,12 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
                 if (dzf != 0.0 && fx_b != 0.0) {
                     const Face fc = face_lin(P, scheme, C[o + cW], C[o + c], C[o + cE], C[o + cEE], vel,
                                              col_m3(P, cW, k) > 0.0, col_m3(P, cEE, k) > 0.0);
-                    atomic_add(&u_b[o + c], fx_b * dzf * fc.f);
+                    gu += fx_b * dzf * fc.f;
                     const double s = fx_b * dzf * vel;
-                    atomic_add(&Cb[o + cW], s * fc.dm);
-                    atomic_add(&Cb[o + c], s * fc.d0);
-                    atomic_add(&Cb[o + cE], s * fc.d1);
-                    atomic_add(&Cb[o + cEE], s * fc.dp);
+                    gc.w += s * fc.dm;
+                    gc.c += s * fc.d0;
+                    gc.e += s * fc.d1;
+                    gc.ee += s * fc.dp;
                 }
             }
             // north face
@@ -368,12 +453,12 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
                 if (dzf != 0.0 && fy_b != 0.0) {
                     const Face fc = face_lin(P, scheme, C[o + cS], C[o + c], C[o + cN], C[o + cNN], vel,
                                              col_m3(P, cS, k) > 0.0, col_m3(P, cNN, k) > 0.0);
-                    atomic_add(&v_b[o + c], fy_b * dzf * fc.f);
+                    gv += fy_b * dzf * fc.f;
                     const double s = fy_b * dzf * vel;
-                    atomic_add(&Cb[o + cS], s * fc.dm);
-                    atomic_add(&Cb[o + c], s * fc.d0);
-                    atomic_add(&Cb[o + cN], s * fc.d1);
-                    atomic_add(&Cb[o + cNN], s * fc.dp);
+                    gc.s += s * fc.dm;
+                    gc.c += s * fc.d0;
+                    gc.n += s * fc.d1;
+                    gc.nn += s * fc.dp;
                 }
             }
             // the top face of cell c (interface k): vdiv[k] = (w[k] cf[k] - w[k+1] cf[k+1]) inv
@@ -387,8 +472,8 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
                 const double wv = w[o + c];
                 if (wcf_b != 0.0) {
                     if (k == 0) {
-                        atomic_add(&w_b[o + c], wcf_b * C[o + c]);
-                        atomic_add(&Cb[o + c], wcf_b * wv);
+                        gw += wcf_b * C[o + c];
+                        gc.c += wcf_b * wv;
                     } else {
                         const bool has_up = k >= 2 && col_m3(P, c, k - 2) > 0.0;
                         const bool has_dn = k + 1 <= nz - 1 && col_m3(P, c, k + 1) > 0.0;
@@ -396,12 +481,12 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
                         const double far_dn = k + 1 <= nz - 1 ? C[o + n2 + c] : 0.0;
                         const int sz = scheme == 2 ? 1 : scheme;  // upwind faces are centred vertically
                         const Face fc = face_lin(P, sz, far_dn, C[o + c], C[o - n2 + c], far_up, wv, has_dn, has_up);
-                        atomic_add(&w_b[o + c], wcf_b * fc.f);
+                        gw += wcf_b * fc.f;
                         const double s = wcf_b * wv;
-                        if (k + 1 <= nz - 1) atomic_add(&Cb[o + n2 + c], s * fc.dm);
-                        atomic_add(&Cb[o + c], s * fc.d0);
-                        atomic_add(&Cb[o - n2 + c], s * fc.d1);
-                        if (k >= 2) atomic_add(&Cb[o - 2 * n2 + c], s * fc.dp);
+                        if (k + 1 <= nz - 1) gc.dn += s * fc.dm;
+                        gc.c += s * fc.d0;
+                        gc.up += s * fc.d1;
+                        if (k >= 2) gc.up2 += s * fc.dp;
                     }
                 }
             }
@@ -412,23 +497,36 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
             const double l_c = lcoef(c), l_e = lcoef(cE), l_n = lcoef(cN);
             const double gx_b = (l_c - l_e) / P.dx64 * col_m3u(P, c, k) / P.dx64;
             const double gy_b = (l_c - l_n) / P.dy64 * col_m3v(P, c, k) / P.dy64;
-            atomic_add(&Cb[o + cE], gx_b);
-            atomic_add(&Cb[o + c], -gx_b - gy_b);
-            atomic_add(&Cb[o + cN], gy_b);
+            gc.e += gx_b;
+            gc.c += -gx_b - gy_b;
+            gc.n += gy_b;
         }
+        double gc_own;
+        scatter_x(Cb, o, gc, gc_own, i, j, nx, mask);
+        atomic_add(&Cb[o + c], gc_own);
+        atomic_add(&Cb[o + cS], gc.s);
+        atomic_add(&Cb[o + cN], gc.n);
+        atomic_add(&Cb[o + cNN], gc.nn);
+        if (k + 1 < nz) atomic_add(&Cb[o + n2 + c], gc.dn);
+        if (k >= 1) atomic_add(&Cb[o - n2 + c], gc.up);
+        if (k >= 2) atomic_add(&Cb[o - 2 * n2 + c], gc.up2);
     }
+    atomic_add(&u_b[o + c], gu);
+    atomic_add(&v_b[o + c], gv);
+    atomic_add(&w_b[o + c], gw);
 }
 
 // back-substitution u = (gh_u - c2 q gx(eta_new) m3u) m3 (model3d_v05.py:404-406):
 // gh_b = u_b m3 and the per-column cotangent of the surface gradient
-__global__ void k_backsub_T(KP P, const double* __restrict__ uo_b, const double* __restrict__ vo_b,
+__global__ void __launch_bounds__(32 * ADJ_LY) k_backsub_T(KP P, const double* __restrict__ uo_b, const double* __restrict__ vo_b,
                             const double* __restrict__ q, double* __restrict__ ghu_b, double* __restrict__ ghv_b,
                             double* __restrict__ gx_b, double* __restrict__ gy_b) {
-    ADJ_PROLOGUE
+    ADJ_LEVELS_PROLOGUE
     const int kb = P.kinfo[c].y;
     const int2 kf = P.kface[c];
     double sx = 0.0, sy = 0.0;
-    for (int k = 0; k < nz; ++k) {
+#pragma unroll 2
+    for (int k = threadIdx.y; k < nz && live; k += ADJ_LY) {
         const size_t o = (size_t)k * n2 + c;
         const double m3 = k < kb ? 1.0 : 0.0;
         const double ub = uo_b[o] * m3, vb = vo_b[o] * m3;
@@ -437,8 +535,9 @@ __global__ void k_backsub_T(KP P, const double* __restrict__ uo_b, const double*
         sx += q[o] * (k < kf.x ? 1.0 : 0.0) * ub;
         sy += q[o] * (k < kf.y ? 1.0 : 0.0) * vb;
     }
-    gx_b[c] = -P.c2 * sx;
-    gy_b[c] = -P.c2 * sy;
+    column_pair_sums(sx, sy, [&](int m, double t) {
+        if (live) (m ? gy_b : gx_b)[c] = -P.c2 * t;
+    });
 }
 
 // eta_b += the transpose of the masked surface gradient (mask_u (E eta - eta) / dx, ...)
@@ -492,14 +591,17 @@ __global__ void k_momentum_solve_T(KP P, double* __restrict__ ghu_b, double* __r
     ADJ_PROLOGUE
     const int2 kf = P.kface[c];
     const int kb = P.kinfo[c].y;
-    for (int k = 0; k < nz; ++k) {
+    const ColGeo gc = ColGeo::load(P, c), ge = ColGeo::load(P, cE), gn = ColGeo::load(P, cN);
+    const double Ug = Ug_b[c], Vg = Vg_b[c];
+    auto rhs = [&](int k, double* y) {
         const size_t o = (size_t)k * n2 + c;
         const double m3 = k < kb ? 1.0 : 0.0;
-        ru_b[o] = (ghu_b[o] + face_thick(P, c, cE, kf.x, k) * Ug_b[c]) * m3;
-        rv_b[o] = (ghv_b[o] + face_thick(P, c, cN, kf.y, k) * Vg_b[c]) * m3;
-    }
-    solve_transposed<NZM>(P, c, P.nu, P.thv_dt_drag, ru_b, ru_b, n2);
-    solve_transposed<NZM>(P, c, P.nu, P.thv_dt_drag, rv_b, rv_b, n2);
+        double m;
+        const double dzc = gc.dz(P, k, m);
+        y[0] = (ghu_b[o] + face_dz(P, kf.x, k, dzc, ge.dz(P, k, m)) * Ug) * m3;
+        y[1] = (ghv_b[o] + face_dz(P, kf.y, k, dzc, gn.dz(P, k, m)) * Vg) * m3;
+    };
+    solve_transposed<NZM>(P, c, P.nu, P.thv_dt_drag, rhs, ru_b, rv_b, n2);
 }
 
 // Coriolis averages (operators_masked.py:45-61): av[c] = sum_q w_q f_q / sum_q w_q * m,
@@ -531,89 +633,85 @@ __device__ __forceinline__ void u_on_v_T(const KP& P, size_t o, int k, int c, in
 }
 
 // predictor gu = u + dt (f0 v_cor + pgx) - c1 gx m3u + c3 dzu, rhs = gu + st_u,
-// v_cor = (1 - tc) av(v) + tc av(v_it): cotangents of its inputs. The old
-// average's cotangent is accumulated in avpv_b; the iterate's is scattered to
-// it_b (u_b for the first pass, whose iterate is the old state).
-__global__ void k_predictor_T(KP P, const double* __restrict__ ru_b, const double* __restrict__ rv_b,
-                              double* __restrict__ u_b, double* __restrict__ v_b, double* __restrict__ uit_b,
-                              double* __restrict__ vit_b, double* __restrict__ avpv_b, double* __restrict__ avpu_b,
-                              double* __restrict__ pgx_b, double* __restrict__ pgy_b, double* __restrict__ dzu_b,
-                              double* __restrict__ dzv_b, double* __restrict__ stu_b, double* __restrict__ stv_b,
-                              double* __restrict__ gx2_b, double* __restrict__ gy2_b) {
-    ADJ_PROLOGUE
+// v_cor = (1 - tc) av(v) + tc av(v_it): cotangents of its inputs. Those that enter every
+// pass alike (u, st_u, pgx, dzu, the old average) are multiples of the right-hand
+// sides' cotangents summed over the passes, so only that sum is kept (stu_b, stv_b) and
+// each of their kernels scales it: ten arrays read and written per pass before, two
+// now (256 x 256 x 32: 188 us a pass by a thread per column, 134 by levels, 43 so). The iterate's average is scattered to it_b (u_b for the first pass, whose
+// iterate is the old state).
+__global__ void __launch_bounds__(32 * ADJ_LY) k_predictor_T(
+    KP P, const double* __restrict__ ru_b, const double* __restrict__ rv_b, double* __restrict__ uit_b,
+    double* __restrict__ vit_b, double* __restrict__ stu_b, double* __restrict__ stv_b, double* __restrict__ gx2_b,
+    double* __restrict__ gy2_b) {
+    ADJ_LEVELS_PROLOGUE
     const int cSE = (j == 0 ? ny - 1 : j - 1) * nx + (i + 1 == nx ? 0 : i + 1);
     const int cNW = (j + 1 == ny ? 0 : j + 1) * nx + (i == 0 ? nx - 1 : i - 1);
     const int2 kf = P.kface[c];
     double sx = 0.0, sy = 0.0;
-    for (int k = 0; k < nz; ++k) {
+#pragma unroll 2
+    for (int k = threadIdx.y; k < nz && live; k += ADJ_LY) {
         const size_t o = (size_t)k * n2;
         const double rb = ru_b[o + c], rvb = rv_b[o + c];
-        u_b[o + c] += rb;
-        v_b[o + c] += rvb;
         stu_b[o + c] += rb;
         stv_b[o + c] += rvb;
-        pgx_b[o + c] += P.dt * rb;
-        pgy_b[o + c] += P.dt * rvb;
-        dzu_b[o + c] += P.c3 * rb;
-        dzv_b[o + c] += P.c3 * rvb;
         sx += (k < kf.x ? 1.0 : 0.0) * rb;
         sy += (k < kf.y ? 1.0 : 0.0) * rvb;
         const double vcor_b = P.dt * P.f0 * rb;
         const double ucor_b = P.dt * P.neg_f0 * rvb;
-        avpv_b[o + c] += P.one_m_tc * vcor_b;
-        avpu_b[o + c] += P.one_m_tc * ucor_b;
         v_on_u_T(P, o, k, c, cS, cE, cSE, k < kf.x ? 1.0 : 0.0, P.theta_cor * vcor_b, vit_b);
         u_on_v_T(P, o, k, c, cW, cN, cNW, k < kf.y ? 1.0 : 0.0, P.theta_cor * ucor_b, uit_b);
     }
-    gx2_b[c] += -P.c1 * sx;
-    gy2_b[c] += -P.c1 * sy;
+    column_pair_sums(sx, sy, [&](int m, double t) {
+        if (live) (m ? gy2_b : gx2_b)[c] += -P.c1 * t;
+    });
 }
 
-// the old-state Coriolis averages (avpv = av(v), avpu = av(u)): scatter
-__global__ void k_coriolis_old_T(KP P, const double* __restrict__ avpv_b, const double* __restrict__ avpu_b,
+// the old-state Coriolis averages (avpv = av(v), avpu = av(u)): scatter of (1 - tc) dt f0 times
+// the summed cotangents
+__global__ void k_coriolis_old_T(KP P, const double* __restrict__ stu_b, const double* __restrict__ stv_b,
                                  double* __restrict__ u_b, double* __restrict__ v_b) {
     ADJ_PROLOGUE
     const int cSE = (j == 0 ? ny - 1 : j - 1) * nx + (i + 1 == nx ? 0 : i + 1);
     const int cNW = (j + 1 == ny ? 0 : j + 1) * nx + (i == 0 ? nx - 1 : i - 1);
     const int2 kf = P.kface[c];
-    for (int k = 0; k < nz; ++k) {
-        const size_t o = (size_t)k * n2;
-        v_on_u_T(P, o, k, c, cS, cE, cSE, k < kf.x ? 1.0 : 0.0, avpv_b[o + c], v_b);
-        u_on_v_T(P, o, k, c, cW, cN, cNW, k < kf.y ? 1.0 : 0.0, avpu_b[o + c], u_b);
-    }
+    const int k = blockIdx.z;
+    const size_t o = (size_t)k * n2;
+    v_on_u_T(P, o, k, c, cS, cE, cSE, k < kf.x ? 1.0 : 0.0, P.one_m_tc * (P.dt * P.f0 * stu_b[o + c]), v_b);
+    u_on_v_T(P, o, k, c, cW, cN, cNW, k < kf.y ? 1.0 : 0.0, P.one_m_tc * (P.dt * P.neg_f0 * stv_b[o + c]), u_b);
 }
 
 // explicit vertical diffusion of the face velocities with the surface stress
 // (dzu = Dz[u; K_m, dz3u, tau_u, drag]) and the stress increment st_u[0] =
-// thv dt tau_u / dz3u[0]: u_b += Dz^T dzu_b, tau_u_b = its surface cotangent
-template <int NZM>
-__global__ void k_explicit_dz_T(KP P, const double* __restrict__ dzu_b, const double* __restrict__ dzv_b,
-                                const double* __restrict__ stu_b, const double* __restrict__ stv_b,
+// thv dt tau_u / dz3u[0], and the predictor's own u: u_b += c3 Dz^T st_u_b + st_u_b,
+// tau_u_b = its surface cotangent
+__global__ void k_explicit_dz_T(KP P, const double* __restrict__ stu_b, const double* __restrict__ stv_b,
                                 double* __restrict__ u_b, double* __restrict__ v_b, double* __restrict__ tau_u_b,
                                 double* __restrict__ tau_v_b) {
     ADJ_PROLOGUE
+    const int k = blockIdx.z;
     const int2 kf = P.kface[c];
-    double dzf[NZM], m3c[NZM], rb[NZM], fb[NZM];
-    for (int k = 0; k < nz; ++k) {
+    const ColGeo g = ColGeo::load(P, c), ge = ColGeo::load(P, cE), gn = ColGeo::load(P, cN);
+    auto wet = [&](int kk) {
         double m;
-        col_dz(P, c, k, m);
-        m3c[k] = m;
-    }
+        g.dz(P, kk, m);
+        return m;
+    };
+#pragma unroll
     for (int f = 0; f < 2; ++f) {
-        const double* src = f == 0 ? dzu_b : dzv_b;
+        const double* src = f == 0 ? stu_b : stv_b;
         double* dst = f == 0 ? u_b : v_b;
-        const int cn = f == 0 ? cE : cN;
-        const int kk = f == 0 ? kf.x : kf.y;
-        for (int k = 0; k < nz; ++k) {
-            dzf[k] = face_thick(P, c, cn, kk, k);
-            rb[k] = src[(size_t)k * n2 + c];
-            fb[k] = 0.0;
-        }
-        const double surf_b = explicit_dz_T<NZM>(P, dzf, m3c, P.nu, P.bottom_drag, rb, fb);
-        for (int k = 0; k < nz; ++k) dst[(size_t)k * n2 + c] += fb[k];
-        const double st0 = (f == 0 ? stu_b : stv_b)[c];
-        const double t = surf_b + P.thv_dt * inv_pos(dzf[0]) * st0;
-        (f == 0 ? tau_u_b : tau_v_b)[c] = t;
+        const ColGeo& gf = f == 0 ? ge : gn;
+        const int kk_f = f == 0 ? kf.x : kf.y;
+        auto thick = [&](int kk) {
+            double m;
+            return face_dz(P, kk_f, kk, g.dz(P, kk, m), gf.dz(P, kk, m));
+        };
+        double surf;
+        const double fb = explicit_dz_T(k, nz, thick, wet, [&](int kk) { return P.c3 * src[(size_t)kk * n2 + c]; }, P.nu,
+                                        P.bottom_drag, 0.0, surf);
+        dst[(size_t)k * n2 + c] += fb + src[(size_t)k * n2 + c];
+        if (k == 0)
+            (f == 0 ? tau_u_b : tau_v_b)[c] = surf + P.thv_dt * inv_pos(thick(0)) * src[c];
     }
 }
 
@@ -637,6 +735,8 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
     const int cSE = (j == 0 ? ny - 1 : j - 1) * nx + (i + 1 == nx ? 0 : i + 1);
     const int cNW = (j + 1 == ny ? 0 : j + 1) * nx + (i == 0 ? nx - 1 : i - 1);
     const double dz_nom = P.dz_nom[k];
+    const unsigned mask = row_mask(i, nx);
+    Scatter gu, gv, gw;
     // adv cotangents: ex = -adv m3f, ex_b = dt st_b
     auto au_b = [&](int cc, int kk) { return -P.dt * stu_b[(size_t)kk * n2 + cc] * col_m3u(P, cc, kk); };
     auto av_b = [&](int cc, int kk) { return -P.dt * stv_b[(size_t)kk * n2 + cc] * col_m3v(P, cc, kk); };
@@ -653,17 +753,17 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                                              col_m3u(P, cWW, k) > 0.0, col_m3u(P, cE, k) > 0.0);
                     val = fc.f;
                     const double s = F_b * ub;
-                    atomic_add(&u_b[o + cWW], s * fc.dm);
-                    atomic_add(&u_b[o + cW], s * fc.d0);
-                    atomic_add(&u_b[o + c], s * fc.d1);
-                    atomic_add(&u_b[o + cE], s * fc.dp);
+                    gu.ww += s * fc.dm;
+                    gu.w += s * fc.d0;
+                    gu.c += s * fc.d1;
+                    gu.e += s * fc.dp;
                 } else {
                     val = ub;
-                    atomic_add(&u_b[o + cW], F_b * ub * 0.5);
-                    atomic_add(&u_b[o + c], F_b * ub * 0.5);
+                    gu.w += F_b * ub * 0.5;
+                    gu.c += F_b * ub * 0.5;
                 }
-                atomic_add(&u_b[o + cW], 0.5 * F_b * val);
-                atomic_add(&u_b[o + c], 0.5 * F_b * val);
+                gu.w += 0.5 * F_b * val;
+                gu.c += 0.5 * F_b * val;
             }
         }
         // ---- u: corner flux fy north of u face c: vbar = (v_c + v_E)/2, face of u between c and N
@@ -677,17 +777,17 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                                              col_m3u(P, cS, k) > 0.0, col_m3u(P, cNN, k) > 0.0);
                     val = fc.f;
                     const double s = fy_b * vb;
-                    atomic_add(&u_b[o + cS], s * fc.dm);
-                    atomic_add(&u_b[o + c], s * fc.d0);
-                    atomic_add(&u_b[o + cN], s * fc.d1);
-                    atomic_add(&u_b[o + cNN], s * fc.dp);
+                    gu.s += s * fc.dm;
+                    gu.c += s * fc.d0;
+                    gu.n += s * fc.d1;
+                    gu.nn += s * fc.dp;
                 } else {
                     val = 0.5 * (u[o + c] + u[o + cN]);
-                    atomic_add(&u_b[o + c], fy_b * vb * 0.5);
-                    atomic_add(&u_b[o + cN], fy_b * vb * 0.5);
+                    gu.c += fy_b * vb * 0.5;
+                    gu.n += fy_b * vb * 0.5;
                 }
-                atomic_add(&v_b[o + c], 0.5 * fy_b * val);
-                atomic_add(&v_b[o + cE], 0.5 * fy_b * val);
+                gv.c += 0.5 * fy_b * val;
+                gv.e += 0.5 * fy_b * val;
             }
         }
         // ---- u: vertical flux at interface k of u face c (1 <= k <= nz-1)
@@ -704,17 +804,17 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                     const Face fc = face_lin(P, scheme, fd, bl, ab, fu, wb, hd, hu);
                     val = fc.f;
                     const double s = fz_b * wb;
-                    if (k + 1 <= nz - 1) atomic_add(&u_b[o + n2 + c], s * fc.dm);
-                    atomic_add(&u_b[o + c], s * fc.d0);
-                    atomic_add(&u_b[o - n2 + c], s * fc.d1);
-                    if (k >= 2) atomic_add(&u_b[o - 2 * n2 + c], s * fc.dp);
+                    if (k + 1 <= nz - 1) gu.dn += s * fc.dm;
+                    gu.c += s * fc.d0;
+                    gu.up += s * fc.d1;
+                    if (k >= 2) gu.up2 += s * fc.dp;
                 } else {
                     val = 0.5 * (ab + bl);
-                    atomic_add(&u_b[o + c], fz_b * wb * 0.5);
-                    atomic_add(&u_b[o - n2 + c], fz_b * wb * 0.5);
+                    gu.c += fz_b * wb * 0.5;
+                    gu.up += fz_b * wb * 0.5;
                 }
-                atomic_add(&w_b[o + c], 0.5 * fz_b * val);
-                atomic_add(&w_b[o + cE], 0.5 * fz_b * val);
+                gw.c += 0.5 * fz_b * val;
+                gw.e += 0.5 * fz_b * val;
             }
         }
         // ---- v: centre flux G[c] = vb_c vc_c, vb_c = (v_S + v_c)/2; by = (G_N - G)/dy at v face c
@@ -728,17 +828,17 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                                              col_m3v(P, cSS, k) > 0.0, col_m3v(P, cN, k) > 0.0);
                     val = fc.f;
                     const double s = G_b * vb;
-                    atomic_add(&v_b[o + cSS], s * fc.dm);
-                    atomic_add(&v_b[o + cS], s * fc.d0);
-                    atomic_add(&v_b[o + c], s * fc.d1);
-                    atomic_add(&v_b[o + cN], s * fc.dp);
+                    gv.ss += s * fc.dm;
+                    gv.s += s * fc.d0;
+                    gv.c += s * fc.d1;
+                    gv.n += s * fc.dp;
                 } else {
                     val = vb;
-                    atomic_add(&v_b[o + cS], G_b * vb * 0.5);
-                    atomic_add(&v_b[o + c], G_b * vb * 0.5);
+                    gv.s += G_b * vb * 0.5;
+                    gv.c += G_b * vb * 0.5;
                 }
-                atomic_add(&v_b[o + cS], 0.5 * G_b * val);
-                atomic_add(&v_b[o + c], 0.5 * G_b * val);
+                gv.s += 0.5 * G_b * val;
+                gv.c += 0.5 * G_b * val;
             }
         }
         // ---- v: corner flux fx east of v face c: ubar = (u_c + u_N)/2, face of v between c and E
@@ -752,17 +852,17 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                                              col_m3v(P, cW, k) > 0.0, col_m3v(P, cEE, k) > 0.0);
                     val = fc.f;
                     const double s = fx_b * ub;
-                    atomic_add(&v_b[o + cW], s * fc.dm);
-                    atomic_add(&v_b[o + c], s * fc.d0);
-                    atomic_add(&v_b[o + cE], s * fc.d1);
-                    atomic_add(&v_b[o + cEE], s * fc.dp);
+                    gv.w += s * fc.dm;
+                    gv.c += s * fc.d0;
+                    gv.e += s * fc.d1;
+                    gv.ee += s * fc.dp;
                 } else {
                     val = 0.5 * (v[o + c] + v[o + cE]);
-                    atomic_add(&v_b[o + c], fx_b * ub * 0.5);
-                    atomic_add(&v_b[o + cE], fx_b * ub * 0.5);
+                    gv.c += fx_b * ub * 0.5;
+                    gv.e += fx_b * ub * 0.5;
                 }
-                atomic_add(&u_b[o + c], 0.5 * fx_b * val);
-                atomic_add(&u_b[o + cN], 0.5 * fx_b * val);
+                gu.c += 0.5 * fx_b * val;
+                gu.n += 0.5 * fx_b * val;
             }
         }
         // ---- v: vertical flux at interface k of v face c
@@ -779,26 +879,27 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
                     const Face fc = face_lin(P, scheme, fd, bl, ab, fu, wb, hd, hu);
                     val = fc.f;
                     const double s = fz_b * wb;
-                    if (k + 1 <= nz - 1) atomic_add(&v_b[o + n2 + c], s * fc.dm);
-                    atomic_add(&v_b[o + c], s * fc.d0);
-                    atomic_add(&v_b[o - n2 + c], s * fc.d1);
-                    if (k >= 2) atomic_add(&v_b[o - 2 * n2 + c], s * fc.dp);
+                    if (k + 1 <= nz - 1) gv.dn += s * fc.dm;
+                    gv.c += s * fc.d0;
+                    gv.up += s * fc.d1;
+                    if (k >= 2) gv.up2 += s * fc.dp;
                 } else {
                     val = 0.5 * (ab + bl);
-                    atomic_add(&v_b[o + c], fz_b * wb * 0.5);
-                    atomic_add(&v_b[o - n2 + c], fz_b * wb * 0.5);
+                    gv.c += fz_b * wb * 0.5;
+                    gv.up += fz_b * wb * 0.5;
                 }
-                atomic_add(&w_b[o + c], 0.5 * fz_b * val);
-                atomic_add(&w_b[o + cN], 0.5 * fz_b * val);
+                gw.c += 0.5 * fz_b * val;
+                gw.n += 0.5 * fz_b * val;
             }
         }
     }
     if (P.a_h > 0.0) {
         // a_h lap(f) with face masks m3u (x) and m3v (y) and cell mask m of the component:
         // lap = m ((gx - W gx)/dx + (gy - S gy)/dy), gx = m3u (E f - f)/dx, gy = m3v (N f - f)/dy
+#pragma unroll
         for (int comp = 0; comp < 2; ++comp) {
             const double* st_b = comp ? stv_b : stu_b;
-            double* fb = comp ? v_b : u_b;
+            Scatter& g = comp ? gv : gu;
             auto lc = [&](int cc) {
                 const double m = comp ? col_m3v(P, cc, k) : col_m3u(P, cc, k);
                 return P.dt * P.a_h * st_b[o + cc] * m;
@@ -806,49 +907,70 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
             const double l_c = lc(c), l_e = lc(cE), l_n = lc(cN);
             const double gx_b = (l_c - l_e) / P.dx64 * col_m3u(P, c, k) / P.dx64;
             const double gy_b = (l_c - l_n) / P.dy64 * col_m3v(P, c, k) / P.dy64;
-            atomic_add(&fb[o + cE], gx_b);
-            atomic_add(&fb[o + c], -gx_b - gy_b);
-            atomic_add(&fb[o + cN], gy_b);
+            g.e += gx_b;
+            g.c += -gx_b - gy_b;
+            g.n += gy_b;
         }
     }
+    double gu_own;
+    scatter_x(u_b, o, gu, gu_own, i, j, nx, mask);
+    atomic_add(&u_b[o + c], gu_own);
+    atomic_add(&u_b[o + cS], gu.s);
+    atomic_add(&u_b[o + cN], gu.n);
+    atomic_add(&u_b[o + cNN], gu.nn);
+    if (k + 1 < nz) atomic_add(&u_b[o + n2 + c], gu.dn);
+    if (k >= 1) atomic_add(&u_b[o - n2 + c], gu.up);
+    if (k >= 2) atomic_add(&u_b[o - 2 * n2 + c], gu.up2);
+    double gv_own;
+    scatter_x(v_b, o, gv, gv_own, i, j, nx, mask);
+    atomic_add(&v_b[o + c], gv_own);
+    atomic_add(&v_b[o + cS], gv.s);
+    atomic_add(&v_b[o + cSS], gv.ss);
+    atomic_add(&v_b[o + cN], gv.n);
+    if (k + 1 < nz) atomic_add(&v_b[o + n2 + c], gv.dn);
+    if (k >= 1) atomic_add(&v_b[o - n2 + c], gv.up);
+    if (k >= 2) atomic_add(&v_b[o - 2 * n2 + c], gv.up2);
+    double gw_own;
+    scatter_x(w_b, o, gw, gw_own, i, j, nx, mask);
+    atomic_add(&w_b[o + c], gw_own);
+    atomic_add(&w_b[o + cN], gw.n);
     (void)cSE;
     (void)cNW;
 }
 
 // pressure gradient (model3d_v05.py:211-230): pg = m3f ((phi_F + b_F (zf - zc_F)) -
 // (phi + b (zf - zc))) / dx at the east / north face: phi_b and b_b gathered
-__global__ void k_pgf_T(KP P, const double* __restrict__ pgx_b, const double* __restrict__ pgy_b,
+__global__ void k_pgf_T(KP P, const double* __restrict__ stu_b, const double* __restrict__ stv_b,
                         double* __restrict__ phi_b, double* __restrict__ b_b) {
     ADJ_PROLOGUE
     const ColGeo gc = ColGeo::load(P, c), gw = ColGeo::load(P, cW), ge = ColGeo::load(P, cE);
     const ColGeo gs = ColGeo::load(P, cS), gn = ColGeo::load(P, cN);
-    for (int k = 0; k < nz; ++k) {
-        const size_t o = (size_t)k * n2;
-        double m;
-        const double zc = gc.above(P, k) + 0.5 * gc.dz(P, k, m);
-        const double zw = gw.above(P, k) + 0.5 * gw.dz(P, k, m);
-        const double ze = ge.above(P, k) + 0.5 * ge.dz(P, k, m);
-        const double zs = gs.above(P, k) + 0.5 * gs.dz(P, k, m);
-        const double zn = gn.above(P, k) + 0.5 * gn.dz(P, k, m);
-        // faces: east of c (c is the left cell), east of W (c is the right cell), same in y
-        const double ge_b = col_m3u(P, c, k) * pgx_b[o + c] / P.dx64;
-        const double gw_b = col_m3u(P, cW, k) * pgx_b[o + cW] / P.dx64;
-        const double gn_b = col_m3v(P, c, k) * pgy_b[o + c] / P.dy64;
-        const double gs_b = col_m3v(P, cS, k) * pgy_b[o + cS] / P.dy64;
-        double pb, bb;
-        if (P.pgf_correction) {
-            pb = gw_b - ge_b + gs_b - gn_b;
-            bb = -ge_b * (0.5 * (zc + ze) - zc) + gw_b * (0.5 * (zw + zc) - zc) - gn_b * (0.5 * (zc + zn) - zc) +
-                 gs_b * (0.5 * (zs + zc) - zc);
-        } else {
-            // pg = m3f (phi_F - phi) / dx m3f
-            pb = col_m3u(P, cW, k) * gw_b - col_m3u(P, c, k) * ge_b + col_m3v(P, cS, k) * gs_b -
-                 col_m3v(P, c, k) * gn_b;
-            bb = 0.0;
-        }
-        phi_b[o + c] = pb;
-        b_b[o + c] += bb;
+    const int k = blockIdx.z;
+    const size_t o = (size_t)k * n2;
+    double m;
+    const double zc = gc.above(P, k) + 0.5 * gc.dz(P, k, m);
+    const double zw = gw.above(P, k) + 0.5 * gw.dz(P, k, m);
+    const double ze = ge.above(P, k) + 0.5 * ge.dz(P, k, m);
+    const double zs = gs.above(P, k) + 0.5 * gs.dz(P, k, m);
+    const double zn = gn.above(P, k) + 0.5 * gn.dz(P, k, m);
+    // faces: east of c (c is the left cell), east of W (c is the right cell), same in y
+    const double ge_b = col_m3u(P, c, k) * (P.dt * stu_b[o + c]) / P.dx64;
+    const double gw_b = col_m3u(P, cW, k) * (P.dt * stu_b[o + cW]) / P.dx64;
+    const double gn_b = col_m3v(P, c, k) * (P.dt * stv_b[o + c]) / P.dy64;
+    const double gs_b = col_m3v(P, cS, k) * (P.dt * stv_b[o + cS]) / P.dy64;
+    double pb, bb;
+    if (P.pgf_correction) {
+        pb = gw_b - ge_b + gs_b - gn_b;
+        bb = -ge_b * (0.5 * (zc + ze) - zc) + gw_b * (0.5 * (zw + zc) - zc) - gn_b * (0.5 * (zc + zn) - zc) +
+             gs_b * (0.5 * (zs + zc) - zc);
+    } else {
+        // pg = m3f (phi_F - phi) / dx m3f
+        pb = col_m3u(P, cW, k) * gw_b - col_m3u(P, c, k) * ge_b + col_m3v(P, cS, k) * gs_b -
+             col_m3v(P, c, k) * gn_b;
+        bb = 0.0;
     }
+    phi_b[o + c] = pb;
+    b_b[o + c] += bb;
 }
 
 // phi[k] = 0.5 dz b[k] + sum_{k' < k} dz b[k'] (vertical_var.py:132-136):
@@ -916,8 +1038,7 @@ struct AdjointWork {
     double *rT_b = nullptr, *rS_b = nullptr;
     double *it_u[2] = {}, *it_v[2] = {};
     double *ghu_b = nullptr, *ghv_b = nullptr, *ru_b = nullptr, *rv_b = nullptr;
-    double *stu_b = nullptr, *stv_b = nullptr, *pgx_b = nullptr, *pgy_b = nullptr;
-    double *dzu_b = nullptr, *dzv_b = nullptr, *avpv_b = nullptr, *avpu_b = nullptr, *phi_b = nullptr;
+    double *stu_b = nullptr, *stv_b = nullptr, *phi_b = nullptr;
     double *gx_b = nullptr, *gy_b = nullptr, *eta_m_b = nullptr, *rhs_b = nullptr, *Ug_b = nullptr,
            *Vg_b = nullptr, *divold_b = nullptr, *gx2_b = nullptr, *gy2_b = nullptr, *tau_u_b = nullptr,
            *tau_v_b = nullptr;
@@ -950,8 +1071,7 @@ static int adjoint_setup(oc_handle* h) {
     bool ok = true;
     for (double** p : {&a->w_old, &a->w_new, &a->w_b}) ok = ok && (*p = adj_alloc(a, n3i));
     for (double** p : {&a->td_b, &a->rT_b, &a->rS_b, &a->it_u[0], &a->it_u[1], &a->it_v[0], &a->it_v[1], &a->ghu_b,
-                       &a->ghv_b, &a->ru_b, &a->rv_b, &a->stu_b, &a->stv_b, &a->pgx_b, &a->pgy_b, &a->dzu_b,
-                       &a->dzv_b, &a->avpv_b, &a->avpu_b, &a->phi_b})
+                       &a->ghv_b, &a->ru_b, &a->rv_b, &a->stu_b, &a->stv_b, &a->phi_b})
         ok = ok && (*p = adj_alloc(a, n3));
     for (double** p : {&a->gx_b, &a->gy_b, &a->eta_m_b, &a->rhs_b, &a->Ug_b, &a->Vg_b, &a->divold_b, &a->gx2_b,
                        &a->gy2_b, &a->tau_u_b, &a->tau_v_b})
@@ -996,6 +1116,7 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
     const size_t n2 = h->n2, n3 = h->n3, n3i = h->n3i;
     const dim3 cb = col_block(), cg = col_grid(P);
     const dim3 vb(32, 4, 1), vg((P.nx + 31) / 32, (P.ny + 3) / 4, P.nz);
+    const dim3 lb(32, ADJ_LY), lg((unsigned)(((P.nx + 31) / 32) * P.ny));
     auto zero = [&](double* p, size_t n) { cudaMemsetAsync(p, 0, n * sizeof(double), s); };
     // forward values: w of the state before and after the step
     launch_wcol(P, x0->u, x0->v, A.w_old, s);
@@ -1003,14 +1124,14 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
     // outputs start from zero
     for (double* p : {x0_b->u, x0_b->v, x0_b->b, x0_b->T, x0_b->S}) zero(p, n3);
     zero(x0_b->eta, n2);
-    for (double* p : {A.stu_b, A.stv_b, A.pgx_b, A.pgy_b, A.dzu_b, A.dzv_b, A.avpv_b, A.avpu_b}) zero(p, n3);
+    for (double* p : {A.stu_b, A.stv_b}) zero(p, n3);
     for (double* p : {A.divold_b, A.gx2_b, A.gy2_b}) zero(p, n2);
     zero(A.w_b, n3i);
     // ---- EOS and the implicit tracer solves
     NZ_DISPATCH_ADJ(P.nz, (k_tracer_solve_T<NZM><<<cg, cb, 0, s>>>(P, x1->T, x1->S, x1_b->T, x1_b->S, x1_b->b,
                                                                     A.rT_b, A.rS_b)));
     // ---- tracer right-hand sides: the identity and vertical diffusion, then advection
-    NZ_DISPATCH_ADJ(P.nz, (k_tracer_rhs_T_col<NZM><<<cg, cb, 0, s>>>(P, A.rT_b, A.rS_b, x0_b->T, x0_b->S)));
+    k_tracer_rhs_T_col<<<vg, vb, 0, s>>>(P, A.rT_b, A.rS_b, x0_b->T, x0_b->S);
     // the last iterate's cotangent starts as the output's
     double* uit_b = A.it_u[0];
     double* vit_b = A.it_v[0];
@@ -1020,10 +1141,10 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
                                      uit_b, vit_b, A.w_b);
     // w of the new velocities
     k_wcol_T1<<<cg, cb, 0, s>>>(P, A.w_b, A.td_b);
-    k_wcol_T2<<<cg, cb, 0, s>>>(P, A.td_b, uit_b, vit_b);
+    k_wcol_T2<<<vg, vb, 0, s>>>(P, A.td_b, uit_b, vit_b);
     // ---- Picard passes, last first
     for (int m = cf.n_picard - 1; m >= 0; --m) {
-        k_backsub_T<<<cg, cb, 0, s>>>(P, uit_b, vit_b, h->q, A.ghu_b, A.ghv_b, A.gx_b, A.gy_b);
+        k_backsub_T<<<lg, lb, 0, s>>>(P, uit_b, vit_b, h->q, A.ghu_b, A.ghv_b, A.gx_b, A.gy_b);
         k_grad2_T<<<cg, cb, 0, s>>>(P, A.gx_b, A.gy_b, A.eta_m_b, 1, m == cf.n_picard - 1 ? x1_b->eta : nullptr);
         rc = A.solver->solve(A.eta_m_b, A.rhs_b, s, h->err);
         if (rc) return rc;
@@ -1037,8 +1158,7 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
             zero(nu_b, n3);
             zero(nv_b, n3);
         }
-        k_predictor_T<<<cg, cb, 0, s>>>(P, A.ru_b, A.rv_b, x0_b->u, x0_b->v, nu_b, nv_b, A.avpv_b, A.avpu_b,
-                                        A.pgx_b, A.pgy_b, A.dzu_b, A.dzv_b, A.stu_b, A.stv_b, A.gx2_b, A.gy2_b);
+        k_predictor_T<<<lg, lb, 0, s>>>(P, A.ru_b, A.rv_b, nu_b, nv_b, A.stu_b, A.stv_b, A.gx2_b, A.gy2_b);
         uit_b = nu_b;
         vit_b = nv_b;
     }
@@ -1049,11 +1169,10 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
     zero(A.w_b, n3i);
     k_mom_adv_T<<<vg, vb, 0, s>>>(P, x0->u, x0->v, A.w_old, A.stu_b, A.stv_b, x0_b->u, x0_b->v, A.w_b);
     k_wcol_T1<<<cg, cb, 0, s>>>(P, A.w_b, A.td_b);
-    k_wcol_T2<<<cg, cb, 0, s>>>(P, A.td_b, x0_b->u, x0_b->v);
-    NZ_DISPATCH_ADJ(P.nz, (k_explicit_dz_T<NZM><<<cg, cb, 0, s>>>(P, A.dzu_b, A.dzv_b, A.stu_b, A.stv_b, x0_b->u,
-                                                                   x0_b->v, A.tau_u_b, A.tau_v_b)));
-    k_coriolis_old_T<<<cg, cb, 0, s>>>(P, A.avpv_b, A.avpu_b, x0_b->u, x0_b->v);
-    k_pgf_T<<<cg, cb, 0, s>>>(P, A.pgx_b, A.pgy_b, A.phi_b, x0_b->b);
+    k_wcol_T2<<<vg, vb, 0, s>>>(P, A.td_b, x0_b->u, x0_b->v);
+    k_explicit_dz_T<<<vg, vb, 0, s>>>(P, A.stu_b, A.stv_b, x0_b->u, x0_b->v, A.tau_u_b, A.tau_v_b);
+    k_coriolis_old_T<<<vg, vb, 0, s>>>(P, A.stu_b, A.stv_b, x0_b->u, x0_b->v);
+    k_pgf_T<<<vg, vb, 0, s>>>(P, A.stu_b, A.stv_b, A.phi_b, x0_b->b);
     k_phi_T<<<cg, cb, 0, s>>>(P, A.phi_b, x0_b->b);
     k_stress_T<<<cg, cb, 0, s>>>(P, A.tau_u_b, A.tau_v_b, taux_b, tauy_b);
     return check_launch(h, "oc_adjoint_step");
