@@ -353,6 +353,171 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
     column_q(P, g, [&](int k) { return km[(size_t)k * n2 + c]; }, cst, q, c, n2);
 }
 
+// The same closure by levels, for the Gaspar lengths, which march over the column from
+// each interface and take most of the time: a CTA takes CL_X columns of a row with
+// CL_Y threads each. The threads form N^2, the lengths and the rows of the column's
+// interfaces side by side, in shared memory; the two eliminations are done by one
+// thread a column, with a column's lengths spread over as many warps as can hide them.
+// Values and their operations are k_closure's. For few columns: us a launch by columns and
+// by levels, 48 x 48 x 12 9.5 and 3.5, 16,384 x 50 211 and 99, 32,000 x 40 96 and 61; at
+// 262,144 x 50 732 and 938, where k_closure has warps enough and the shared arrays leave
+// this one 24 to an SM. Four or sixteen threads a column are within 20% of eight.
+constexpr int CL_X = 32, CL_Y = 8;
+__global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
+    KPR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b, real* __restrict__ e,
+    real* __restrict__ km, real* __restrict__ kh, real* __restrict__ q) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    const int tiles = (P.nx + CL_X - 1) / CL_X;
+    const int j = blockIdx.x / tiles, i_own = (blockIdx.x - j * tiles) * CL_X + threadIdx.x;
+    const bool live = i_own < P.nx;  // the others repeat the last column and store nothing
+    const int i = live ? i_own : P.nx - 1;
+    const int nz = P.nz, nx = P.nx, rows = (nz + 1) * CL_X, first = threadIdx.y;
+    const size_t n2 = (size_t)P.n2;
+    const int c = j * nx + i, cw = j * nx + wrapi(i - 1, nx), cs_ = wrapi(j - 1, P.ny) * nx + i;
+    const ColGeoR g = ColGeoR::load(P, c);
+    // of the thread's column, interface k at [k * CL_X]: N^2, then the new K_m; the rows,
+    // of which sup becomes the elimination's coefficient and rhs the solution
+    real* s_n2 = reinterpret_cast<real*>(s_dyn) + threadIdx.x;
+    real *s_sub = s_n2 + rows, *s_dia = s_sub + rows, *s_sup = s_dia + rows, *s_rhs = s_sup + rows;
+    auto wet = [&](int k) { return k < g.kb ? real(1.0) : real(0.0); };
+    auto inner = [&](int k) { return (k >= 1 && k <= nz - 1) ? wet(k - 1) * wet(k) : real(0.0); };
+    // x of the rows: forward elimination, then back, in place
+    auto solve = [&](int n) {
+        real cp = real(0.0), ds = real(0.0);
+#pragma unroll 2
+        for (int k = 0; k < n; ++k) {
+            const real sub = s_sub[k * CL_X], dia = s_dia[k * CL_X], sup = s_sup[k * CL_X], rhs = s_rhs[k * CL_X];
+            if (k == 0) {
+                cp = sup / dia;
+                ds = rhs / dia;
+            } else {
+                const real den = dia - sub * cp;
+                cp = sup / den;
+                ds = (rhs - sub * ds) / den;
+            }
+            s_sup[k * CL_X] = cp;
+            s_rhs[k * CL_X] = ds;
+        }
+#pragma unroll 4
+        for (int k = n - 2; k >= 0; --k) {
+            ds = s_rhs[k * CL_X] - s_sup[k * CL_X] * ds;
+            s_rhs[k * CL_X] = ds;
+        }
+    };
+    // shear^2 (in the place of sub) and N^2 on interfaces (closure.py:150-161)
+#pragma unroll 2
+    for (int k = first; k <= nz; k += CL_Y) {
+        real sh2 = real(0.0), nn2 = real(0.0);
+        if (k >= 1 && k < nz) {
+            const size_t o = (size_t)k * n2, a = o - n2;
+            const real uc_prev = real(0.5) * (u[a + c] + u[a + cw]), uc = real(0.5) * (u[o + c] + u[o + cw]);
+            const real vc_prev = real(0.5) * (v[a + c] + v[a + cs_]), vc = real(0.5) * (v[o + c] + v[o + cs_]);
+            const real wk = wet(k), idz = g.rdzi(P, k);
+            const real du = (uc_prev - uc) * idz;
+            const real dv = (vc_prev - vc) * idz;
+            sh2 = (du * du + dv * dv) * wk;
+            // the difference of two fp64 buoyancies (their ~1e-2 relative
+            // vertical contrast would lose digits in FP32)
+            const real db = real((b[a + c] - b[o + c]) * idz);
+            nn2 = db * wk;
+        }
+        s_n2[k * CL_X] = nn2;
+        s_sub[k * CL_X] = sh2;
+    }
+    __syncthreads();
+    // lengths and implicit TKE rows (closure.py:65-104, 171-198)
+    const real depth = g.above(P, nz);
+    for (int k = first; k <= nz; k += CL_Y) {
+        const size_t o = (size_t)k * n2 + c;
+        const real km_cur = km[o], e_old = e[o], kh_old = kh[o];
+        const real km_prev = k >= 1 ? km[o - n2] : real(0.0), km_next = k < nz ? km[o + n2] : real(0.0);
+        const real wk = inner(k), zi = g.above(P, k);
+        const real zb = fmax(depth - zi, real(0.0));
+        const real ek = fmax(e_old, P.e_min);
+        // away from interface k until the energy budget is spent; once the budget is
+        // zero the reference's remaining steps add exactly 0
+        auto march = [&](int kk, int end, int step_k) {
+            real l = real(0.0), bud = ek;
+            for (; kk != end && bud > real(0.0); kk += step_k) {
+                const real n2j = fmax(s_n2[kk * CL_X], real(0.0)), dzj = col_dzi(P, g, kk);
+                const real cost = n2j * dzj * (l + real(0.5) * dzj);
+                const bool full = cost <= bud;
+                real step = dzj;
+                if (!full && n2j > real(0.0)) {
+                    const real part = sqrt(fmax(l * l + real(2.0) * bud / n2j, real(0.0))) - l;
+                    step = fmin(fmax(part, real(0.0)), dzj);
+                }
+                l = l + step;
+                bud = full ? bud - cost : real(0.0);
+            }
+            return l;
+        };
+        const real lu = fmin(march(k - 1, -1, -1), zi + P.z_0) * wk;
+        const real ld = fmin(march(k + 1, nz + 1, 1), zb + P.z_0) * wk;
+        const real lk_k = fmax(P.l_min, sqrt(lu * ld));
+        const real le_k = fmax(P.l_min, fmin(lu, ld));
+        if (live) kh[o] = lk_k;  // until this thread turns it into K_h
+        const real prod = (km_cur - P.nu) * s_sub[k * CL_X] - (kh_old - P.kappa) * s_n2[k * CL_X];
+        const real diss = P.c_eps * sqrt(fmax(e_old, P.e_min)) / le_k;
+        real a_up = real(0.0), a_dn = real(0.0);
+        if (k >= 1 && k <= nz - 1) {
+            const real idzi = g.rdzi(P, k);
+            a_up = P.dt * (real(0.5) * (km_prev + km_cur)) * g.rdz(P, k - 1) * idzi;
+            a_dn = P.dt * (real(0.5) * (km_cur + km_next)) * g.rdz(P, k) * idzi;
+        }
+        real sub = -a_up, sup = -a_dn;
+        real diag = real(1.0) + a_up + a_dn + P.dt * diss;
+        real rhs = e_old + P.dt * prod;
+        if (wk <= real(0.0)) {
+            diag = real(1.0);
+            sub = real(0.0);
+            sup = real(0.0);
+            rhs = P.e_min;
+        }
+        if (k == 0) rhs = (g.kb > 0) ? P.e_bb * P.ustar2[c] : P.e_min;
+        s_sub[k * CL_X] = sub;
+        s_dia[k * CL_X] = diag;
+        s_sup[k * CL_X] = sup;
+        s_rhs[k * CL_X] = rhs;
+    }
+    __syncthreads();
+    if (threadIdx.y == 0) solve(nz + 1);
+    __syncthreads();
+    // e/K update (closure.py:198-205)
+    for (int k = first; k <= nz; k += CL_Y) {
+        const size_t o = (size_t)k * n2 + c;
+        const real wk = inner(k);
+        real en = fmax(s_rhs[k * CL_X], P.e_min);
+        en = (wk > real(0.0)) ? en : P.e_min;
+        if (k == 0) en = (g.kb > 0) ? P.e_bb * P.ustar2[c] : P.e_min;
+        const real kmn = P.c_k * kh[o] * sqrt(en) * wk + P.nu;
+        const real kx = kmn - P.nu;
+        const real khn = (P.pr_t == real(1.0) ? kx : kx / P.pr_t) + P.kappa;
+        s_n2[k * CL_X] = kmn;
+        if (live) {
+            e[o] = en;
+            km[o] = kmn;
+            kh[o] = khn;
+        }
+    }
+    __syncthreads();
+    // q for the new K_m (column_q)
+    for (int k = first; k < nz; k += CL_Y) {
+        real sub, diag, sup;
+        implicit_row_inv(P, k, g.rdz(P, k), wet(k), wet(k + 1), k == 0 ? g.rdz(P, 0) : g.rdzi(P, k),
+                         k + 1 < nz ? g.rdzi(P, k + 1) : real(0.0), s_n2[k * CL_X], s_n2[(k + 1) * CL_X],
+                         P.thv_dt_drag, sub, diag, sup);
+        s_sub[k * CL_X] = sub;
+        s_dia[k * CL_X] = diag;
+        s_sup[k * CL_X] = sup;
+        s_rhs[k * CL_X] = real(1.0);
+    }
+    __syncthreads();
+    if (threadIdx.y == 0) solve(nz);
+    __syncthreads();
+    for (int k = first; k < nz && live; k += CL_Y) q[(size_t)k * n2 + c] = s_rhs[k * CL_X];
+}
+
 // ------------------------------------------------------------------ sums over levels
 // Kernels whose levels are independent but for a running sum: a CTA takes LV_X columns
 // of a row with LV_Y threads each. The threads of a column form its levels' terms
@@ -1779,6 +1944,123 @@ __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restr
     }
 }
 
+// The same by levels, for few columns: a CTA takes SL_X columns of a row with SL_Y threads
+// each, which form the column's rows side by side in shared memory and, after the
+// elimination by a lane per column and field, its levels' EOS. us a launch by columns and
+// by levels: 16,384 x 50 65 and 44, 512 x 32 13.6 and 5.6, 46,937 x 37 38 and 35, 65,536 x 32 75
+// and 77, 262,144 x 50 306 and 448. (The momentum solve in this form gains at 16,384 and loses
+// from 32,000 on.)
+constexpr int SL_X = 32, SL_Y = 8;
+
+struct SolveRows {  // of the thread's column, level k at [k * SL_X]
+    real *sub, *dia, *sup, *r[2];
+    __device__ __forceinline__ SolveRows(unsigned char* s, int nz, int col) {
+        sub = reinterpret_cast<real*>(s) + col;
+        dia = sub + nz * SL_X;
+        sup = dia + nz * SL_X;
+        r[0] = sup + nz * SL_X;
+        r[1] = r[0] + nz * SL_X;
+    }
+};
+
+// Forward elimination and back substitution of all the CTA's columns, by its first two
+// warps: 16 columns each, the lanes of a warp's halves for the two right-hand sides. The
+// halves form the same coefficients and store them in the place of sup.
+__device__ __forceinline__ void solve_pairs(unsigned char* s, int nz) {
+    if (threadIdx.y >= 2) return;
+    const int lane = threadIdx.x;
+    const SolveRows R(s, nz, threadIdx.y * 16 + (lane & 15));
+    real* r = lane < 16 ? R.r[0] : R.r[1];
+    real cp = real(0.0), x = real(0.0);
+#pragma unroll 2
+    for (int k = 0; k < nz; ++k) {
+        const real sub = R.sub[k * SL_X], dia = R.dia[k * SL_X], sup = R.sup[k * SL_X], y = r[k * SL_X];
+        __syncwarp();  // both halves have read sup
+        if (k == 0) {
+            cp = sup / dia;
+            x = y / dia;
+        } else {
+            const real den = dia - sub * cp;
+            cp = sup / den;
+            x = (y - sub * x) / den;
+        }
+        R.sup[k * SL_X] = cp;
+        r[k * SL_X] = x;
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int k = nz - 2; k >= 0; --k) {
+        x = r[k * SL_X] - R.sup[k * SL_X] * x;
+        r[k * SL_X] = x;
+    }
+}
+
+// the rows of level k of a column (implicit_row_inv)
+__device__ __forceinline__ void solve_row(const KPR& P, const ColGeoR& g, int k, real k_top, real k_bot, real drag,
+                                          const SolveRows& R) {
+    const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
+    const real rdzi_k = k == 0 ? g.rdz(P, 0) : g.rdzi(P, k), rdzi_k1 = k + 1 < P.nz ? g.rdzi(P, k + 1) : real(0.0);
+    real sub, diag, sup;
+    implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, k_top, k_bot, drag, sub, diag, sup);
+    R.sub[k * SL_X] = sub;
+    R.dia[k * SL_X] = diag;
+    R.sup[k * SL_X] = sup;
+}
+
+__global__ void __launch_bounds__(SL_X * SL_Y, 3) k_tracer_levels(KPR P, const real* __restrict__ rT,
+                                                                 const real* __restrict__ rS,
+                                                                 const real* __restrict__ kh, real* __restrict__ T_out,
+                                                                 real* __restrict__ S_out, wide* __restrict__ b_out) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    const int tiles = (P.nx + SL_X - 1) / SL_X;
+    const int j = blockIdx.x / tiles, i_own = (blockIdx.x - j * tiles) * SL_X + threadIdx.x;
+    const bool live = i_own < P.nx;  // the others repeat the last column and store nothing
+    const int i = live ? i_own : P.nx - 1, nz = P.nz, first = threadIdx.y;
+    const size_t n2 = (size_t)P.n2;
+    const int c = j * P.nx + i;
+    const ColGeoR g = ColGeoR::load(P, c);
+    const SolveRows R(s_dyn, nz, threadIdx.x);
+    const bool ts = P.tracers_ts;
+#pragma unroll 2
+    for (int k = first; k < nz; k += SL_Y) {
+        const size_t o = (size_t)k * n2 + c;
+        const real r1 = rT[o], r2 = ts ? rS[o] : real(0.0);
+        solve_row(P, g, k, kh[o], kh[o + n2], P.thv_dt_zero, R);
+        R.r[0][k * SL_X] = r1;
+        R.r[1][k * SL_X] = r2;
+    }
+    __syncthreads();
+    solve_pairs(s_dyn, nz);
+    __syncthreads();
+#ifdef OC_MIXED
+    const ColGeo64 g64 = ColGeo64::load(P, c);
+#endif
+#pragma unroll 2
+    for (int k = first; k < nz; k += SL_Y) {
+        const size_t o = (size_t)k * n2 + c;
+        real m3;
+        const real dz = g.dz(P, k, m3);
+        const real Tn = R.r[0][k * SL_X] * m3;
+        wide bn;
+        if (ts) {
+            const real Sn = R.r[1][k * SL_X] * m3;
+#ifdef OC_MIXED
+            const wide zc = g64.above(P, k) + 0.5 * g64.dz(P, k);
+            (void)dz;
+#else
+            const wide zc = g.above(P, k) + real(0.5) * dz;
+#endif
+            bn = buoyancy_of(P, wide(Tn), wide(Sn), zc) * wide(m3);  // EOS in fp64 on both paths
+            if (live) {
+                T_out[o] = Tn;
+                S_out[o] = Sn;
+            }
+        } else {
+            bn = wide(Tn);
+        }
+        if (live) b_out[o] = bn;
+    }
+}
 
 // diagnose b = EOS(T, S, zc) * m3 on the model grid (initial states)
 __global__ void k_diag_buoyancy(KPR P, const real* __restrict__ T, const real* __restrict__ S,
@@ -1870,6 +2152,22 @@ static void closure_nzm(const KPR& P, const real* u, const real* v, const wide* 
 }
 void launch_closure(const KPR& P, const real* u, const real* v, const wide* b, real* e,
                     real* km, real* kh, real* q, cudaStream_t s) {
+    if (!P.mxl_recursive && P.n2 <= kFewColumns) {
+        const size_t row = (size_t)5 * CL_X * sizeof(real);
+        // above 48 KB a kernel's dynamic shared memory is opt-in, once per device
+        static std::atomic<unsigned long long> opted{0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ULL << (dev & 63);
+        if (!(opted.load() & bit)) {
+            cudaFuncSetAttribute(k_closure_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)((OC_MAXNZ + 1) * row));
+            opted.fetch_or(bit);
+        }
+        const unsigned ctas = (unsigned)(((P.nx + CL_X - 1) / CL_X) * P.ny);
+        k_closure_levels<<<ctas, dim3(CL_X, CL_Y), (P.nz + 1) * row, s>>>(P, u, v, b, e, km, kh, q);
+        return;
+    }
     NZ_DISPATCH(P.nz, (closure_nzm<NZM>(P, u, v, b, e, km, kh, q, s)));
 }
 void launch_kukv(const KPR& P, const real* q, wide* Ku, wide* Kv, cudaStream_t s) {
@@ -1959,6 +2257,21 @@ void launch_tracer_rhs(const KPR& P, const real* C0, const real* S, const real* 
 }
 void launch_tracer_solve(const KPR& P, const real* rT, const real* rS, const real* kh,
                          real* T_out, real* S_out, wide* b_out, cudaStream_t s) {
+    if (P.n2 <= kFewColumns) {
+        const size_t row = (size_t)5 * SL_X * sizeof(real);
+        // above 48 KB a kernel's dynamic shared memory is opt-in, once per device
+        static std::atomic<unsigned long long> opted{0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ULL << (dev & 63);
+        if (!(opted.load() & bit)) {
+            cudaFuncSetAttribute(k_tracer_levels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(OC_MAXNZ * row));
+            opted.fetch_or(bit);
+        }
+        const unsigned ctas = (unsigned)(((P.nx + SL_X - 1) / SL_X) * P.ny);
+        k_tracer_levels<<<ctas, dim3(SL_X, SL_Y), P.nz * row, s>>>(P, rT, rS, kh, T_out, S_out, b_out);
+        return;
+    }
     NZ_DISPATCH(P.nz, (k_tracer_solve<NZM><<<col_grid(P), col_block(), 0, s>>>(P, rT, rS, kh, T_out,
                                                                              S_out, b_out)));
 }
