@@ -353,14 +353,14 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
     column_q(P, g, [&](int k) { return km[(size_t)k * n2 + c]; }, cst, q, c, n2);
 }
 
-// The same closure by levels, for the Gaspar lengths, which march over the column from
-// each interface and take most of the time: a CTA takes CL_X columns of a row with
-// CL_Y threads each. The threads form N^2, the lengths and the rows of the column's
+// The same closure by levels (the Gaspar lengths, which march over the column from each
+// interface, take most of its time): a CTA takes CL_X columns of a row with CL_Y threads
+// each. The threads form N^2, the lengths and the rows of the column's
 // interfaces side by side, in shared memory; the two eliminations are done by one
 // thread a column, with a column's lengths spread over as many warps as can hide them.
 // Values and their operations are k_closure's. For few columns: us a launch by columns and
-// by levels, 48 x 48 x 12 9.5 and 3.5, 16,384 x 50 211 and 99, 32,000 x 40 96 and 61; at
-// 262,144 x 50 732 and 938, where k_closure has warps enough and the shared arrays leave
+// by levels, 48 x 48 x 12 9.5 and 3.5, 16,384 x 50 211 and 99, 32,000 x 40 96 and 61, with
+// recursive lengths 46,937 x 37 206 and 170; at 262,144 x 50 732 and 938, where k_closure has warps enough and the shared arrays leave
 // this one 24 to an SM. Four or sixteen threads a column are within 20% of eight.
 constexpr int CL_X = 32, CL_Y = 8;
 __global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
@@ -425,8 +425,35 @@ __global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
         s_sub[k * CL_X] = sh2;
     }
     __syncthreads();
-    // lengths and implicit TKE rows (closure.py:65-104, 171-198)
     const real depth = g.above(P, nz);
+    if (P.mxl_recursive) {
+        // recursive lengths (closure.py:106-129), in the place of dia: the two sweeps over
+        // the column by one thread
+        for (int k = first; k <= nz; k += CL_Y) {
+            const real zi = g.above(P, k);
+            const real zb = fmax(depth - zi, real(0.0));
+            const real ek = fmax(e[(size_t)k * n2 + c], P.e_min);
+            const real n2c = fmax(s_n2[k * CL_X], P.n2_min);
+            const real ell = sqrt(real(2.0) * ek / n2c);
+            s_dia[k * CL_X] = fmin(ell, fmin(zi + P.z_0, zb + P.z_0));
+        }
+        __syncthreads();
+        if (threadIdx.y == 0) {
+            real l = s_dia[0];
+#pragma unroll 4
+            for (int k = 1; k <= nz; ++k) {
+                l = fmin(s_dia[k * CL_X], l + col_dzi(P, g, k));
+                s_dia[k * CL_X] = l;
+            }
+#pragma unroll 4
+            for (int k = nz - 1; k >= 0; --k) {
+                l = fmin(s_dia[k * CL_X], l + col_dzi(P, g, k + 1));
+                s_dia[k * CL_X] = l;
+            }
+        }
+        __syncthreads();
+    }
+    // lengths and implicit TKE rows (closure.py:65-104, 171-198)
     for (int k = first; k <= nz; k += CL_Y) {
         const size_t o = (size_t)k * n2 + c;
         const real km_cur = km[o], e_old = e[o], kh_old = kh[o];
@@ -452,8 +479,13 @@ __global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
             }
             return l;
         };
-        const real lu = fmin(march(k - 1, -1, -1), zi + P.z_0) * wk;
-        const real ld = fmin(march(k + 1, nz + 1, 1), zb + P.z_0) * wk;
+        real lu, ld;
+        if (!P.mxl_recursive) {
+            lu = fmin(march(k - 1, -1, -1), zi + P.z_0) * wk;
+            ld = fmin(march(k + 1, nz + 1, 1), zb + P.z_0) * wk;
+        } else {
+            lu = ld = s_dia[k * CL_X] * wk;
+        }
         const real lk_k = fmax(P.l_min, sqrt(lu * ld));
         const real le_k = fmax(P.l_min, fmin(lu, ld));
         if (live) kh[o] = lk_k;  // until this thread turns it into K_h
@@ -2152,7 +2184,7 @@ static void closure_nzm(const KPR& P, const real* u, const real* v, const wide* 
 }
 void launch_closure(const KPR& P, const real* u, const real* v, const wide* b, real* e,
                     real* km, real* kh, real* q, cudaStream_t s) {
-    if (!P.mxl_recursive && P.n2 <= kFewColumns) {
+    if (P.n2 <= kFewColumns) {
         const size_t row = (size_t)5 * CL_X * sizeof(real);
         // above 48 KB a kernel's dynamic shared memory is opt-in, once per device
         static std::atomic<unsigned long long> opted{0};

@@ -1,8 +1,8 @@
 """The column kernels, the adjoint's scatter and the EOS at the sizes where their forms change.
 
 Up to a number of columns a column's levels are shared by several threads (w, K_u and K_v,
-the back substitution) and its components by two (the momentum solve); above it a
-thread takes a column. Fields equal the oracle's bit for bit on both sides of the
+the back substitution, the closure, the tracer solve) and its components by two (the
+momentum solve); above it a thread takes a column. Fields equal the oracle's bit for bit on both sides of the
 limit, at level counts around the chunk of levels.
 """
 
@@ -14,15 +14,17 @@ from oracle import ocean_oracle as orc
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("mxl", ["integral", "recursive"])
 @pytest.mark.parametrize("nx,ny,nz", [
     (256, 192, 3), (256, 193, 3),   # the limit of the few-column forms, and just above it
     (128, 192, 2), (193, 128, 2),   # half of it (K_u, K_v)
     (45, 3, 33), (33, 5, 8), (7, 4, 1), (64, 2, 41),  # part-filled warps; around a chunk of levels
 ])
-def test_column_forms_match_oracle(nx, ny, nz):
+def test_column_forms_match_oracle(nx, ny, nz, mxl):
     from hydrostatic_ocean_core_benchmark_b200 import cases
     from hydrostatic_ocean_core_benchmark_b200.stepper import OceanStepper
-    s = cases.seamount_basin(nx=nx, ny=ny, nz=nz, seed=nx + ny, solver_kind="pcg_jacobi", rtol=1e-10)
+    s = cases.seamount_basin(nx=nx, ny=ny, nz=nz, seed=nx + ny, solver_kind="pcg_jacobi", rtol=1e-10,
+                             mxl=mxl)
     p = s.params
     geo = orc.Geometry(p, s.H, s.mask, s.dzr)
     b = orc.buoyancy(p.eos, s.T, s.S, geo.zc, p.g, p.rho0, p.alpha_t, p.beta_s, p.t0, p.s0) * geo.mask3
@@ -34,7 +36,7 @@ def test_column_forms_match_oracle(nx, ny, nz):
         state = ref.step(state)
         st.step(1)
         got = st.get_state()
-        for f in ("eta", "u", "v", "b", "T", "S"):
+        for f in ("eta", "u", "v", "b", "T", "S", "e"):
             assert np.array_equal(got[f], getattr(state, f)), f"step {step + 1}: {f} differs"
     st.close()
 
