@@ -518,7 +518,8 @@ __global__ void k_tracer_adv_T(KP P, const double* __restrict__ T, const double*
 
 // back-substitution u = (gh_u - c2 q gx(eta_new) m3u) m3 (model3d_v05.py:404-406):
 // gh_b = u_b m3 and the per-column cotangent of the surface gradient
-__global__ void __launch_bounds__(32 * ADJ_LY) k_backsub_T(KP P, const double* __restrict__ uo_b, const double* __restrict__ vo_b,
+__global__ void __launch_bounds__(32 * ADJ_LY) k_backsub_T(KP P, const double* __restrict__ uo_b,
+                            const double* __restrict__ vo_b,
                             const double* __restrict__ q, double* __restrict__ ghu_b, double* __restrict__ ghv_b,
                             double* __restrict__ gx_b, double* __restrict__ gy_b) {
     ADJ_LEVELS_PROLOGUE
@@ -637,8 +638,9 @@ __device__ __forceinline__ void u_on_v_T(const KP& P, size_t o, int k, int c, in
 // pass alike (u, st_u, pgx, dzu, the old average) are multiples of the right-hand
 // sides' cotangents summed over the passes, so only that sum is kept (stu_b, stv_b) and
 // each of their kernels scales it: ten arrays read and written per pass before, two
-// now (256 x 256 x 32: 188 us a pass by a thread per column, 134 by levels, 43 so). The iterate's average is scattered to it_b (u_b for the first pass, whose
-// iterate is the old state).
+// now (256 x 256 x 32: 188 us a pass by a thread per column, 134 by levels, 43 so). The
+// iterate's average is scattered to it_b (u_b for the first pass, whose iterate is the
+// old state).
 __global__ void __launch_bounds__(32 * ADJ_LY) k_predictor_T(
     KP P, const double* __restrict__ ru_b, const double* __restrict__ rv_b, double* __restrict__ uit_b,
     double* __restrict__ vit_b, double* __restrict__ stu_b, double* __restrict__ stv_b, double* __restrict__ gx2_b,

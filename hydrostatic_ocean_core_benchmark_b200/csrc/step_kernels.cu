@@ -357,11 +357,11 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
 // interface, take most of its time): a CTA takes CL_X columns of a row with CL_Y threads
 // each. The threads form N^2, the lengths and the rows of the column's
 // interfaces side by side, in shared memory; the two eliminations are done by one
-// thread a column, with a column's lengths spread over as many warps as can hide them.
-// Values and their operations are k_closure's. For few columns: us a launch by columns and
-// by levels, 48 x 48 x 12 9.5 and 3.5, 16,384 x 50 211 and 99, 32,000 x 40 96 and 61, with
-// recursive lengths 46,937 x 37 206 and 170; at 262,144 x 50 732 and 938, where k_closure has warps enough and the shared arrays leave
-// this one 24 to an SM. Four or sixteen threads a column are within 20% of eight.
+// thread a column. Values and their operations are k_closure's. For few columns: us a
+// launch by columns and by levels, 48 x 48 x 12 9.5 and 3.5, 16,384 x 50 211 and 99, 32,000 x
+// 40 96 and 61, with recursive lengths 46,937 x 37 206 and 170; at 262,144 x 50 732 and 938,
+// where k_closure has warps enough and the shared arrays leave this one 24 to an SM. Four
+// or sixteen threads a column are within 20% of eight.
 constexpr int CL_X = 32, CL_Y = 8;
 __global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
     KPR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b, real* __restrict__ e,
