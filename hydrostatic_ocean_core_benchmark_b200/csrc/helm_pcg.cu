@@ -210,7 +210,6 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
             re = re - apply_at(L0, H.coef, H.x, cell_of(nx, H.ny, g));
         }
         if constexpr (KEEP == PCG_KEEP_ALL) x[e] = H.warm ? __ldcg(H.x + g) : 0.0;
-        else if (!H.warm) x[e] = 0.0;
         const double ze = H.inv_diag[g] * re;
         r[e] = re;
         ap[e] = ze;
@@ -221,6 +220,11 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_helm_pcg(const PcgParams H) 
         const double b = H.rhs[s0 + e] * H.mask[s0 + e];
         return make_double2(b * b, r[e] * ap[e]);
     }, leafs[0], leafs[1]);
+    if constexpr (KEEP != PCG_KEEP_ALL)
+        if (!H.warm) {
+            __syncthreads();  // x may be the right-hand side's array, which the sums have read
+            for (int e = tid; e < own; e += PCG_THREADS) x[e] = 0.0;
+        }
     ok = pcg_sync<MODE>(H);
     if (ok) {
         const double* lv[2] = {leafs[0], leafs[1]};

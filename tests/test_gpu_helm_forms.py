@@ -103,3 +103,23 @@ def test_multigrid_forms_match_oracle(nx, ny):
         assert rep.iterations == itr and rep.converged == ok
         assert np.array_equal(x, xr)
     solver.close()
+
+
+@pytest.mark.parametrize("kind,nx,ny", [("pcg_jacobi", 40, 30), ("pcg_jacobi", 120, 130), ("pcg_jacobi", 400, 390),
+                                        ("pcg_jacobi", 1000, 720), ("pcg_jacobi", 5000, 300),
+                                        ("multigrid", 48, 40), ("multigrid", 256, 192)])
+def test_a_solve_in_place_gives_the_same_solution(kind, nx, ny):
+    """x may be the right-hand side's own device array."""
+    import ctypes as C
+    import torch
+    from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+    dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx, walls=True)
+    solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind=kind, rtol=1e-9)
+    want, rep = solver.solve(rhs)
+    a = torch.as_tensor(rhs, device="cuda:0").contiguous()
+    its, conv = C.c_int32(), C.c_int32()
+    solver._check(solver.lib.oc_helm_solve(solver.h, a.data_ptr(), a.data_ptr(), 1, C.byref(its), C.byref(conv),
+                                           torch.cuda.current_stream().cuda_stream), "oc_helm_solve")
+    assert its.value == rep.iterations
+    assert np.array_equal(a.cpu().numpy(), want)
+    solver.close()
