@@ -737,6 +737,21 @@ static PwNode pairwise_build_two_level(long start, long n, long block_leaves, Tw
 static constexpr long kFoldOneLevelLeaves = 16384;
 static constexpr long kFoldBlockLeaves = 8192;
 
+// Raises a solve kernel's shared-memory allowance on device `dev` to `smem` dynamic bytes.
+// The allowance belongs to the kernel on the device, not to a solver, and only ever
+// grows, so the solvers of other grids keep launching. What a kernel may have without it
+// is 48 KB less its static shared memory, so every size asks.
+static cudaError_t allow_smem(const void* kernel, size_t smem, int dev) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> allowance;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& a = allowance[{dev, kernel}];
+    if (smem <= a) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) a = smem;
+    return e;
+}
+
 void* HelmSolver::dalloc(size_t nbytes) {
     void* p = nullptr;
     if (cudaMalloc(&p, nbytes) != cudaSuccess) return nullptr;
@@ -1013,17 +1028,10 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         err = "Helmholtz grid too large for the single-pass reduction tree";
         return OC_ERR_UNSUPPORTED;
     }
-    if (smem_ > 48 * 1024) {
-        // the allowance belongs to the kernel on this device, not to this solver:
-        // it only ever grows, so the solvers of other grids keep launching
-        static std::mutex mu;
-        static std::map<int, size_t> allowance;
-        std::lock_guard<std::mutex> lock(mu);
-        size_t& a = allowance[dev];
-        if (smem_ > a) {
-            cudaFuncSetAttribute(k_helm_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_);
-            a = smem_;
-        }
+    if (const cudaError_t e = allow_smem((const void*)k_helm_solve, smem_, dev); e != cudaSuccess) {
+        cudaGetLastError();
+        err = std::string("Helmholtz solve kernel's shared memory: ") + cudaGetErrorString(e);
+        return OC_ERR_CUDA;
     }
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_helm_solve, block_, smem_);
@@ -1127,15 +1135,10 @@ int helm_batch_plan(HelmSolver* const* solvers, const double* const* rhs, double
         err = "batched Helmholtz solve: a system needs more shared memory than a CTA has";
         return OC_ERR_UNSUPPORTED;
     }
-    if (smem > 48 * 1024) {
-        static std::mutex mu;
-        static std::map<int, size_t> allowance;
-        std::lock_guard<std::mutex> lock(mu);
-        size_t& a = allowance[dev];
-        if (smem > a) {
-            cudaFuncSetAttribute(k_helm_solve_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            a = smem;
-        }
+    if (const cudaError_t e = allow_smem((const void*)k_helm_solve_batched, smem, dev); e != cudaSuccess) {
+        cudaGetLastError();
+        err = std::string("batched Helmholtz solve kernel's shared memory: ") + cudaGetErrorString(e);
+        return OC_ERR_CUDA;
     }
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_helm_solve_batched, 512, smem);

@@ -6,6 +6,9 @@ perfect tree in which grids of other sizes leave slots empty. Iteration counts a
 solutions are the oracle's bit for bit in every form.
 """
 
+import subprocess
+import sys
+from pathlib import Path
 from types import SimpleNamespace
 
 import numpy as np
@@ -123,3 +126,47 @@ def test_a_solve_in_place_gives_the_same_solution(kind, nx, ny):
     assert its.value == rep.iterations
     assert np.array_equal(a.cpu().numpy(), want)
     solver.close()
+
+
+# run in a process of its own: a solver built earlier may have raised the kernels'
+# shared-memory allowance for all that follow
+FRESH_SOLVE = """
+import sys
+from types import SimpleNamespace
+import numpy as np
+from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
+from oracle import ocean_oracle as orc
+from tests.test_gpu_helm_forms import _system
+nx, ny = int(sys.argv[1]), int(sys.argv[2])
+dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx + ny, walls=True)
+solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind="multigrid", rtol=1e-8,
+                      max_iter=4)
+x, rep = solver.solve(rhs)
+xr, itr, ok = orc.Helmholtz(nx, ny, 4.0e6, 5.0e6, coef, ku, kv, mask, "multigrid", 1e-8, 4).solve(rhs)
+assert rep.iterations == itr and rep.converged == ok
+assert np.array_equal(x, xr)
+"""
+
+FRESH_ENSEMBLE = """
+import sys
+from tests.test_gpu_ensemble import _member, _same
+from hydrostatic_ocean_core_benchmark_b200.stepper import OceanEnsemble
+sizes = [(int(sys.argv[1]), int(sys.argv[2]), 3, seed) for seed in (1, 2)]
+together, alone = [_member(*s) for s in sizes], [_member(*s) for s in sizes]
+OceanEnsemble(together).step(2)
+for a, b in zip(together, alone):
+    b.step(2)
+    _same(a, b, "ensemble member")
+"""
+
+
+@pytest.mark.parametrize("script,nx,ny", [
+    (FRESH_SOLVE, 104, 104), (FRESH_SOLVE, 52, 52), (FRESH_SOLVE, 26, 26), (FRESH_SOLVE, 80, 172),
+    (FRESH_SOLVE, 108, 128), (FRESH_ENSEMBLE, 104, 104),
+])
+def test_multigrid_near_the_default_shared_memory_limit(script, nx, ny):
+    """Solvers whose dynamic shared memory is under 48 KB and whose dynamic and static
+    shared memory together are not (46,480 to 48,896 bytes beside 2.8 KB)."""
+    r = subprocess.run([sys.executable, "-c", script, str(nx), str(ny)], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parents[1])
+    assert r.returncode == 0, r.stderr[-2000:]
