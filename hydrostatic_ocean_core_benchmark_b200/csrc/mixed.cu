@@ -95,8 +95,11 @@ void convert_params(const KP& a, KPT<float>& b) {
         b.thin[k] = (float)a.thin[k];
         b.dz_nom[k] = (float)a.dz_nom[k];
     }
+    b.face_rule = a.face_rule;
     for (int k = 0; k < a.nz; ++k) {
-        b.fdz[k] = (float)a.fdz[k];
+        // by the kernels' own FP32 operations: the harmonic mean of two equal thicknesses
+        // rounds differently in fp64
+        b.fdz[k] = face_combine(b, b.dzr[k], b.dzr[k]);
         b.rfdz[k] = b.fdz[k] > 0.0f ? 1.0f / b.fdz[k] : 0.0f;
         const float dzi = k > 0 ? 0.5f * (b.fdz[k - 1] + b.fdz[k]) : 0.0f;
         b.rfdzi[k] = dzi > 0.0f ? 1.0f / dzi : 0.0f;
@@ -104,7 +107,7 @@ void convert_params(const KP& a, KPT<float>& b) {
         b.dzi[k] = k > 0 ? 0.5f * (b.dzr[k - 1] + b.dzr[k]) : b.dzr[0];
         b.rdzi[k] = k > 0 ? 1.0f / b.dzi[k] : 0.0f;
     }
-    b.kinfo = a.kinfo, b.kface = a.kface, b.face_rule = a.face_rule;
+    b.kinfo = a.kinfo, b.kface = a.kface;
     b.mom_kl = a.mom_kl, b.tr_kl = a.tr_kl;
     b.dx64 = a.dx64, b.dy64 = a.dy64;
     b.rho0_64 = a.rho0_64, b.alpha_t64 = a.alpha_t64, b.beta_s64 = a.beta_s64;

@@ -232,9 +232,10 @@ __device__ __forceinline__ T col_above(const KPT<T>& P, int c, int k) {
     return above;
 }
 
-
+// face thickness between cells of thickness a and b; on the host too, so that a table of
+// thicknesses holds what the kernels form
 template <class T>
-__device__ __forceinline__ T face_combine(const KPT<T>& P, T a, T b) {
+__host__ __device__ __forceinline__ T face_combine(const KPT<T>& P, T a, T b) {
     if (P.face_rule == 0) return fmin(a, b);
     if (P.face_rule == 1) return T(0.5) * (a + b);
     T tot = a + b;

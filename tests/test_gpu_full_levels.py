@@ -77,3 +77,39 @@ def test_full_levels_match_oracle(bc_x, bc_y, advection, face_rule, mix, tracers
     assert st.solve_log() == ref.solve_log
     st.close()
     tuned.close()
+
+
+@pytest.mark.parametrize("face_rule", ["harmonic", "mean", "min"])
+def test_mixed_full_levels_do_not_depend_on_the_tiling(face_rule):
+    """A slab of levels starts with fluxes formed from the columns' own thicknesses, and
+    the levels below carry those of the level table: the FP32 step's bits are the same
+    wherever slabs start, in tiles of full, partial and mixed columns."""
+    from hydrostatic_ocean_core_benchmark_b200.stepper import OceanStepper
+    nx, ny = 100, 40
+    p = _case("closed", "periodic", "up3_tvd", face_rule, 50.0, "TS", "none", True)[0].replace(
+        nx=nx, ny=ny, lx=4.0e3 * nx, ly=3.5e3 * ny, nu=2.0e3, kappa=2.0e3)  # large explicit fluxes between levels
+    H, mask = np.full((ny, nx), 2000.0), np.ones((ny, nx))
+    H[14:18, 45:60] = 700.0
+    rng = np.random.default_rng(2)
+    shape = (NZ, ny, nx)
+    u, v = 0.2 * rng.standard_normal(shape), 0.2 * rng.standard_normal(shape)
+    T, S = 10.0 + rng.standard_normal(shape), 35.0 + 0.1 * rng.standard_normal(shape)
+    eta = 0.1 * rng.standard_normal((ny, nx))
+    dzr = 60.0 + 200.0 * np.random.default_rng(3).random(NZ)
+    dzr *= 2000.0 / dzr.sum()
+    d = dzr.astype(np.float32)
+    if face_rule == "harmonic":  # levels where the fp64 mean rounded to FP32 is another number
+        assert np.any((2.0 * dzr * dzr / (dzr + dzr)).astype(np.float32) != np.float32(2.0) * d * d / (d + d))
+    fields = []
+    for levels in (None, (1, 1), (3, 4), (4, 3), (NZ, NZ)):
+        st = OceanStepper(p, H, mask, dzr=dzr, precision="mixed")
+        if levels:
+            st.set_tiling(*levels)
+        st.set_state(eta=eta, u=u, v=v, T=T, S=S)
+        st.step(3)
+        fields.append(st.get_state())
+        st.close()
+    for f in ("eta", "u", "v", "b", "T", "S"):
+        assert np.all(np.isfinite(fields[0][f]))
+        for other in fields[1:]:
+            assert np.array_equal(fields[0][f], other[f]), f"{f} depends on the levels per CTA"
