@@ -128,6 +128,33 @@ def test_a_solve_in_place_gives_the_same_solution(kind, nx, ny):
     solver.close()
 
 
+@pytest.mark.parametrize("nx,ny", [(40, 30), (120, 130), (400, 390), (1000, 720), (5000, 300)])
+def test_pcg_jacobi_warm_start(nx, ny):
+    """The mixed-precision step's solves start from the elevation they are given, in every
+    form: one step's elevation against that of PCG-RBGS (the general kernel). Both stop at
+    |r| <= rtol |b| and A - 1 is positive, so they are within 2 rtol |b| <= 2 rtol |A| |x|."""
+    from hydrostatic_ocean_core_benchmark_b200 import cases
+    from hydrostatic_ocean_core_benchmark_b200.stepper import OceanStepper
+    rtol, got = 1e-9, {}
+    y, x = np.mgrid[0:ny, 0:nx]
+    eta = 0.3 * np.sin(3.0 * x / nx) * np.cos(5.0 * y / ny)
+    for kind in ("pcg_jacobi", "pcg_rbgs"):
+        s = cases.seamount_basin(nx=nx, ny=ny, nz=2, seed=4, dt=120.0, solver_kind=kind, rtol=rtol, n_picard=1,
+                                 closure="none")
+        p = s.params
+        st = OceanStepper(p, s.H, s.mask, dzr=s.dzr, taux_c=s.taux_c, tauy_c=s.tauy_c, precision="mixed")
+        st.set_state(eta=eta, u=s.u, v=s.v, T=s.T, S=s.S)
+        st.step(1)
+        got[kind] = st.get_state()["eta"]
+        assert st.stats()["solver_failures"] == 0
+        st.close()
+    norm_A = 1.0 + 4.0 * p.g * (p.theta * p.dt) ** 2 * float(s.H.max()) * (1.0 / p.dx ** 2 + 1.0 / p.dy ** 2)
+    err = np.linalg.norm(got["pcg_jacobi"] - got["pcg_rbgs"])
+    assert err <= 2.0 * rtol * norm_A * np.linalg.norm(got["pcg_rbgs"])
+    # and the step moved the elevation by much more than that
+    assert np.linalg.norm(got["pcg_rbgs"] - eta) > 1e3 * err
+
+
 # run in a process of its own: a solver built earlier may have raised the kernels'
 # shared-memory allowance for all that follow
 FRESH_SOLVE = """
@@ -163,7 +190,7 @@ for a, b in zip(together, alone):
 @pytest.mark.parametrize("script,nx,ny", [
     (FRESH_SOLVE, 104, 104), (FRESH_SOLVE, 52, 52), (FRESH_SOLVE, 26, 26), (FRESH_SOLVE, 80, 172),
     (FRESH_SOLVE, 108, 128), (FRESH_ENSEMBLE, 104, 104),
-])
+], ids=lambda a: {FRESH_SOLVE: "solve", FRESH_ENSEMBLE: "ensemble"}.get(a, a))
 def test_multigrid_near_the_default_shared_memory_limit(script, nx, ny):
     """Solvers whose dynamic shared memory is under 48 KB and whose dynamic and static
     shared memory together are not (46,480 to 48,896 bytes beside 2.8 KB)."""
