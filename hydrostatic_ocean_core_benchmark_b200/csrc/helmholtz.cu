@@ -131,7 +131,7 @@ __device__ void leaf_phase(const HelmParams& H, F f, double* outA, double* outB)
     const int nwarps = s_grid.ncta * (blockDim.x >> 5);
     const int my = (threadIdx.x >> 5) * s_grid.ncta + s_grid.cta;  // leaf L runs on CTA L mod grid
     for (int L = my; L < H.n_leaves; L += nwarps) {
-        const int s = H.leaf_start[L];
+        const int s = H.leaf_start[L], slot = H.leaf_slot[L];
         const int len = H.leaf_start[L + 1] - s;
         double va[4], vb[4];
 #pragma unroll
@@ -145,7 +145,6 @@ __device__ void leaf_phase(const HelmParams& H, F f, double* outA, double* outB)
         const double a = leaf_sum_warp(va, len);
         const double bsum = outB ? leaf_sum_warp(vb, len) : 0.0;
         if (lane == 0) {
-            const int slot = H.leaf_slot[L];
             outA[slot] = a;
             if (outB) outB[slot] = bsum;
         }
@@ -324,7 +323,7 @@ __device__ __noinline__ void residual_leaves(const double* x) {
     if (rank >= n) return;
     const int lane = threadIdx.x & 31;
     for (int L = (threadIdx.x >> 5) * n + rank; L < H.n_leaves; L += n * warps) {
-        const int s = H.leaf_start[L], len = H.leaf_start[L + 1] - s;
+        const int s = H.leaf_start[L], len = H.leaf_start[L + 1] - s, slot = H.leaf_slot[L];
         double v[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -336,7 +335,7 @@ __device__ __noinline__ void residual_leaves(const double* x) {
             }
         }
         const double a = leaf_sum_warp(v, len);
-        if (lane == 0) H.leafA[H.leaf_slot[L]] = a;
+        if (lane == 0) H.leafA[slot] = a;
     }
 }
 
@@ -353,18 +352,22 @@ __device__ __forceinline__ void solve_log(const HelmParams& H, bool ok, int iter
     *H.log_count = idx + 1;
 }
 
+// MG: with the V-cycle; without it the multigrid kinds are not reached.
+template <bool MG>
 __device__ __forceinline__ void helm_solve_body() {
     const HelmParams& H = s_helm;
-    if (H.one_cta) {
-        int its, cv;
-        helm_one_cta(its, cv);
-        solve_log(H, true, its, cv);
-        return;
+    if constexpr (MG) {
+        if (H.one_cta) {
+            int its, cv;
+            helm_one_cta(its, cv);
+            solve_log(H, true, its, cv);
+            return;
+        }
     }
     // with H.persist0 the first 4 SN doubles (6 with its x and b) hold level 0's tile for the
     // whole solve; every other use of shared memory works above them
-    const int persist = H.persist0 ? 0 : -1;
-    const int smo = H.persist0 ? (H.keep_x0 ? 6 : 4) * TileWide::SN : 0;
+    const int persist = MG && H.persist0 ? 0 : -1;
+    const int smo = MG && H.persist0 ? (H.keep_x0 ? 6 : 4) * TileWide::SN : 0;
     double* sm = smem_all + smo;
     const HLevel& L0 = H.lv[0];
     const double* rhs = H.rhs;
@@ -388,17 +391,21 @@ __device__ __forceinline__ void helm_solve_body() {
                H.leafA, nullptr);
     ok = grid_sync(H);
     const double norm_b = ok ? sqrt(fold_sum(H, H.leafA, sm, ok)) : 0.0;
-    if (persist >= 0) persist_level0(smo, persist);  // the coefficients are fixed during the solve
-    if (s_grid.cta == 0 && H.coarse_from < H.n_levels) coarse_tab_init(smo, coarse_coef_at(H, smo, persist));
-    if (s_grid.cta == 0 && H.coarse_from < H.n_levels && s_coarse_held) {
-        coarse_coef_load();
-        cpa_wait_all();
-        __syncthreads();
+    if constexpr (MG) {
+        if (persist >= 0) persist_level0(smo, persist);  // the coefficients are fixed during the solve
+        if (s_grid.cta == 0 && H.coarse_from < H.n_levels) {
+            coarse_tab_init(smo, coarse_coef_at(H, smo, persist));
+            if (s_coarse_held) {
+                coarse_coef_load();
+                cpa_wait_all();
+                __syncthreads();
+            }
+        }
     }
     if (!ok || norm_b == 0.0) goto done;
     {
         const double tol = H.rtol * norm_b;
-        if (H.kind == HK_RBGS || H.kind == HK_MULTIGRID) {
+        if (H.kind == HK_RBGS || (MG && H.kind == HK_MULTIGRID)) {
             // stationary iteration with the true residual (solvers_var.py:170-179)
             conv = 0;
             double* xc = x;  // the level-0 buffer holding the current iterate
@@ -406,20 +413,22 @@ __device__ __forceinline__ void helm_solve_body() {
             // beside the next cycle's first phase, on the CTAs that have no tile in it if
             // they are enough: a grid barrier and a pass of their own less per cycle, for
             // one phase that the last cycle runs in vain.
-            const bool piped = H.kind == HK_MULTIGRID && !H.fused_res && H.coarse_from > 0 && H.n_levels > 1;
+            const bool piped = MG && H.kind == HK_MULTIGRID && !H.fused_res && H.coarse_from > 0 && H.n_levels > 1;
             for (int it = 1; it <= H.max_iter && ok; ++it) {
-                if (H.kind == HK_MULTIGRID) {
-                    // the previous iterate's residual and its test, beside this cycle's first phase
-                    const double* xp = xc;
-                    xc = vcycle_tiled(H, xc, xc == H.lv[0].x ? H.lv[0].x2 : H.lv[0].x, smo, persist, ok,
-                                      [&]() { if (piped && it > 1) residual_leaves(xp); },
-                                      [&]() {
-                                          if (!piped || it == 1) return false;
-                                          iters = it - 1;
-                                          conv = sqrt(fold_sum(H, H.leafA, sm, ok)) <= tol ? 1 : 0;
-                                          return conv != 0 || !ok;
-                                      });
-                    if (conv) break;
+                if (MG && H.kind == HK_MULTIGRID) {
+                    if constexpr (MG) {
+                        // the previous iterate's residual and its test, beside this cycle's first phase
+                        const double* xp = xc;
+                        xc = vcycle_tiled(H, xc, xc == H.lv[0].x ? H.lv[0].x2 : H.lv[0].x, smo, persist, ok,
+                                          [&]() { if (piped && it > 1) residual_leaves(xp); },
+                                          [&]() {
+                                              if (!piped || it == 1) return false;
+                                              iters = it - 1;
+                                              conv = sqrt(fold_sum(H, H.leafA, sm, ok)) <= tol ? 1 : 0;
+                                              return conv != 0 || !ok;
+                                          });
+                        if (conv) break;
+                    }
                 } else {
                     colour_phase(L0, x, b0, 0, grid_team());
                     ok = grid_sync(H);
@@ -431,7 +440,7 @@ __device__ __forceinline__ void helm_solve_body() {
                 if (piped && it < H.max_iter) continue;
                 // the true residual's leaf sums: formed by the last up phase when
                 // level 0's tiles are NumPy's leaves, else by a pass of their own
-                if (!(H.kind == HK_MULTIGRID && H.fused_res)) {
+                if (!(MG && H.kind == HK_MULTIGRID && H.fused_res)) {
                     const double* xr = xc;
                     leaf_phase(H,
                                [&](int e) {
@@ -469,20 +478,22 @@ __device__ __forceinline__ void helm_solve_body() {
             // z = M^-1 r
             auto precondition = [&](bool& okp) {
                 if (jac) return;
-                if (H.kind == HK_PCG_MG) {
-                    // one V(2,2) cycle on level 0's rhs r from a zero iterate (symmetric:
-                    // red-black pre-smoothing, black-red post-smoothing)
-                    for (int e = grid_team().first; e < L0.n; e += grid_team().stride) {
-                        b0[e] = __ldcg(r + e);
-                        z[e] = 0.0;
+                if constexpr (MG) {
+                    if (H.kind == HK_PCG_MG) {
+                        // one V(2,2) cycle on level 0's rhs r from a zero iterate (symmetric:
+                        // red-black pre-smoothing, black-red post-smoothing)
+                        for (int e = grid_team().first; e < L0.n; e += grid_team().stride) {
+                            b0[e] = __ldcg(r + e);
+                            z[e] = 0.0;
+                        }
+                        okp = grid_sync(H);
+                        if (!okp) return;
+                        double* zr = vcycle_tiled(H, z, L0.x2, smo, persist, okp, []() {}, []() { return false; });
+                        if (!okp || zr == z) return;
+                        for (int e = grid_team().first; e < L0.n; e += grid_team().stride) z[e] = __ldcg(zr + e);
+                        okp = grid_sync(H);
+                        return;
                     }
-                    okp = grid_sync(H);
-                    if (!okp) return;
-                    double* zr = vcycle_tiled(H, z, L0.x2, smo, persist, okp, []() {}, []() { return false; });
-                    if (!okp || zr == z) return;
-                    for (int e = grid_team().first; e < L0.n; e += grid_team().stride) z[e] = __ldcg(zr + e);
-                    okp = grid_sync(H);
-                    return;
                 }
                 for (int e = grid_team().first; e < L0.n; e += grid_team().stride) z[e] = 0.0;
                 okp = grid_sync(H);
@@ -577,20 +588,30 @@ done:
 // The parameters are read through a reference throughout the solve: a copy in
 // shared memory, made once per CTA (a reference to the kernel parameter itself
 // would give every thread a copy of its own in local memory).
-__global__ void __launch_bounds__(512) k_helm_solve(HelmParams H) {
+// One kernel for the multigrid kinds and one for the others, which in one kernel with the
+// V-cycle spill (128 registers and 328 bytes of stack; 110 and none apart). us a solve
+// together and apart: PCG-RBGS 48 x 48 294 and 279, 1000 x 720 1019 and 979; RBGS 128 x 96
+// 237 and 229; four steps of eight PCG-Jacobi members, batched, 34.3 and 32.4
+// ms. Without the bound of one CTA per SM the compiler gives the second one 64
+// registers and spills, and two CTAs per SM wait for one another: PCG-RBGS 128 x 96 321
+// against 297.
+template <bool MG>
+__global__ void __launch_bounds__(512, MG ? 0 : 1) k_helm_solve(HelmParams H) {
     if (threadIdx.x == 0) s_grid = SolveGrid{(int)blockIdx.x, (int)gridDim.x};
     const int* src = reinterpret_cast<const int*>(&H);
     int* dst = reinterpret_cast<int*>(&s_helm);
     for (int t = threadIdx.x; t < (int)(sizeof(HelmParams) / sizeof(int)); t += blockDim.x) dst[t] = src[t];
     __syncthreads();
-    helm_solve_body();
+    helm_solve_body<MG>();
 }
 
 // Several systems in one cooperative launch: system m runs on CTAs
 // [cta_start[m], cta_start[m + 1]) with its own parameters (copied into shared
 // memory), its own barrier counter, status word and solve log; the systems
 // never wait on one another.
-__global__ void __launch_bounds__(512) k_helm_solve_batched(const HelmParams* __restrict__ systems,
+// MG: at least one of them is of a multigrid kind.
+template <bool MG>
+__global__ void __launch_bounds__(512, MG ? 0 : 1) k_helm_solve_batched(const HelmParams* __restrict__ systems,
                                                             const int* __restrict__ cta_start, int n) {
     __shared__ int s_m;
     if (threadIdx.x == 0) {
@@ -604,7 +625,7 @@ __global__ void __launch_bounds__(512) k_helm_solve_batched(const HelmParams* __
     int* dst = reinterpret_cast<int*>(&s_helm);
     for (int t = threadIdx.x; t < (int)(sizeof(HelmParams) / sizeof(int)); t += blockDim.x) dst[t] = src[t];
     __syncthreads();
-    helm_solve_body();
+    helm_solve_body<MG>();
 }
 
 // ------------------------------------------------------------------ level rebuild
@@ -1017,8 +1038,9 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     };
     int smem_optin = 0;
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    kernel_ = mg_levels ? k_helm_solve<true> : k_helm_solve<false>;
     cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, k_helm_solve);  // static shared memory (the barrier's word) comes first
+    cudaFuncGetAttributes(&fa, kernel_);  // static shared memory (the barrier's word) comes first
     // level 0 keeps what fits: everything, its coefficients, or nothing
     auto fits = [&](int kept) { return solve_smem(kept) + fa.sharedSizeBytes <= (size_t)smem_optin; };
     if (H.keep_x0 && !fits(6)) H.keep_x0 = 0;
@@ -1028,13 +1050,13 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
         err = "Helmholtz grid too large for the single-pass reduction tree";
         return OC_ERR_UNSUPPORTED;
     }
-    if (const cudaError_t e = allow_smem((const void*)k_helm_solve, smem_, dev); e != cudaSuccess) {
+    if (const cudaError_t e = allow_smem((const void*)kernel_, smem_, dev); e != cudaSuccess) {
         cudaGetLastError();
         err = std::string("Helmholtz solve kernel's shared memory: ") + cudaGetErrorString(e);
         return OC_ERR_CUDA;
     }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_helm_solve, block_, smem_);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_, block_, smem_);
     if (per_sm < 1) {
         err = "Helmholtz solve kernel cannot be resident";
         return OC_ERR_CUDA;
@@ -1115,6 +1137,7 @@ int helm_batch_plan(HelmSolver* const* solvers, const double* const* rhs, double
     }
     size_t smem = 0;
     double total = 0.0;
+    bool mg = false;
     std::vector<HelmParams> hp(n);
     for (int m = 0; m < n; ++m) {
         if (!solvers[m]->batchable()) {
@@ -1122,6 +1145,7 @@ int helm_batch_plan(HelmSolver* const* solvers, const double* const* rhs, double
             return OC_ERR_UNSUPPORTED;
         }
         hp[m] = solvers[m]->batched_params(rhs[m], x[m]);
+        mg = mg || hp[m].kind == HK_MULTIGRID || hp[m].kind == HK_PCG_MG;
         smem = std::max(smem, solvers[m]->batched_smem());
         total += solvers[m]->work_weight();
     }
@@ -1130,18 +1154,19 @@ int helm_batch_plan(HelmSolver* const* solvers, const double* const* rhs, double
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, k_helm_solve_batched);
+    const auto kernel = mg ? k_helm_solve_batched<true> : k_helm_solve_batched<false>;
+    cudaFuncGetAttributes(&fa, kernel);
     if (smem + fa.sharedSizeBytes > (size_t)smem_optin) {
         err = "batched Helmholtz solve: a system needs more shared memory than a CTA has";
         return OC_ERR_UNSUPPORTED;
     }
-    if (const cudaError_t e = allow_smem((const void*)k_helm_solve_batched, smem, dev); e != cudaSuccess) {
+    if (const cudaError_t e = allow_smem((const void*)kernel, smem, dev); e != cudaSuccess) {
         cudaGetLastError();
         err = std::string("batched Helmholtz solve kernel's shared memory: ") + cudaGetErrorString(e);
         return OC_ERR_CUDA;
     }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_helm_solve_batched, 512, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 512, smem);
     if (per_sm < 1) {
         err = "batched Helmholtz solve kernel cannot be resident";
         return OC_ERR_CUDA;
@@ -1183,6 +1208,7 @@ int helm_batch_plan(HelmSolver* const* solvers, const double* const* rhs, double
     b.n = n;
     b.grid = b.cta_start[n];
     b.smem = smem;
+    b.mg = mg;
     return OC_OK;
 }
 
@@ -1204,8 +1230,8 @@ int helm_batch_launch(const HelmBatch& b, cudaStream_t s, std::string& err) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_helm_solve_batched, (const HelmParams*)b.d_params,
-                                             (const int*)b.d_cta_start, b.n);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, b.mg ? k_helm_solve_batched<true> : k_helm_solve_batched<false>,
+                                             (const HelmParams*)b.d_params, (const int*)b.d_cta_start, b.n);
     if (e != cudaSuccess) {
         err = std::string("batched Helmholtz solve launch: ") + cudaGetErrorString(e);
         return OC_ERR_CUDA;
@@ -1283,7 +1309,7 @@ int HelmSolver::solve(const double* rhs, double* x, cudaStream_t s, std::string&
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_helm_solve, H);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel_, H);
     if (e != cudaSuccess) {
         err = std::string("Helmholtz solve launch: ") + cudaGetErrorString(e);
         return OC_ERR_CUDA;

@@ -125,6 +125,7 @@ class HelmSolver {
     bool pcg_ = false;  // the on-chip PCG-Jacobi kernel takes the solves
     PcgPlan pcg_plan_{};
     std::vector<void*> allocs_;
+    void (*kernel_)(HelmParams) = nullptr;  // the solve kernel of this kind
     int grid_ = 0, block_ = 512;
     size_t smem_ = 0, smem_batched_ = 0;
     size_t bytes_ = 0;
@@ -137,6 +138,7 @@ class HelmSolver {
 struct HelmBatch {
     int n = 0, grid = 0;
     size_t smem = 0;
+    bool mg = false;  // a system of a multigrid kind among them
     HelmParams* d_params = nullptr;
     int* d_cta_start = nullptr;
     std::vector<int> cta_start;
