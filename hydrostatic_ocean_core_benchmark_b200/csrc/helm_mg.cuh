@@ -10,7 +10,7 @@
 // the whole-grid sweep produces (same inputs, same operations), so the result is
 // that of sweeping the level with a grid barrier between half-sweeps, with two
 // barriers per level instead of nine. Levels of at most kCoarseCells cells run
-// inside CTA 0; grids of at most kOneCtaCells cells run wholly in one CTA.
+// inside CTA 0; a stationary solve of at most kOneCtaCells cells runs wholly in one CTA.
 //
 // A half-sweep is bound by shared-memory bandwidth (ten reads and a write per
 // updated cell), so the two colours of every array are stored apart: cell (i, j) of
