@@ -45,38 +45,41 @@ int helm_fail(oc_helm* h, int code, const std::string& msg) {
 
 // rho' for linear and S-EOS (eos.py:103-127), full in-situ rho for polyTEOS10-bsq
 // (eos.py:68-100): what the reference's EOS bench evaluates per cell. A thread takes
-// kCells cells at a time, a block's width apart: their loads are all in flight before
+// CELLS cells at a time, a block's width apart: their loads are all in flight before
 // the first polynomial, and a coefficient fetched for one cell serves the others. Bound
 // by fp64 issue (the polynomial is about 110 operations a cell): polyTEOS10 at 2e7 cells
-// takes 208 us with one cell at a time and the kind tested inside, 189 with four.
-constexpr int kCells = 4;
-
+// takes 208 us with one cell at a time and the kind tested inside, 189 with four. Where
+// one cell per thread is at most two rounds of CTAs a call is bound by its latency instead, and
+// a thread with four cells has four times the instructions to fetch and issue: a call of
+// polyTEOS10 on 1,000 cells takes 14.2 us until its result with four, 11.8 with one, on
+// 150,000 13.5 and 12.9 (among others 6.0 and 4.2, 4.5 and 4.2); on 320,000 7.2 and 6.2 among
+// others, on 600,000 8.2 both.
 template <int EOS>
 __device__ __forceinline__ double density_of(double rho0, double alpha_t, double beta_s, double t0, double s0, double T,
                                              double S, double z) {
     return EOS == OC_EOS_TEOS10 ? oc::rho_teos10(T, S, z) : oc::rho_anomaly_of(EOS, rho0, alpha_t, beta_s, t0, s0, T, S, z);
 }
 
-template <int EOS>
+template <int EOS, int CELLS>
 __global__ void __launch_bounds__(256) k_density(double rho0, double alpha_t, double beta_s, double t0, double s0,
                                                  const double* __restrict__ T, const double* __restrict__ S,
                                                  const double* __restrict__ z, double* __restrict__ rho, int64_t n) {
-    const int64_t tile = (int64_t)blockDim.x * kCells;
+    const int64_t tile = (int64_t)blockDim.x * CELLS;
     for (int64_t base = blockIdx.x * tile + threadIdx.x; base < n; base += gridDim.x * tile) {
-        double Tv[kCells], Sv[kCells], zv[kCells];
-        if (base + (int64_t)(kCells - 1) * blockDim.x < n) {
+        double Tv[CELLS], Sv[CELLS], zv[CELLS];
+        if (base + (int64_t)(CELLS - 1) * blockDim.x < n) {
 #pragma unroll
-            for (int q = 0; q < kCells; ++q) {
+            for (int q = 0; q < CELLS; ++q) {
                 const int64_t t = base + (int64_t)q * blockDim.x;
                 Tv[q] = T[t];
                 Sv[q] = S[t];
                 zv[q] = z[t];
             }
 #pragma unroll
-            for (int q = 0; q < kCells; ++q)
+            for (int q = 0; q < CELLS; ++q)
                 rho[base + (int64_t)q * blockDim.x] = density_of<EOS>(rho0, alpha_t, beta_s, t0, s0, Tv[q], Sv[q], zv[q]);
         } else {
-            for (int q = 0; q < kCells; ++q) {
+            for (int q = 0; q < CELLS; ++q) {
                 const int64_t t = base + (int64_t)q * blockDim.x;
                 if (t < n) rho[t] = density_of<EOS>(rho0, alpha_t, beta_s, t0, s0, T[t], S[t], z[t]);
             }
@@ -86,14 +89,19 @@ __global__ void __launch_bounds__(256) k_density(double rho0, double alpha_t, do
 
 template <int EOS>
 void density_launch(double rho0, double alpha_t, double beta_s, double t0, double s0, const double* T, const double* S,
-                    const double* z, double* rho, int64_t count, int sms, cudaStream_t stream) {
-    const int block = 256;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_density<EOS>, block, 0);
-    const int64_t need = (count + (int64_t)block * kCells - 1) / ((int64_t)block * kCells);
-    const int64_t cap = (int64_t)(sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1) * 4;
-    k_density<EOS><<<(unsigned)(need < cap ? need : cap), block, 0, stream>>>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho,
-                                                                            count);
+                    const double* z, double* rho, int64_t count, cudaStream_t stream) {
+    // CTAs that a B200's 148 SMs hold at once: eight an SM (five of polyTEOS10 with four cells). A
+    // constant, as a query costs a small call more than it gives; on a part of a GPU the CTAs
+    // only come in more rounds.
+    constexpr int64_t block = 256, round = 148 * 8, cap = 4 * 148 * (EOS == OC_EOS_TEOS10 ? 5 : 8);
+    if (count <= 2 * round * block) {
+        k_density<EOS, 1><<<(unsigned)((count + block - 1) / block), block, 0, stream>>>(rho0, alpha_t, beta_s, t0, s0, T, S,
+                                                                                    z, rho, count);
+        return;
+    }
+    const int64_t need = (count + block * 4 - 1) / (block * 4);
+    k_density<EOS, 4><<<(unsigned)(need < cap ? need : cap), block, 0, stream>>>(rho0, alpha_t, beta_s, t0, s0, T,
+                                                                                        S, z, rho, count);
 }
 
 }  // namespace
@@ -217,12 +225,9 @@ extern "C" int oc_density(int32_t eos, double rho0, double alpha_t, double beta_
                           void* stream) {
     if (!T || !S || !z || !rho || count < 0 || eos < OC_EOS_LINEAR || eos > OC_EOS_TEOS10) return OC_ERR_ARG;
     if (count == 0) return OC_OK;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const cudaStream_t st = (cudaStream_t)stream;
-    if (eos == OC_EOS_LINEAR) density_launch<OC_EOS_LINEAR>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, sms, st);
-    else if (eos == OC_EOS_SEOS) density_launch<OC_EOS_SEOS>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, sms, st);
-    else density_launch<OC_EOS_TEOS10>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, sms, st);
+    if (eos == OC_EOS_LINEAR) density_launch<OC_EOS_LINEAR>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, st);
+    else if (eos == OC_EOS_SEOS) density_launch<OC_EOS_SEOS>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, st);
+    else density_launch<OC_EOS_TEOS10>(rho0, alpha_t, beta_s, t0, s0, T, S, z, rho, count, st);
     return cudaGetLastError() == cudaSuccess ? OC_OK : OC_ERR_CUDA;
 }

@@ -41,7 +41,8 @@ def test_column_forms_match_oracle(nx, ny, nz, mxl):
     st.close()
 
 
-@pytest.mark.parametrize("n", [1, 255, 257, 769, 1023, 1024, 1025, 700001])
+# one cell a thread up to 2 x 148 x 8 x 256 cells, four above; the last leaves each remainder of four blocks' widths
+@pytest.mark.parametrize("n", [1, 255, 257, 769, 1023, 1024, 1025, 606208, 606209, 606977, 700001])
 @pytest.mark.parametrize("kind", ["linear", "seos", "teos10"])
 def test_density_matches_oracle(kind, n):
     import torch
