@@ -1348,7 +1348,9 @@ __global__ void __launch_bounds__(256) k_predictor_rhs(
 // right-hand sides arrive in gh_u/gh_v; the forward elimination overwrites them
 // with its intermediate values, the back substitution with the solution, and
 // the transports are summed in a last, downward pass to keep the reference's
-// order. Only the elimination coefficients stay in the thread.
+// order. Only the elimination coefficients stay in the thread. The rows are divided out
+// here: with the level table's reciprocals 512 x 512 x 50 takes 254 us a launch instead of
+// 250 (FP32 175 and 167), 256 x 256 x 128 281 instead of 275 (FP32 218 and 206).
 template <int NZM>
 __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __restrict__ km,
                                                         real* __restrict__ ghu,
@@ -1360,7 +1362,8 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
     const int c = nb.c;
     const ColGeoR g = ColGeoR::load(P, c);
     real cs[NZM];
-    real rdzi_k = g.rdz(P, 0);
+    real m3_k, dz_k = g.dz(P, 0, m3_k);
+    real dzi_k = dz_k;
     real km_k = km[c];
     real du = real(0.0), dv = real(0.0), cp = real(0.0);
 #pragma unroll 4
@@ -1368,10 +1371,11 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
         const size_t o = (size_t)k * n2 + c;
         const real km_k1 = km[o + n2];
         const real ru = ghu[o], rv = ghv[o];
-        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
-        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
+        real m3_k1 = real(0.0), dz_k1 = real(0.0);
+        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
+        const real dzi_k1 = (k + 1 < nz) ? real(0.5) * (dz_k + dz_k1) : dz_k;
         real sub, diag, sup;
-        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
+        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, km_k, km_k1, P.thv_dt_drag, sub, diag, sup);
         if (k == 0) {
             cp = sup / diag;
             du = ru / diag;
@@ -1386,7 +1390,9 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
         ghu[o] = du;
         ghv[o] = dv;
         km_k = km_k1;
-        rdzi_k = rdzi_k1;
+        dz_k = dz_k1;
+        m3_k = m3_k1;
+        dzi_k = dzi_k1;
     }
     real xu = du, xv = dv;
     {
@@ -1898,7 +1904,9 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P,
 // (model3d_v05.py:514-533). The forward elimination stores its right-hand sides
 // in the outputs; the back substitution finishes each level there, EOS
 // included, with the level-centre depth in closed form (col_above is the
-// sequential sum of the thicknesses above, bit for bit).
+// sequential sum of the thicknesses above, bit for bit). The rows are divided out here, as in
+// k_momentum_solve: with the level table's reciprocals 256 x 256 x 128 takes 312 us instead of
+// 305 (FP32 267 and 256), 512 x 512 x 50 311 and 312 (FP32 239 and 233).
 template <int NZM>
 __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restrict__ rT,
                                                       const real* __restrict__ rS,
@@ -1918,19 +1926,21 @@ __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restr
 #else
     real* __restrict__ o1 = ts ? T_out : b_out;
 #endif
-    real rdzi_k = g.rdz(P, 0);
+    real m3_k, dz_k = g.dz(P, 0, m3_k);
+    real dzi_k = dz_k;
     real kh_k = kh[c];
     real d1 = real(0.0), d2 = real(0.0), cp = real(0.0);
 #pragma unroll 4
     for (int k = 0; k < nz; ++k) {
         const size_t o = (size_t)k * n2 + c;
         const real kh_k1 = kh[o + n2];
-        const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
-        const real rdzi_k1 = (k + 1 < nz) ? g.rdzi(P, k + 1) : real(0.0);
+        real m3_k1 = real(0.0), dz_k1 = real(0.0);
+        if (k + 1 < nz) dz_k1 = g.dz(P, k + 1, m3_k1);
+        const real dzi_k1 = (k + 1 < nz) ? real(0.5) * (dz_k + dz_k1) : dz_k;
         const real r1 = rT[o];
         const real r2 = ts ? rS[o] : real(0.0);
         real sub, diag, sup;
-        implicit_row_inv(P, k, g.rdz(P, k), m3_k, m3_k1, rdzi_k, rdzi_k1, kh_k, kh_k1, P.thv_dt_zero, sub, diag, sup);
+        implicit_row(P, k, dz_k, m3_k, m3_k1, dzi_k, dzi_k1, kh_k, kh_k1, P.thv_dt_zero, sub, diag, sup);
         if (k == 0) {
             cp = sup / diag;
             d1 = r1 / diag;
@@ -1947,7 +1957,9 @@ __global__ void __launch_bounds__(128) k_tracer_solve(KPR P, const real* __restr
             if (ts) S_out[o] = d2;
         }
         kh_k = kh_k1;
-        rdzi_k = rdzi_k1;
+        dz_k = dz_k1;
+        m3_k = m3_k1;
+        dzi_k = dzi_k1;
     }
     real x1 = d1, x2 = d2;
 #pragma unroll 4
