@@ -1114,7 +1114,7 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
     int rc = adjoint_setup(h);
     if (rc) return rc;
     AdjointWork& A = *h->adj;
-    const KP& P = h->P;
+    const KL& P = h->P;
     const size_t n2 = h->n2, n3 = h->n3, n3i = h->n3i;
     const dim3 cb = col_block(), cg = col_grid(P);
     const dim3 vb(32, 4, 1), vg((P.nx + 31) / 32, (P.ny + 3) / 4, P.nz);
@@ -1183,7 +1183,7 @@ int adjoint_step(oc_handle* h, const oc_state_view* x0, const oc_state_view* x1,
 int adjoint_eos(oc_handle* h, const double* T, const double* S, const double* b_b, double* T_b, double* S_b,
                 cudaStream_t s) {
     if (!T || !S || !b_b || !T_b || !S_b) return fail(h, OC_ERR_ARG, "T, S, b_b, T_b and S_b are required");
-    const KP& P = h->P;
+    const KL& P = h->P;
     k_eos_T<<<col_grid(P), col_block(), 0, s>>>(P, T, S, b_b, T_b, S_b);
     return check_launch(h, "oc_adjoint_eos");
 }

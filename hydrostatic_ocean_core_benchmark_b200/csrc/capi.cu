@@ -120,7 +120,7 @@ int validate(const oc_config* c, std::string& err) {
 // scalar constants of the step, formed in the reference's operation order
 void fill_scalars(oc_handle* h) {
     const oc_config& c = h->cfg;
-    KP& P = h->P;
+    KL& P = h->P;
     P.nx = c.nx;
     P.ny = c.ny;
     P.nz = c.nz;
@@ -203,7 +203,7 @@ double face_host(int rule, double a, double b) {
 void build_host_geometry(oc_handle* h) {
     const int nx = h->nx, ny = h->ny, nz = h->nz;
     const size_t n2 = h->n2, n3 = h->n3;
-    const KP& P = h->P;
+    const KL& P = h->P;
     h->dz3.assign(n3, 0.0);
     h->mask3.assign(n3, 0.0);
     for (int k = 0; k < nz; ++k)
@@ -324,7 +324,7 @@ int prof_class(oc_handle* h, const char* name) {
 int step_once(oc_handle* h, cudaStream_t s) {
     if (h->mixed) return step_once_mixed(h, s);
     const oc_config& c = h->cfg;
-    const KP& P = h->P;
+    const KL& P = h->P;
     const int cur = h->cur, nxt = 1 - cur;
     double *u = h->U[cur], *v = h->V[cur], *b = h->B[cur], *eta = h->ETA[cur];
     double *un = h->U[nxt], *vn = h->V[nxt], *etan = h->ETA[nxt];
@@ -644,7 +644,7 @@ static int set_domain_impl(oc_handle* h, const double* Hh, const double* maskh, 
             h->dzr[k] = dzrh[k];
         }
     }
-    KP& P = h->P;
+    KL& P = h->P;
     P.edge[0] = 0.0;
     for (int k = 0; k < nz; ++k) {
         P.edge[k + 1] = (k == 0) ? h->dzr[0] : P.edge[k] + h->dzr[k];
@@ -963,32 +963,32 @@ int oc_autotune(oc_handle* h, int32_t* mom_levels, int32_t* tracer_levels) {
     int mk, tk;
     if (h->mixed) {
         // the FP32 kernels of the mixed path on its FP32 fields (TS tracers)
-        const KPT<float>& P = h->P32;
+        const KLT<float>& P = h->P32;
         launch_phi(P, h->B[c], h->phi, s);  // the explicit momentum terms read phi
         mk = best_of(P.mom_kl, [&](int kl) {
-            KPT<float> Q = P;
+            KLT<float> Q = P;
             Q.mom_kl = kl;
             launch_mom_explicit(Q, h->U32[c], h->V32[c], h->B[c], h->phi, h->w32, h->km32, h->gx2, h->gy2, h->pgx32,
                                 h->pgy32, h->avpv32, h->avpu32, h->dzu32, h->dzv32, h->stu32, h->stv32, h->ghu32,
                                 h->ghv32, s);
         });
         tk = best_of(P.tr_kl, [&](int kl) {
-            KPT<float> Q = P;
+            KLT<float> Q = P;
             Q.tr_kl = kl;
             launch_tracer_rhs(Q, h->T32[c], h->S32[c], h->U32[c], h->V32[c], h->w32, h->kh32, h->pgx32, h->pgy32,
                               s);
         });
     } else {
-        const KP& P = h->P;
+        const KL& P = h->P;
         launch_phi(P, h->B[c], h->phi, s);
         mk = best_of(P.mom_kl, [&](int kl) {
-            KP Q = P;
+            KL Q = P;
             Q.mom_kl = kl;
             launch_mom_explicit(Q, h->U[c], h->V[c], h->B[c], h->phi, h->w, h->km, h->gx2, h->gy2, h->pgx, h->pgy,
                                 h->avpv, h->avpu, h->dzu, h->dzv, h->stu, h->stv, h->ghu, h->ghv, s);
         });
         tk = best_of(P.tr_kl, [&](int kl) {
-            KP Q = P;
+            KL Q = P;
             Q.tr_kl = kl;
             launch_tracer_rhs(Q, h->cfg.tracers == OC_TRACERS_TS ? h->Tt[c] : h->B[c], h->Ss[c], h->U[c], h->V[c],
                               h->w, h->kh, h->pgx, h->pgy, s);

@@ -18,14 +18,14 @@ struct BatchRecorder;
 }
 
 using oc::HelmSolver;
-using oc::KP;
-using oc::KPT;
+using oc::KL;
+using oc::KLT;
 
 struct oc_handle {
     oc_config cfg{};
     std::string err;
     bool has_domain = false, has_state = false;
-    KP P{};
+    KL P{};
     int nx = 0, ny = 0, nz = 0;
     size_t n2 = 0, n3 = 0, n3i = 0;
     double h_max = 0.0;
@@ -87,7 +87,7 @@ struct oc_handle {
     // of the state and of the step in FP32; b, phi, eta and every 2D field stay
     // fp64 in the buffers above. The fp64 3D buffers above are then not allocated.
     bool mixed = false;
-    KPT<float> P32{};
+    KLT<float> P32{};
     float *U32[2] = {}, *V32[2] = {}, *T32[2] = {}, *S32[2] = {};
     float *e32 = nullptr, *km32 = nullptr, *kh32 = nullptr, *q32 = nullptr, *w32 = nullptr;
     float *pgx32 = nullptr, *pgy32 = nullptr, *avpv32 = nullptr, *avpu32 = nullptr;

@@ -70,7 +70,7 @@ float* falloc(oc_handle* h, size_t n) {
 
 // the FP32 parameter block: every scalar of the fp64 one rounded once (the
 // scalar products are formed in fp64 first), the fp64 copies kept as they are
-void convert_params(const KP& a, KPT<float>& b) {
+void convert_params(const KL& a, KLT<float>& b) {
     b.nx = a.nx, b.ny = a.ny, b.nz = a.nz, b.n2 = a.n2, b.n3 = a.n3, b.n3i = a.n3i;
     b.dx = (float)a.dx, b.dy = (float)a.dy;
     b.eos = a.eos, b.pgf_remove = a.pgf_remove, b.pgf_correction = a.pgf_correction;
@@ -185,7 +185,7 @@ int mixed_alloc(oc_handle* h, const std::vector<int2>& kinfo, const std::vector<
         tmp[2 * c + 1] = (float)dzx[c].y;
     }
     cudaMemcpy(h->dzx32, tmp.data(), 2 * n2 * sizeof(float), cudaMemcpyHostToDevice);
-    KPT<float>& Q = h->P32;
+    KLT<float>& Q = h->P32;
     convert_params(h->P, Q);
     Q.H = h->H32;
     Q.mask = h->mask32;
@@ -284,7 +284,7 @@ int mixed_get_state(oc_handle* h, const oc_state_view* s, int32_t on_device, cud
 int step_once_mixed(oc_handle* h, cudaStream_t s) {
     const oc_config& c = h->cfg;
     const KP& P = h->P;          // 2D kernels: fp64
-    const KPT<float>& Q = h->P32;  // 3D kernels: FP32
+    const KLT<float>& Q = h->P32;  // 3D kernels: FP32
     const int cur = h->cur, nxt = 1 - cur;
     const float *u = h->U32[cur], *v = h->V32[cur];
     float *un = h->U32[nxt], *vn = h->V32[nxt];

@@ -67,11 +67,6 @@ struct KPT {
     T dzr[OC_MAXNZ];
     T thin[OC_MAXNZ];       // min_partial * dzr
     T dz_nom[OC_MAXNZ];     // spacing of the momentum vertical advection per level
-    // where both columns of a face have their full thickness: the face's thickness at
-    // level k, 1 over it, and 1 over the spacing of the interface between k - 1 and k
-    T fdz[OC_MAXNZ], rfdz[OC_MAXNZ], rfdzi[OC_MAXNZ];
-    T rdz[OC_MAXNZ], rdzi[OC_MAXNZ];  // the same reciprocals of a full column's cells
-    T dzi[OC_MAXNZ];                  // and the interface spacing itself (0: the level below it)
     // static 2D fields
     const T* H;
     const T* mask;
@@ -97,6 +92,19 @@ struct KPT {
     double dzr64[OC_MAXNZ];
 };
 using KP = KPT<double>;
+
+// The same with a table of a full column's levels, for the kernels that read it. A launch
+// copies its parameters: with these 6 KB in every kernel's, each one launched outside a
+// graph took one to two us longer (back substitution of 64 x 64 x 8 10.6 us, without 9.1).
+template <class T>
+struct KLT : KPT<T> {
+    // where both columns of a face have their full thickness: the face's thickness at
+    // level k, 1 over it, and 1 over the spacing of the interface between k - 1 and k
+    T fdz[OC_MAXNZ], rfdz[OC_MAXNZ], rfdzi[OC_MAXNZ];
+    T rdz[OC_MAXNZ], rdzi[OC_MAXNZ];  // the same reciprocals of a full column's cells
+    T dzi[OC_MAXNZ];                  // and the interface spacing itself (0: the level below it)
+};
+using KL = KLT<double>;
 
 __device__ __forceinline__ int wrapi(int i, int n) {
     if (i < 0) i += n;
@@ -152,11 +160,11 @@ struct ColGeoT {
     }
     // 1 over the thickness of level k, and over the spacing of the interface between
     // k - 1 and k: from the level table while the column is full there, so no division
-    __device__ __forceinline__ T rdz(const KPT<T>& P, int k) const {
+    __device__ __forceinline__ T rdz(const KLT<T>& P, int k) const {
         T m;
         return k < kf ? P.rdz[k] : inv_pos(dz(P, k, m));
     }
-    __device__ __forceinline__ T rdzi(const KPT<T>& P, int k) const {
+    __device__ __forceinline__ T rdzi(const KLT<T>& P, int k) const {
         if (k < kf) return P.rdzi[k];
         T m;
         const T a = dz(P, k - 1, m);

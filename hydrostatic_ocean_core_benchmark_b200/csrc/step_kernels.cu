@@ -63,6 +63,7 @@ typedef double wide;
 #endif
 #endif
 using KPR = KPT<real>;
+using KLR = KLT<real>;  // with the level table
 using ColGeoR = ColGeoT<real>;
 
 // ------------------------------------------------------------------ helpers
@@ -86,7 +87,7 @@ __device__ __forceinline__ real m3_at(const KPR& P, const Nbr& n, int dj, int di
 // ------------------------------------------------------------------ q = A^-1 1 on a column
 // interface spacing of the column (closure.py:43-62): dz[0] at the surface,
 // dz[nz-1] at the bottom, the mean of the two levels elsewhere
-__device__ __forceinline__ real col_dzi(const KPR& P, const ColGeoR& g, int k) {
+__device__ __forceinline__ real col_dzi(const KLR& P, const ColGeoR& g, int k) {
     if (k < g.kf) return P.dzi[k];
     real m;
     if (k == 0) return g.dz(P, 0, m);
@@ -100,7 +101,7 @@ __device__ __forceinline__ real col_dzi(const KPR& P, const ColGeoR& g, int k) {
 // elimination keeps its coefficients in cs and its right-hand sides in q, which
 // the back substitution then overwrites with the solution.
 template <class KM>
-__device__ __forceinline__ void column_q(const KPR& P, const ColGeoR& g, KM Km, real* cs,
+__device__ __forceinline__ void column_q(const KLR& P, const ColGeoR& g, KM Km, real* cs,
                                          real* __restrict__ q, int c, size_t n2) {
     const int nz = P.nz;
     real rdzi_k = g.rdz(P, 0);
@@ -137,7 +138,7 @@ __device__ __forceinline__ void column_q(const KPR& P, const ColGeoR& g, KM Km, 
 }
 
 template <int NZM>
-__global__ void __launch_bounds__(128) k_qsolve(KPR P, const real* __restrict__ km,
+__global__ void __launch_bounds__(128) k_qsolve(KLR P, const real* __restrict__ km,
                                                 real* __restrict__ q) {
     COLUMN_PROLOGUE
     const int c = nb.c;
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(128) k_qsolve(KPR P, const real* __restrict__ 
 // 512 x 512 x 50: 817 us a launch before, 750 now (FP32 542 and 465); fewer CTAs per SM
 // make it slower, so its loads' latency bounds it, not the caches' size.
 template <int NZM>
-__global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const real* __restrict__ u,
+__global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KLR P, const real* __restrict__ u,
                                                  const real* __restrict__ v,
                                                  const wide* __restrict__ b,
                                                  real* __restrict__ e, real* __restrict__ km,
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(128, OC_MINB_CLOSURE) k_closure(KPR P, const r
 // or sixteen threads a column are within 20% of eight.
 constexpr int CL_X = 32, CL_Y = 8;
 __global__ void __launch_bounds__(CL_X * CL_Y, 3) k_closure_levels(
-    KPR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b, real* __restrict__ e,
+    KLR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b, real* __restrict__ e,
     real* __restrict__ km, real* __restrict__ kh, real* __restrict__ q) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     const int tiles = (P.nx + CL_X - 1) / CL_X;
@@ -1012,7 +1013,7 @@ struct MomOut {
 // v; COMP 1 is v: along y, u. The terms are those of the general form below, operation
 // for operation; where a factor is 1 or a difference of equal depths 0 it is left out.
 template <int COMP>
-__device__ __forceinline__ void mom_full_level(const KPR& P, const real* __restrict__ X, const real* __restrict__ Y,
+__device__ __forceinline__ void mom_full_level(const KLR& P, const real* __restrict__ X, const real* __restrict__ Y,
                                                unsigned fl, int kff, int k, real x_p2, real K_1, real w_c, real w_f,
                                                wide phc, wide phf, wide bc, wide bf, real tau, real g2, size_t at,
                                                const MomOut& out, MomCarry& q) {
@@ -1109,7 +1110,7 @@ __device__ __forceinline__ unsigned mom_face_flags(const int* own, const int* ot
 // 512 x 512 x 50: 1114 before with 242 of a first k_predictor_rhs beside it, 1043 now (FP32 751
 // with 159, now 636).
 __global__ void __launch_bounds__(MOM_TX * MOM_TY * 2, OC_MINB_MOM) k_mom_column(
-    KPR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b,
+    KLR P, const real* __restrict__ u, const real* __restrict__ v, const wide* __restrict__ b,
     const wide* __restrict__ phi, const real* __restrict__ w, const real* __restrict__ km,
     const wide* __restrict__ gx2, const wide* __restrict__ gy2, real* __restrict__ pgx, real* __restrict__ pgy,
     real* __restrict__ avpv, real* __restrict__ avpu, real* __restrict__ dzu, real* __restrict__ dzv,
@@ -1435,7 +1436,7 @@ __global__ void __launch_bounds__(128) k_momentum_solve(KPR P, const real* __res
 // columns and by components: 16,384 x 50 60 and 51, 512 x 32 33 and 23, 46,937 x 37 39 and 31,
 // 65,536 x 32 52 and 48, 122,880 x 30 67 and 84.
 template <int NZM>
-__global__ void __launch_bounds__(128) k_momentum_solve_few(KPR P, const real* __restrict__ km,
+__global__ void __launch_bounds__(128) k_momentum_solve_few(KLR P, const real* __restrict__ km,
                                                             real* __restrict__ ghu, real* __restrict__ ghv,
                                                             wide* __restrict__ Ug, wide* __restrict__ Vg) {
     COLUMN_PROLOGUE
@@ -1614,7 +1615,7 @@ __device__ __forceinline__ real tracer_vface(const KPR& P, const ColGeoR& g, int
     return real(0.5) * (f_m1 + f_0);
 }
 
-__global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KPR P, const real* __restrict__ C0,
+__global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KLR P, const real* __restrict__ C0,
                                                              const real* __restrict__ S,
                                                              const real* __restrict__ u,
                                                              const real* __restrict__ v,
@@ -2040,7 +2041,7 @@ __device__ __forceinline__ void solve_pairs(unsigned char* s, int nz) {
 }
 
 // the rows of level k of a column (implicit_row_inv)
-__device__ __forceinline__ void solve_row(const KPR& P, const ColGeoR& g, int k, real k_top, real k_bot, real drag,
+__device__ __forceinline__ void solve_row(const KLR& P, const ColGeoR& g, int k, real k_top, real k_bot, real drag,
                                           const SolveRows& R) {
     const real m3_k = k < g.kb ? real(1.0) : real(0.0), m3_k1 = k + 1 < g.kb ? real(1.0) : real(0.0);
     const real rdzi_k = k == 0 ? g.rdz(P, 0) : g.rdzi(P, k), rdzi_k1 = k + 1 < P.nz ? g.rdzi(P, k + 1) : real(0.0);
@@ -2051,7 +2052,7 @@ __device__ __forceinline__ void solve_row(const KPR& P, const ColGeoR& g, int k,
     R.sup[k * SL_X] = sup;
 }
 
-__global__ void __launch_bounds__(SL_X * SL_Y, 3) k_tracer_levels(KPR P, const real* __restrict__ rT,
+__global__ void __launch_bounds__(SL_X * SL_Y, 3) k_tracer_levels(KLR P, const real* __restrict__ rT,
                                                                  const real* __restrict__ rS,
                                                                  const real* __restrict__ kh, real* __restrict__ T_out,
                                                                  real* __restrict__ S_out, wide* __restrict__ b_out) {
@@ -2170,11 +2171,11 @@ __global__ void __launch_bounds__(LV_X * LV_Y) k_transport(KPR P, const real* __
             CALL;                            \
         }                                    \
     } while (0)
-void launch_qsolve(const KPR& P, const real* km, real* q, cudaStream_t s) {
+void launch_qsolve(const KLR& P, const real* km, real* q, cudaStream_t s) {
     NZ_DISPATCH(P.nz, (k_qsolve<NZM><<<col_grid(P), col_block(), 0, s>>>(P, km, q)));
 }
 template <int NZM>
-static void closure_nzm(const KPR& P, const real* u, const real* v, const wide* b, real* e, real* km, real* kh,
+static void closure_nzm(const KLR& P, const real* u, const real* v, const wide* b, real* e, real* km, real* kh,
                         real* q, cudaStream_t s) {
     const dim3 blk = col_block();
 #ifdef OC_MIXED
@@ -2194,7 +2195,7 @@ static void closure_nzm(const KPR& P, const real* u, const real* v, const wide* 
 #endif
     k_closure<NZM><<<col_grid(P), blk, smem, s>>>(P, u, v, b, e, km, kh, q);
 }
-void launch_closure(const KPR& P, const real* u, const real* v, const wide* b, real* e,
+void launch_closure(const KLR& P, const real* u, const real* v, const wide* b, real* e,
                     real* km, real* kh, real* q, cudaStream_t s) {
     if (P.n2 <= kFewColumns) {
         const size_t row = (size_t)5 * CL_X * sizeof(real);
@@ -2262,7 +2263,7 @@ void default_levels(const KPR& P, int& mom_kl, int& tr_kl) {
 }
 static dim3 cell_block() { return dim3(32, 8, 1); }
 static dim3 cell_grid(const KPR& P) { return dim3((P.nx + 31) / 32, (P.ny + 7) / 8, P.nz); }
-void launch_mom_explicit(const KPR& P, const real* u, const real* v, const wide* b,
+void launch_mom_explicit(const KLR& P, const real* u, const real* v, const wide* b,
                          const wide* phi, const real* w, const real* km, const wide* gx2, const wide* gy2,
                          real* pgx, real* pgy, real* avpv, real* avpu, real* dzu, real* dzv, real* stu, real* stv,
                          real* ru, real* rv, cudaStream_t s) {
@@ -2278,7 +2279,7 @@ void launch_predictor_rhs(const KPR& P, const real* u, const real* v, const real
     k_predictor_rhs<<<cell_grid(P), cell_block(), 0, s>>>(P, u, v, u_it, v_it, pgx, pgy, avpv, avpu, dzu,
                                                           dzv, stu, stv, gx2, gy2, ru, rv);
 }
-void launch_momentum_solve(const KPR& P, const real* km, real* ghu, real* ghv, wide* Ug, wide* Vg,
+void launch_momentum_solve(const KLR& P, const real* km, real* ghu, real* ghv, wide* Ug, wide* Vg,
                            cudaStream_t s) {
     if (P.n2 <= kFewColumns) {
         const dim3 grid((P.nx + 31) / 32, (P.ny + 1) / 2);
@@ -2294,12 +2295,12 @@ void launch_backsub(const KPR& P, const real* ghu, const real* ghv, const real* 
     else
         k_backsub<<<col_grid(P), col_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
 }
-void launch_tracer_rhs(const KPR& P, const real* C0, const real* S, const real* u, const real* v,
+void launch_tracer_rhs(const KLR& P, const real* C0, const real* S, const real* u, const real* v,
                        const real* w, const real* kh, real* rT, real* rS, cudaStream_t s) {
     const dim3 grid((P.nx + TRX - 1) / TRX, (P.ny + TRY - 1) / TRY, (P.nz + P.tr_kl - 1) / P.tr_kl);
     k_tracer_rhs<<<grid, dim3(TRX, TRY), 0, s>>>(P, C0, S, u, v, w, kh, rT, rS);
 }
-void launch_tracer_solve(const KPR& P, const real* rT, const real* rS, const real* kh,
+void launch_tracer_solve(const KLR& P, const real* rT, const real* rS, const real* kh,
                          real* T_out, real* S_out, wide* b_out, cudaStream_t s) {
     if (P.n2 <= kFewColumns) {
         const size_t row = (size_t)5 * SL_X * sizeof(real);

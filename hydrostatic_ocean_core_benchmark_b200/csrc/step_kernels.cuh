@@ -3,7 +3,7 @@
 // The 3D kernels (step_kernels.cu) exist for two floating types of the 3D
 // fields: double (the fp64 path, bit-identical to the reference) and float (the
 // mixed-precision path). Their launchers are overloads on the parameter block
-// KPT<R>; b, phi and every 2D field are double on both. The 2D kernels
+// (KPT<R>, or KLT<R> with the level table); b, phi and every 2D field are double on both. The 2D kernels
 // (step2d_kernels.cu) are fp64 only.
 #pragma once
 
@@ -12,15 +12,15 @@
 namespace oc {
 
 #define OC_DECLARE_3D_LAUNCHERS(R)                                                                              \
-    void launch_qsolve(const KPT<R>& P, const R* km, R* q, cudaStream_t s);                                     \
-    void launch_closure(const KPT<R>& P, const R* u, const R* v, const double* b, R* e, R* km, R* kh, R* q,    \
+    void launch_qsolve(const KLT<R>& P, const R* km, R* q, cudaStream_t s);                                     \
+    void launch_closure(const KLT<R>& P, const R* u, const R* v, const double* b, R* e, R* km, R* kh, R* q,    \
                         cudaStream_t s);                                                                        \
     /* levels per CTA of the two level-marching kernels for this grid on the current device */                \
     void default_levels(const KPT<R>& P, int& mom_kl, int& tr_kl);                                             \
     void launch_kukv(const KPT<R>& P, const R* q, double* Ku, double* Kv, cudaStream_t s);                      \
     void launch_wcol(const KPT<R>& P, const R* u, const R* v, R* w, cudaStream_t s);                            \
     void launch_phi(const KPT<R>& P, const double* b, double* phi, cudaStream_t s);                             \
-    void launch_mom_explicit(const KPT<R>& P, const R* u, const R* v, const double* b, const double* phi,      \
+    void launch_mom_explicit(const KLT<R>& P, const R* u, const R* v, const double* b, const double* phi,      \
                              const R* w, const R* km, const double* gx2, const double* gy2, R* pgx, R* pgy,    \
                              R* avpv, R* avpu, R* dzu, R* dzv, R* stu, R* stv, R* ru, R* rv, cudaStream_t s);  \
     /* right-hand sides of the momentum tridiagonals for a later Picard pass (per cell) */                      \
@@ -29,14 +29,14 @@ namespace oc {
                               const R* dzv, const R* stu, const R* stv, const double* gx2, const double* gy2,   \
                               R* ru, R* rv, cudaStream_t s);                                                    \
     /* both column solves in place on gh_u/gh_v, then the transports */                                        \
-    void launch_momentum_solve(const KPT<R>& P, const R* km, R* ghu, R* ghv, double* Ug, double* Vg,           \
+    void launch_momentum_solve(const KLT<R>& P, const R* km, R* ghu, R* ghv, double* Ug, double* Vg,           \
                                cudaStream_t s);                                                                 \
     void launch_backsub(const KPT<R>& P, const R* ghu, const R* ghv, const R* q, const double* eta_new,         \
                         R* u_out, R* v_out, cudaStream_t s);                                                    \
     /* C0: T with TS tracers, else the buoyancy (fp64 path only) */                                             \
-    void launch_tracer_rhs(const KPT<R>& P, const R* C0, const R* S, const R* u, const R* v, const R* w,        \
+    void launch_tracer_rhs(const KLT<R>& P, const R* C0, const R* S, const R* u, const R* v, const R* w,        \
                            const R* kh, R* rT, R* rS, cudaStream_t s);                                          \
-    void launch_tracer_solve(const KPT<R>& P, const R* rT, const R* rS, const R* kh, R* T_out, R* S_out,      \
+    void launch_tracer_solve(const KLT<R>& P, const R* rT, const R* rS, const R* kh, R* T_out, R* S_out,      \
                              double* b_out, cudaStream_t s);                                                    \
     void launch_diag_buoyancy(const KPT<R>& P, const R* T, const R* S, double* b, cudaStream_t s);             \
     void launch_transport(const KPT<R>& P, const R* u, const R* v, double* U, double* V, cudaStream_t s);
