@@ -22,6 +22,7 @@
 //   k_tracer_solve    model3d_v05.py:514-533 + eos.py:68-133
 //   2D kernels        model3d_v05.py:290-335, 376-384, 396-400, 410-413, 440-461
 
+#include <algorithm>
 #include <atomic>
 
 #include "oc_internal.cuh"
@@ -567,7 +568,55 @@ constexpr int LV_X = 32, LV_Y = 8, LV_B = 4, LV_K = LV_Y * LV_B;
 // columns' geometry for little arithmetic: half the limit) at 16,384 x 50 35 and 13, at
 // 46,937 x 37 22 and 26. One grid alone still gains at 65,536 (back substitution 26 and 16),
 // but eight members of an ensemble, which fill the GPU together, lost 5% there.
+// Each kernel has less to gain where a column has few levels, and those that keep a
+// column's rows in shared memory where it has many: their limits below, from both forms
+// timed at 4,096 to 49,152 columns of 4 to 128 levels.
 constexpr int kFewColumns = 49152;
+constexpr bool kFp64 = sizeof(real) == 8;
+
+// Sums over levels (w, Ku and Kv): a chunk costs LV_K levels however many it has. us a launch of
+// w by columns and by levels: 43,264 x 64 82 and 61, x 24 33 and 31, x 16 24 and 29, x 8 16 and
+// 25; 33,792 x 16 24 and 22, x 8 16 and 21; 25,600 x 8 15 and 19; 20,448 x 12 within 2%.
+static int level_sum_columns(int nz) {
+    const int slots = (nz + LV_K - 1) / LV_K * LV_K;
+    if (2 * nz < slots) return 98304 * nz / slots - 16384;
+    return 10 * nz < 6 * slots ? 36864 : kFewColumns;
+}
+
+// Back substitution: with fewer levels than a column has threads, and in FP32 up to two levels
+// a thread, the columns' form is as fast or faster from there on (us by columns and by levels:
+// 33,792 x 4 10.9 and 12.1, 23,040 x 4 11.1 and 10.3; FP32 49,152 x 8 10.0 and 11.0, 33,792 x 12 11.0
+// and 10.6).
+static int backsub_columns(int nz) {
+    if (nz < LV_Y) return kFp64 ? 24576 : 16384;
+    return !kFp64 && nz < 2 * LV_Y ? 36864 : kFewColumns;
+}
+
+// CTAs with that much dynamic shared memory that an SM holds: of its 228 KB a CTA takes 1 KB
+// more than it asks for
+static int smem_ctas(size_t bytes) { return (int)((228 * 1024) / (bytes + 1024)); }
+
+// Closure: with one CTA an SM (from 90 levels on in fp64) from about 27,000 columns on the
+// columns' form is faster (us by columns and by levels: 43,264 x 88 592 and 425, x 104 719
+// and 907; 25,600 x 104 634 and 527), and with few levels, where the lengths' marches are short,
+// earlier too (43,264 x 8 42 and 51, 25,600 x 8 37 and 30; FP32 43,264 x 8 29 and 29).
+static int closure_columns(int nz) {
+    const int limit = smem_ctas((size_t)5 * (nz + 1) * 32 * sizeof(real)) >= 2 ? kFewColumns : 26624;
+    const int shallow = (kFp64 ? 21504 : 32768) + 1024 * nz;
+    return nz < (kFp64 ? 14 : 10) && shallow < limit ? shallow : limit;
+}
+
+// Tracer solve: the two eliminations stay with one warp in four, so the lines lie lower.
+// us by columns and by levels: 43,264 x 128 285 and 475, x 88 199 and 195, x 64 143 and 146, x 40
+// 86 and 78, x 24 47 and 52, x 8 20 and 25; 25,600 x 104 200 and 230, x 24 41 and 33; FP32 43,264 x
+// 128 238 and 206, x 24 38 and 37, x 16 28 and 28, x 8 17 and 19.
+static int tracer_columns(int nz) {
+    if (nz < 8) return 16384;
+    if (!kFp64) return nz < 20 ? 36864 : kFewColumns;
+    if (nz < 32) return nz < 24 ? 25600 : 28672;
+    const int ctas = smem_ctas((size_t)5 * nz * 32 * sizeof(real));
+    return ctas >= 3 ? kFewColumns : ctas == 2 ? 40960 : 16384;
+}
 
 #define LEVELS_PROLOGUE                                          \
     const int lv_tiles = (P.nx + LV_X - 1) / LV_X;               \
@@ -2197,7 +2246,7 @@ static void closure_nzm(const KLR& P, const real* u, const real* v, const wide* 
 }
 void launch_closure(const KLR& P, const real* u, const real* v, const wide* b, real* e,
                     real* km, real* kh, real* q, cudaStream_t s) {
-    if (P.n2 <= kFewColumns) {
+    if (P.n2 <= closure_columns(P.nz)) {
         const size_t row = (size_t)5 * CL_X * sizeof(real);
         // above 48 KB a kernel's dynamic shared memory is opt-in, once per device
         static std::atomic<unsigned long long> opted{0};
@@ -2216,13 +2265,13 @@ void launch_closure(const KLR& P, const real* u, const real* v, const wide* b, r
     NZ_DISPATCH(P.nz, (closure_nzm<NZM>(P, u, v, b, e, km, kh, q, s)));
 }
 void launch_kukv(const KPR& P, const real* q, wide* Ku, wide* Kv, cudaStream_t s) {
-    if (P.n2 <= kFewColumns / 2)
+    if (P.n2 <= std::min(kFewColumns / 2, level_sum_columns(P.nz)))
         k_kukv_few<<<level_grid(P), level_block(), 0, s>>>(P, q, Ku, Kv);
     else
         k_kukv<<<col_grid(P), col_block(), 0, s>>>(P, q, Ku, Kv);
 }
 void launch_wcol(const KPR& P, const real* u, const real* v, real* w, cudaStream_t s) {
-    if (P.n2 <= kFewColumns)
+    if (P.n2 <= level_sum_columns(P.nz))
         k_wcol_few<<<level_grid(P), level_block(), 0, s>>>(P, u, v, w);
     else
         k_wcol<<<col_grid(P), col_block(), 0, s>>>(P, u, v, w);
@@ -2290,7 +2339,7 @@ void launch_momentum_solve(const KLR& P, const real* km, real* ghu, real* ghv, w
 }
 void launch_backsub(const KPR& P, const real* ghu, const real* ghv, const real* q,
                     const wide* eta_new, real* u_out, real* v_out, cudaStream_t s) {
-    if (P.n2 <= kFewColumns)
+    if (P.n2 <= backsub_columns(P.nz))
         k_backsub_few<<<level_grid(P), level_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
     else
         k_backsub<<<col_grid(P), col_block(), 0, s>>>(P, ghu, ghv, q, eta_new, u_out, v_out);
@@ -2302,7 +2351,7 @@ void launch_tracer_rhs(const KLR& P, const real* C0, const real* S, const real* 
 }
 void launch_tracer_solve(const KLR& P, const real* rT, const real* rS, const real* kh,
                          real* T_out, real* S_out, wide* b_out, cudaStream_t s) {
-    if (P.n2 <= kFewColumns) {
+    if (P.n2 <= tracer_columns(P.nz)) {
         const size_t row = (size_t)5 * SL_X * sizeof(real);
         // above 48 KB a kernel's dynamic shared memory is opt-in, once per device
         static std::atomic<unsigned long long> opted{0};

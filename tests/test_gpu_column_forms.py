@@ -19,6 +19,9 @@ pytestmark = pytest.mark.gpu
     (256, 192, 3), (256, 193, 3),   # the limit of the few-column forms, and just above it
     (128, 192, 2), (193, 128, 2),   # half of it (K_u, K_v)
     (45, 3, 33), (33, 5, 8), (7, 4, 1), (64, 2, 41),  # part-filled warps; around a chunk of levels
+    # the kernels' own limits, which depend on the levels: few of them, one CTA of rows an SM
+    (224, 128, 24), (225, 128, 24), (256, 144, 16), (256, 145, 16), (128, 32, 8), (128, 65, 8), (128, 129, 7),
+    (41, 30, 90), (41, 30, 128),
 ])
 def test_column_forms_match_oracle(nx, ny, nz, mxl):
     from hydrostatic_ocean_core_benchmark_b200 import cases
