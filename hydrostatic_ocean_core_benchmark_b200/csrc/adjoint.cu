@@ -734,8 +734,6 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
     const int cEE = j * nx + (i + 2 >= nx ? i + 2 - nx : i + 2);
     const int cSS = ((j <= 1) ? j - 2 + ny : j - 2) * nx + i;
     const int cNN = ((j + 2 >= ny) ? j + 2 - ny : j + 2) * nx + i;
-    const int cSE = (j == 0 ? ny - 1 : j - 1) * nx + (i + 1 == nx ? 0 : i + 1);
-    const int cNW = (j + 1 == ny ? 0 : j + 1) * nx + (i == 0 ? nx - 1 : i - 1);
     const double dz_nom = P.dz_nom[k];
     const unsigned mask = row_mask(i, nx);
     Scatter gu, gv, gw;
@@ -936,8 +934,6 @@ __global__ void k_mom_adv_T(KP P, const double* __restrict__ u, const double* __
     scatter_x(w_b, o, gw, gw_own, i, j, nx, mask);
     atomic_add(&w_b[o + c], gw_own);
     atomic_add(&w_b[o + cN], gw.n);
-    (void)cSE;
-    (void)cNW;
 }
 
 // pressure gradient (model3d_v05.py:211-230): pg = m3f ((phi_F + b_F (zf - zc_F)) -

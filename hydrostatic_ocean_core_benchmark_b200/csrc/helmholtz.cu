@@ -672,7 +672,7 @@ struct PwNode {
     int lo, height;
 };
 
-// The tree embedded in a perfect one: the slot of each leaf, in order, under a
+// The tree embedded in a perfect one: where each leaf starts and its slot, in order, under a
 // node of height `height` (2^height slots) whose first slot is `slot`. A leaf
 // above height 0 takes the first slot of its subtree.
 static int pairwise_height(long n) {
@@ -682,15 +682,16 @@ static int pairwise_height(long n) {
     return std::max(pairwise_height(h), pairwise_height(n - h)) + 1;
 }
 
-static void pairwise_slots(long n, int height, int slot, std::vector<int>& slots) {
+static void pairwise_slots(long start, long n, int height, int slot, std::vector<int>& leaves, std::vector<int>& slots) {
     if (n <= 128) {
+        leaves.push_back((int)start);
         slots.push_back(slot);
         return;
     }
     long h = n / 2;
     h -= h % 8;
-    pairwise_slots(h, height - 1, slot, slots);
-    pairwise_slots(n - h, height - 1, slot + (1 << (height - 1)), slots);
+    pairwise_slots(start, h, height - 1, slot, leaves, slots);
+    pairwise_slots(start + h, n - h, height - 1, slot + (1 << (height - 1)), leaves, slots);
 }
 
 static PwNode pairwise_build(long start, long n, std::vector<int>& leaves,
@@ -874,29 +875,23 @@ int HelmSolver::init(int nx, int ny, double dx0, double dy0, double coef, int ki
     H.p = (double*)dalloc(sizeof(double) * n);
     H.Ap = (double*)dalloc(sizeof(double) * n);
     // pairwise plan (two-level for grids whose leaf sums exceed shared memory)
-    std::vector<int> leaves;
-    std::vector<std::vector<int2>> by_height;  // of the whole tree; the embedded fold does not need it
+    std::vector<int> leaves, slots;
     TwoLevelPlan two;
     H.big_fold = pairwise_leaves((long)n) > kFoldOneLevelLeaves ? 1 : 0;
     if (H.big_fold) {
         pairwise_build_two_level(0, (long)n, kFoldBlockLeaves, two);
         leaves = two.leaves;
+        // the two-level fold reads the leaves in order
+        for (int q = 0; q < (int)leaves.size(); ++q) slots.push_back(q);
+        H.n_slots = (int)slots.size();
     } else {
-        pairwise_build(0, (long)n, leaves, by_height);
+        // the leaves' slots in the perfect tree (at least one warp's 32)
+        const int height = pairwise_height((long)n);
+        pairwise_slots(0, (long)n, height, 0, leaves, slots);
+        H.n_slots = std::max(32, 1 << height);
     }
     leaves.push_back((int)n);
     H.n_leaves = (int)leaves.size() - 1;
-    // the leaves' slots in the perfect tree (at least one warp's 32); the two-level
-    // fold reads the leaves in order
-    std::vector<int> slots;
-    if (H.big_fold) {
-        for (int q = 0; q < H.n_leaves; ++q) slots.push_back(q);
-        H.n_slots = H.n_leaves;
-    } else {
-        const int height = pairwise_height((long)n);
-        pairwise_slots((long)n, height, 0, slots);
-        H.n_slots = std::max(32, 1 << height);
-    }
     int* d_leaves = (int*)dalloc(sizeof(int) * leaves.size());
     int* d_slots = (int*)dalloc(sizeof(int) * slots.size());
     H.leafA = (double*)dalloc(sizeof(double) * H.n_slots);  // zeroed: slots without a leaf stay 0

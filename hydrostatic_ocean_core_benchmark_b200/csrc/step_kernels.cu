@@ -1595,7 +1595,7 @@ __global__ void __launch_bounds__(LV_X * LV_Y) k_backsub_few(KPR P, const real* 
 // A CTA owns a TRX x TRY tile of columns and P.tr_kl levels and marches down the
 // levels. At each level the horizontal face fluxes of the tile -- TRX + 1 east
 // faces per row, TRY + 1 north faces per column -- are formed once into shared
-// memory (double-buffered, one barrier per level); a per-cell form would form
+// memory, the level below it staged meanwhile; a per-cell form would form
 // every face twice, once from each side. The vertical face at the bottom of a
 // cell is carried to the next level as the face at its top, and the column's
 // tracer values, w and K_h roll in registers. Every face and cell value is
@@ -1605,47 +1605,6 @@ __global__ void __launch_bounds__(LV_X * LV_Y) k_backsub_few(KPR P, const real* 
 // level table and need no mask but the open faces. 512 x 512 x 50: 887 us a launch with one
 // form for all levels, 694 with the short one above the general one (FP32 548, now 438).
 constexpr int TRX = 32, TRY = 8;
-
-struct Stencil4 {
-    int cm, c0, c1, cp;  // far upstream, the two cells of the face, far downstream (flat 2D)
-};
-
-// the east face of column i in row j (cells i-1, i, i+1, i+2), periodic index layout
-__device__ __forceinline__ Stencil4 xstencil(int j, int i, int nx, int ny) {
-    const int r = wrapi(j, ny) * nx;
-    return Stencil4{r + wrapi(i - 1, nx), r + wrapi(i, nx), r + wrapi(i + 1, nx), r + wrapi(i + 2, nx)};
-}
-
-// the north face of row j in column i (rows j-1, j, j+1, j+2)
-__device__ __forceinline__ Stencil4 ystencil(int j, int i, int nx, int ny) {
-    const int ii = wrapi(i, nx);
-    return Stencil4{wrapi(j - 1, ny) * nx + ii, wrapi(j, ny) * nx + ii, wrapi(j + 1, ny) * nx + ii,
-                    wrapi(j + 2, ny) * nx + ii};
-}
-
-// tracer value on a horizontal face: centred, kappa/TVD with the dry far-cell
-// fallback, or first-order upwind (model3d_v05.py:482-497)
-__device__ __forceinline__ real tracer_face(const KPR& P, const real* __restrict__ C, size_t o,
-                                              const Stencil4& s, real vel, int k) {
-    const real a = C[o + s.c0], b = C[o + s.c1];
-    if (P.advection == 1) return real(0.5) * (a + b);
-    if (P.advection >= 3)
-        return kappa_face(P, C[o + s.cm], a, b, C[o + s.cp], vel, col_m3(P, s.cm, k), col_m3(P, s.cp, k),
-                          P.advection == 4);
-    return vel > real(0.0) ? a : b;
-}
-
-// flux through an east (ax = 0) or north (ax = 1) face: face thickness x
-// normal velocity x face value (model3d_v05.py:498-501)
-__device__ __forceinline__ real tracer_flux(const KPR& P, const real* __restrict__ C,
-                                              const real* __restrict__ vel_f, size_t o,
-                                              const Stencil4& s, int k, int ax) {
-    const real vel = vel_f[o + s.c0];
-    const int2 kf = P.kface[s.c0];
-    real m;
-    const real dzf = face_dz(P, ax == 0 ? kf.x : kf.y, k, col_dz(P, s.c0, k, m), col_dz(P, s.c1, k, m));
-    return dzf * vel * tracer_face(P, C, o, s, vel, k);
-}
 
 // tracer value on interface kk of a column (0 = surface) from the column values
 // at kk-2, kk-1, kk, kk+1 and w there (model3d_v05.py:502-510)
@@ -1729,7 +1688,8 @@ __global__ void __launch_bounds__(TRX * TRY, OC_MINB_TRACER) k_tracer_rhs(KLR P,
         return k == q.x ? s_d0[r] : s_d1[r];
     };
     // flux through a face with stencil cells (cm, c0, c1, cp) of the region,
-    // normal velocity vel and face wet levels kfa (tracer_flux from shared memory)
+    // normal velocity vel and face wet levels kfa: face thickness x velocity x face value
+    // (model3d_v05.py:482-501)
     auto sflux = [&](const real* F, int cm, int c0, int c1, int cp, real vel, int kfa, int k) {
         real m;
         const real dzf = face_dz(P, kfa, k, sdz(c0, k, m), sdz(c1, k, m));
