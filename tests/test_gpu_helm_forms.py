@@ -90,11 +90,13 @@ def test_uneven_leaf_trees_match_oracle(kind, nx, ny):
     (6, 4), (62, 30), (64, 40), (40, 64),  # one CTA: tiny, an odd coarsest level, the largest
     (66, 40), (52, 50),                               # just above it
     (128, 96), (128, 128),                            # tiles over one-CTA coarse levels
-    (384, 256), (384, 272),                           # wide tiles with their x and b kept
+    (384, 256), (384, 272),                           # 32 x 32 tiles
+    (384, 512), (256, 640),                           # 128 x 16 tiles with their x and b kept, the test piped
+    (512, 512),                                       # the same, the residual formed in the up phase
     (512, 520), (1024, 400),                          # a partial last row of tiles; more tiles than SMs
 ])
 def test_multigrid_forms_match_oracle(nx, ny):
-    """The V-cycle on one CTA and on tiles of every form."""
+    """The V-cycle on one CTA and on tiles of every form (those of a B200's 148 SMs)."""
     from hydrostatic_ocean_core_benchmark_b200.solvers_var import HelmholtzVar
     dx, dy, coef, ku, kv, mask, rhs = _system(nx, ny, nx + 7 * ny, walls=True)
     solver = HelmholtzVar(SimpleNamespace(nx=nx, ny=ny, dx=dx, dy=dy), coef, ku, kv, mask, kind="multigrid",
