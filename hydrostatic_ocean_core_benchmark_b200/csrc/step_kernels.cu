@@ -576,11 +576,12 @@ constexpr bool kFp64 = sizeof(real) == 8;
 
 // Sums over levels (w, Ku and Kv): a chunk costs LV_K levels however many it has. us a launch of
 // w by columns and by levels: 43,264 x 64 82 and 61, x 24 33 and 31, x 16 24 and 29, x 8 16 and
-// 25; 33,792 x 16 24 and 22, x 8 16 and 21; 25,600 x 8 15 and 19; 20,448 x 12 within 2%.
+// 25; 33,792 x 16 24 and 22, x 8 16 and 21; 25,600 x 8 15 and 19; 20,448 x 12 within 2%; of two
+// chunks 43,264 x 40 within 2%, x 33 43 and 47, 46,937 x 37 48 and 41.
 static int level_sum_columns(int nz) {
     const int slots = (nz + LV_K - 1) / LV_K * LV_K;
     if (2 * nz < slots) return 98304 * nz / slots - 16384;
-    return 10 * nz < 6 * slots ? 36864 : kFewColumns;
+    return 100 * nz < (nz <= LV_K ? 60 : 55) * slots ? 36864 : kFewColumns;
 }
 
 // Back substitution: with fewer levels than a column has threads, and in FP32 up to two levels
