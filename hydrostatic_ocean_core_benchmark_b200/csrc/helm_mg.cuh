@@ -781,22 +781,53 @@ __device__ __noinline__ void mg_coarse(const double* xin_cf, double* xout_cf, bo
     __syncthreads();
 }
 
-// ------------------------------------------------------------------ flat tiles (coarsest level only)
+// ------------------------------------------------------------------ the coarsest level on the grid
 __device__ __forceinline__ bool level_even(const HLevel& L) { return ((L.nx | L.ny) & 1) == 0; }
 
-// smoothing of a coarsest level too large for CTA 0 and possibly odd-sized: two forward
-// or two reverse sweeps on 32 x 32 tiles in the flat order, each cell tested for its
-// colour by its grid coordinates
-template <int SHRINK>
-__device__ void flat_half_sweep(const HLevel& L, int i0, int j0, TileRefs t, int colour, bool unit, bool even) {
+// The region of an odd-sized level's tile in the flat order; all of a thread's loads are
+// issued before its first store to shared memory. code[k] is twice the ring of the
+// thread's k-th cell plus its colour, which the grid coordinates give (-1: no cell).
+static constexpr int kFlatCells = (Tile32::RN + kSolveThreads - 1) / kSolveThreads;
+__device__ __forceinline__ void flat_load(const HLevel& L, int i0, int j0, const double* xin, TileRefs t,
+                                          int (&code)[kFlatCells]) {
     constexpr int RW = Tile32::RW, RH = Tile32::RH;
-    for (int r = threadIdx.x; r < Tile32::RN; r += kSolveThreads) {
+    double xv[kFlatCells], bv[kFlatCells];
+#pragma unroll
+    for (int k = 0; k < kFlatCells; ++k) {
+        const int r = threadIdx.x + k * kSolveThreads;
+        xv[k] = bv[k] = 0.0;
+        code[k] = -1;
+        if (r >= Tile32::RN) continue;
         const int rj = r / RW, ri = r - rj * RW;
-        if (ri < SHRINK || ri >= RW - SHRINK || rj < SHRINK || rj >= RH - SHRINK) continue;
-        // a wrap by an even size keeps the colour, so the region coordinates give it
-        int par = ri + rj;
-        if (!even) par = wrap_any(i0 - HALO + ri, L.nx) + wrap_any(j0 - HALO + rj, L.ny);
-        if ((par & 1) != colour) continue;
+        const int gi = wrap_any(i0 - HALO + ri, L.nx), gj = wrap_any(j0 - HALO + rj, L.ny);
+        const int g = gj * L.nx + gi;
+        code[k] = 2 * min(min(ri, RW - 1 - ri), min(rj, RH - 1 - rj)) + ((gi + gj) & 1);
+        cpa_ca8(t.ku + r, L.Ku + g);
+        cpa_ca8(t.kv + r, L.Kv + g);
+        cpa_ca8(t.id + r, L.idm + g);
+        cpa_ca8(t.m + r, L.mask + g);
+        if (xin) xv[k] = __ldcg(xin + g);
+        bv[k] = __ldcg(L.b + g);
+    }
+#pragma unroll
+    for (int k = 0; k < kFlatCells; ++k) {
+        const int r = threadIdx.x + k * kSolveThreads;
+        if (r >= Tile32::RN) continue;
+        t.x[r] = xv[k];
+        t.b[r] = bv[k];
+    }
+    cpa_wait_all();
+    __syncthreads();
+}
+
+// a half-sweep of such a tile: the cells of colour `colour` on the rings from `ring` on
+__device__ __forceinline__ void flat_half_sweep(const HLevel& L, TileRefs t, const int (&code)[kFlatCells], int ring,
+                                                int colour, bool unit) {
+    constexpr int RW = Tile32::RW;
+#pragma unroll
+    for (int k = 0; k < kFlatCells; ++k) {
+        if (code[k] < 2 * ring || (code[k] & 1) != colour) continue;
+        const int r = threadIdx.x + k * kSolveThreads;
         const double nb = L.cx * (t.ku[r] * t.x[r + 1] + t.ku[r - 1] * t.x[r - 1]) +
                           L.cy * (t.kv[r] * t.x[r + RW] + t.kv[r - RW] * t.x[r - RW]);
         double v = t.id[r] * (t.b[r] + nb);
@@ -806,6 +837,10 @@ __device__ void flat_half_sweep(const HLevel& L, int i0, int j0, TileRefs t, int
     __syncthreads();
 }
 
+// Smoothing of a coarsest level too large for CTA 0: two forward or two reverse sweeps on
+// 32 x 32 tiles, colours apart where the level is even. us a solve with all tiles in the flat
+// order, loaded cell by cell and each cell's colour worked out in every sweep, and so:
+// 1000 x 10 199 and 170, 75 x 75 218 and 188, 257 x 129 223 and 196.
 __device__ __noinline__ void mg_smooth(int l, const double* xin, double* xout, bool reverse, int smem) {
     using S = Tile32;
     const HelmParams& H = s_helm;
@@ -817,28 +852,21 @@ __device__ __noinline__ void mg_smooth(int l, const double* xin, double* xout, b
     const bool even = level_even(L);
     for (int tile = s_grid.cta; tile < tx * ty; tile += s_grid.ncta) {
         const int i0 = (tile % tx) * S::TX, j0 = (tile / tx) * S::TY;
-        for (int r = threadIdx.x; r < S::RN; r += kSolveThreads) {
-            const int rj = r / S::RW, ri = r - rj * S::RW;
-            const int g = wrap_any(j0 - HALO + rj, L.ny) * L.nx + wrap_any(i0 - HALO + ri, L.nx);
-            cpa_ca8(t.ku + r, L.Ku + g);
-            cpa_ca8(t.kv + r, L.Kv + g);
-            cpa_ca8(t.id + r, L.idm + g);
-            cpa_ca8(t.m + r, L.mask + g);
-            const double bv = __ldcg(L.b + g);
-            t.x[r] = xin ? __ldcg(xin + g) : 0.0;
-            t.b[r] = bv;
-        }
-        cpa_wait_all();
-        __syncthreads();
-        flat_half_sweep<1>(L, i0, j0, t, c0, unit, even);
-        flat_half_sweep<2>(L, i0, j0, t, 1 - c0, unit, even);
-        flat_half_sweep<3>(L, i0, j0, t, c0, unit, even);
-        flat_half_sweep<4>(L, i0, j0, t, 1 - c0, unit, even);
-        for (int r = threadIdx.x; r < S::TX * S::TY; r += kSolveThreads) {
-            const int cj = r / S::TX, ci = r - cj * S::TX;
-            const int gi = i0 + ci, gj = j0 + cj;
-            if (gi >= L.nx || gj >= L.ny) continue;
-            xout[gj * L.nx + gi] = t.x[(cj + HALO) * S::RW + ci + HALO];
+        if (even) {
+            tile_load<S, true>(L, i0, j0, xin, nullptr, 0, t);
+            tile_four_half_sweeps<S>(L, t, c0, unit);
+            tile_store_x<S>(L, i0, j0, t, xout);
+        } else {
+            int code[kFlatCells];
+            flat_load(L, i0, j0, xin, t, code);
+#pragma unroll 1
+            for (int h = 0; h < 4; ++h) flat_half_sweep(L, t, code, h + 1, (c0 + h) & 1, unit);
+            for (int r = threadIdx.x; r < S::TX * S::TY; r += kSolveThreads) {
+                const int cj = r / S::TX, ci = r - cj * S::TX;
+                const int gi = i0 + ci, gj = j0 + cj;
+                if (gi >= L.nx || gj >= L.ny) continue;
+                xout[gj * L.nx + gi] = t.x[(cj + HALO) * S::RW + ci + HALO];
+            }
         }
         __syncthreads();
     }

@@ -90,6 +90,7 @@ def test_uneven_leaf_trees_match_oracle(kind, nx, ny):
     (6, 4), (62, 30), (64, 40), (40, 64),  # one CTA: tiny, an odd coarsest level, the largest
     (66, 40), (52, 50),                               # just above it
     (128, 96), (128, 128),                            # tiles over one-CTA coarse levels
+    (300, 14), (75, 77), (290, 142),                  # a coarsest level on the grid: even; odd; below a finer one
     (384, 256), (384, 272),                           # 32 x 32 tiles
     (384, 512), (256, 640),                           # 128 x 16 tiles with their x and b kept, the test piped
     (512, 512),                                       # the same, the residual formed in the up phase
